@@ -10,7 +10,7 @@ namespace {
 // the thin y sweep of batch.cuh in the mixed form: the boundary-face states in FP64 (side_states), their primitives
 // rounded to FP32, the Riemann solver and the balance in FP32 (as mixed_axis does for boundary faces)
 template <int RIEMANN>
-__device__ __forceinline__ float thin_face_mixed(const StageArgs& a, const Eos<float>& ef, float sb, int side, int i, St<float, 4>& F) {
+__device__ __forceinline__ float thin_face_mixed(const StageArgs& a, const GasF& ef, float sb, int side, int i, St<float, 4>& F) {
     St<double, 4> UL, UR;
     side_states<4, false>(a.m, a.bc, a.eos, a.U, side, i, 0, 0, UL, UR);
     const St<double, 4> dl = c2p(a.eos, UL), dr = c2p(a.eos, UR);
@@ -24,7 +24,7 @@ __device__ __forceinline__ float thin_face_mixed(const StageArgs& a, const Eos<f
 }
 
 template <int RIEMANN, int TX, int NT>
-__device__ __forceinline__ void thin_y_mixed(const StageArgs& a, const Eos<float>& ef, float sb, float* __restrict__ acc, const int o3[3], float& smax) {
+__device__ __forceinline__ void thin_y_mixed(const StageArgs& a, const GasF& ef, float sb, float* __restrict__ acc, const int o3[3], float& smax) {
     const Mesh& m = a.m;
     const float A = (float)m.area[1];
     const bool same = copy_side(a.bc.type[2]) && copy_side(a.bc.type[3]);
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(NT) batch_mixed_kernel(const BatchArgs b) {
         if (tid == 0) batch_item_args(b, b.prob[it.prob], sa);
         __syncthreads();
         const Mesh& m = sa.m;
-        const Eos<float> ef{sa.eos.type, (float)sa.eos.gamma, (float)sa.eos.p_inf};
+        const GasF ef = gas_f(sa.eos);
         const float sb = (float)sa.shock_blend, weps = (float)sa.weno_eps;
         const int tx = (m.nx + TX - 1) / TX;
         const int o3[3] = {(it.tile % tx) * TX, (it.tile / tx) * TY, 0};

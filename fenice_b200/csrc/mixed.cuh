@@ -24,41 +24,150 @@
 
 namespace fvg {
 
-// HLLC / low-Mach HLLC of a face from its two primitive states (the Riemann solver of the mixed form)
-template <int RIEMANN, int NV>
-__device__ __forceinline__ float face_flux_prim(const Eos<float>& e, float shock_blend, St<float, NV> WL, St<float, NV> WR, int axis, St<float, NV>& F) {
-    WL[0] = vmax(WL[0], Num<float>::eos_eps);
-    WL[3] = vmax(WL[3], Num<float>::eos_eps);
-    WR[0] = vmax(WR[0], Num<float>::eos_eps);
-    WR[3] = vmax(WR[3], Num<float>::eos_eps);
-    const float inv_L = 1.0f / WL[0], inv_R = 1.0f / WR[0];
-    const float c_L = sound_speed_inv(e, WL[3], inv_L), c_R = sound_speed_inv(e, WR[3], inv_R);
-    if constexpr (RIEMANN == kLowMach) {
-        float mL2 = WL[1] * WL[1] + WL[2] * WL[2], mR2 = WR[1] * WR[1] + WR[2] * WR[2];
-        if constexpr (NV == 5) {
-            mL2 += WL[4] * WL[4];
-            mR2 += WR[4] * WR[4];
-        }
-        const float M_L = sqrtf(mL2) / (c_L + Num<float>::mach_eps);
-        const float M_R = sqrtf(mR2) / (c_R + Num<float>::mach_eps);
-        const float z = vmin(vmax(vmax(M_L, M_R), 1e-4f), 1.0f);
-#pragma unroll
-        for (int a = 0; a < (NV == 5 ? 3 : 2); ++a) {
-            const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-            const float avg = 0.5f * (WL[m] + WR[m]);
-            const float half = 0.5f * (WL[m] - WR[m]);
-            WL[m] = avg + z * half;
-            WR[m] = avg - z * half;
-        }
-    }
-    return hllc_core(WL, WR, p2c(e, WL), p2c(e, WR), inv_L, inv_R, c_L, c_R, axis, shock_blend, F);
+// The gas of the mixed form's Riemann solver: gamma, p_inf (0 for an ideal gas), 1 / (gamma - 1) and gamma p_inf.
+struct GasF {
+    float g, pi, g1, gpi;
+};
+__device__ __forceinline__ GasF gas_f(const Eos<double>& e) {
+    GasF s;
+    s.g = (float)e.gamma;
+    s.pi = e.type == kIdeal ? 0.0f : (float)e.p_inf;
+    s.g1 = __frcp_rn((float)(e.gamma - 1.0));
+    s.gpi = __fmul_rn(s.g, s.pi);
+    return s;
+}
+// maximum / minimum of two floats in one instruction, a NaN operand kept
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
-// the fifth-order upwind value right of c2 from c0 .. c4: 0.1 p0 + 0.6 p1 + 0.3 p2 of the three candidate stencils
-// (explicitly rounded FMAs, as the single-precision weno5z: the same bits in every kernel)
-__device__ __forceinline__ float lin5(float c0, float c1, float c2, float c3, float c4) {
-    const float s = __fmaf_rn(-3.0f, c4, __fmaf_rn(27.0f, c3, __fmaf_rn(47.0f, c2, __fmaf_rn(-13.0f, c1, __fmul_rn(2.0f, c0)))));
-    return __fmul_rn(s, 1.0f / 60.0f);
+// HLLC / low-Mach HLLC of a face from its two primitive states (the Riemann solver of the mixed form), every operation
+// rounded explicitly so that each kernel that solves a face gets the same flux.
+//
+// The star flux is written from the side the contact leaves to the other: with S the wave speed of that side, q =
+// rho (S - u_n) and f = q / (S - S_M), the mass flux is f S_M, the momentum flux f S_M v (+ p* = p + q (S_M - u_n) along
+// the normal) and the energy flux S_M (f E + ... + p*): the same flux as F + S (U* - U) of both sides and a choice
+// between the four, in exact arithmetic, with one side's states instead of two, two reciprocals instead of five and no
+// difference of nearly equal products at low Mach numbers. A supersonic face is the same formulas with S_M = u_n, f = rho,
+// p* = p. The Mach number of the low-Mach scaling takes one reciprocal and one square root for both sides.
+template <int RIEMANN, int NV>
+__device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend, St<float, NV> WL, St<float, NV> WR, int axis, St<float, NV>& F) {
+    constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
+    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
+    const float rL = max_nan(WL[0], Num<float>::eos_eps), pL = max_nan(WL[3], Num<float>::eos_eps);
+    const float rR = max_nan(WR[0], Num<float>::eos_eps), pR = max_nan(WR[3], Num<float>::eos_eps);
+    const float iL = rcp_f(rL), iR = rcp_f(rR);
+    const float aL = __fmul_rn(__fmul_rn(e.g, __fadd_rn(pL, e.pi)), iL), aR = __fmul_rn(__fmul_rn(e.g, __fadd_rn(pR, e.pi)), iR);   // c^2
+    const float cL = sqrt_f(aL), cR = sqrt_f(aR);
+    if constexpr (RIEMANN == kLowMach) {
+        float mL = __fmul_rn(WL[1], WL[1]), mR = __fmul_rn(WR[1], WR[1]);
+        mL = __fmaf_rn(WL[2], WL[2], mL);
+        mR = __fmaf_rn(WR[2], WR[2], mR);
+        if constexpr (NV == 5) {
+            mL = __fmaf_rn(WL[4], WL[4], mL);
+            mR = __fmaf_rn(WR[4], WR[4], mR);
+        }
+        const bool gl = __fmul_rn(mL, aR) > __fmul_rn(mR, aL);   // the larger Mach number's side
+        const float M = sqrt_f(__fmul_rn(gl ? mL : mR, rcp_f(gl ? aL : aR)));
+        const float z = min_nan(max_nan(M, 1e-4f), 1.0f);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
+            const float avg = __fmul_rn(0.5f, __fadd_rn(WL[m], WR[m]));
+            const float half = __fmul_rn(0.5f, __fsub_rn(WL[m], WR[m]));
+            WL[m] = __fmaf_rn(z, half, avg);
+            WR[m] = __fmaf_rn(-z, half, avg);
+        }
+    }
+    const float uL = WL[mn], uR = WR[mn];
+    const float SL = min_nan(__fsub_rn(uL, cL), __fsub_rn(uR, cR)), SR = max_nan(__fadd_rn(uL, cL), __fadd_rn(uR, cR));
+    const float qL = __fmul_rn(rL, __fsub_rn(SL, uL)), qR = __fmul_rn(rR, __fsub_rn(SR, uR));
+    const float num = __fmaf_rn(qR, uR, __fmaf_rn(-qL, uL, __fsub_rn(pL, pR)));
+    float SM = __fmul_rn(num, rcp_f(max_nan(__fsub_rn(qR, qL), Num<float>::denom_eps)));   // (qR >= 0 >= qL)
+    const bool sup = SL >= 0.0f || SR < 0.0f;
+    const bool left = SR >= 0.0f && (SL >= 0.0f || SM >= 0.0f);
+    const bool fail = !sup && !(SM >= 0.0f) && !(SM < 0.0f);   // a NaN speed: no flux
+    const float rho = left ? rL : rR, p = left ? pL : pR, un = left ? uL : uR, q = left ? qL : qR;
+    float vt[NA];   // the side's velocity
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
+        vt[a] = left ? WL[m] : WR[m];
+    }
+    float ke = __fmul_rn(vt[0], vt[0]);
+#pragma unroll
+    for (int a = 1; a < NA; ++a) ke = __fmaf_rn(vt[a], vt[a], ke);
+    const float E = __fmaf_rn(0.5f, ke, __fmul_rn(__fmul_rn(__fadd_rn(p, e.gpi), e.g1), left ? iL : iR));   // per unit mass
+    const float d = __fsub_rn(SM, un);
+    const float w = __fsub_rn(left ? SL : SR, SM);
+    const float rc = rcp_f(copysignf(max_nan(fabsf(w), Num<float>::denom_eps), w));
+    float f = __fmul_rn(q, rc), ps = __fmaf_rn(q, d, p);
+    float Es = __fmaf_rn(f, __fmaf_rn(d, SM, E), __fmul_rn(__fmul_rn(d, p), rc));
+    if (sup) {
+        SM = un;
+        f = rho;
+        ps = p;
+        Es = __fmul_rn(rho, E);
+    }
+    const float G = __fmul_rn(f, SM);
+    F[0] = G;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
+        F[m] = a == axis ? __fmaf_rn(G, SM, ps) : __fmul_rn(G, vt[a]);
+    }
+    F[3] = __fmul_rn(SM, __fadd_rn(Es, ps));
+    const float jump = fabsf(__fsub_rn(pR, pL)), pm = min_nan(pL, pR);
+    if (shock_blend > 0.0f && jump > __fmul_rn(shock_blend, pm) && !sup) {
+        // a strong pressure jump: the HLL flux blended in
+        const float phi = min_nan(__fmul_rn(__fsub_rn(__fmul_rn(jump, rcp_f(pm)), shock_blend), rcp_f(shock_blend)), 1.0f);
+        const float inv = rcp_f(__fsub_rn(SR, SL)), ss = __fmul_rn(SL, SR);
+        const float mL = __fmul_rn(rL, uL), mR = __fmul_rn(rR, uR);
+        float kL = __fmul_rn(WL[1], WL[1]), kR = __fmul_rn(WR[1], WR[1]);
+        kL = __fmaf_rn(WL[2], WL[2], kL);
+        kR = __fmaf_rn(WR[2], WR[2], kR);
+        if constexpr (NV == 5) {
+            kL = __fmaf_rn(WL[4], WL[4], kL);
+            kR = __fmaf_rn(WR[4], WR[4], kR);
+        }
+        const float EL = __fmaf_rn(__fmul_rn(0.5f, rL), kL, __fmul_rn(__fadd_rn(pL, e.gpi), e.g1));
+        const float ER = __fmaf_rn(__fmul_rn(0.5f, rR), kR, __fmul_rn(__fadd_rn(pR, e.gpi), e.g1));
+        const auto blend = [&](float f0, float fl, float fr, float ul, float ur) {
+            const float h = __fmul_rn(__fmaf_rn(ss, __fsub_rn(ur, ul), __fmaf_rn(SR, fl, -__fmul_rn(SL, fr))), inv);
+            return __fmaf_rn(phi, h, __fmul_rn(__fsub_rn(1.0f, phi), f0));
+        };
+        F[0] = blend(F[0], mL, mR, rL, rR);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
+            F[m] = blend(F[m], a == axis ? __fmaf_rn(mL, WL[m], pL) : __fmul_rn(mL, WL[m]), a == axis ? __fmaf_rn(mR, WR[m], pR) : __fmul_rn(mR, WR[m]),
+                         __fmul_rn(rL, WL[m]), __fmul_rn(rR, WR[m]));
+        }
+        F[3] = blend(F[3], __fmul_rn(uL, __fadd_rn(EL, pL)), __fmul_rn(uR, __fadd_rn(ER, pR)), EL, ER);
+    }
+    if (fail)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) F[k] = 0.0f;
+    return max_nan(fabsf(SL), fabsf(SR));
+}
+
+// The two linear face values of six cells: the fifth-order upwind value right of c2 from c0 .. c4, 0.1 p0 + 0.6 p1 + 0.3 p2
+// of the three candidate stencils, and its mirror image left of c3 from c5 .. c1, in the two lanes of packed operations
+// (half the issue slots of two scalar evaluations; explicitly rounded, as weno5z_pair: the same bits in every kernel).
+__device__ __forceinline__ void lin5_pair(float c0, float c1, float c2, float c3, float c4, float c5, float& wl, float& wr) {
+    F2 s = f2_mul(f2(2.0f, 2.0f), f2(c0, c5));
+    s = f2_fma(f2(-13.0f, -13.0f), f2(c1, c4), s);
+    s = f2_fma(f2(47.0f, 47.0f), f2(c2, c3), s);
+    s = f2_fma(f2(27.0f, 27.0f), f2(c3, c2), s);
+    s = f2_fma(f2(-3.0f, -3.0f), f2(c4, c1), s);
+    f2_get(f2_mul(s, f2(1.0f / 60.0f, 1.0f / 60.0f)), wl, wr);
 }
 
 template <int DIM, int RECON, int TX, int TY, int TZ> struct MixedShape {
@@ -85,7 +194,7 @@ template <int DIM, int RECON, int TX, int TY, int TZ> struct MixedShape {
 // arrays (free during the load) and converted from there; the others take the index-mapping loader. `phase` counts the
 // barrier's completed copies (its parity is the one to wait for).
 template <int AXIS, int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool GATED = false, bool FULL = true, bool TMA = false>
-__device__ __forceinline__ void mixed_axis(const StageArgs& a, const Eos<float>& ef, float sb, float weps, float* __restrict__ P,
+__device__ __forceinline__ void mixed_axis(const StageArgs& a, const GasF& ef, float sb, float weps, float* __restrict__ P,
                                            float* __restrict__ WL, float* __restrict__ WR, float* __restrict__ acc, unsigned char* __restrict__ Sf,
                                            const int o3[3], float& smax, const CUtensorMap* maps = nullptr, unsigned long long* bar = nullptr,
                                            unsigned* phase = nullptr) {
@@ -194,11 +303,9 @@ __device__ __forceinline__ void mixed_axis(const StageArgs& a, const Eos<float>&
                     if (!(f3[AXIS] == 0 ? seam_lo : (f3[AXIS] == hi_face ? seam_hi : true))) continue;
                     // linear fifth-order upwind values where the sensor passed the tile (the WENO-Z weights at their
                     // linear values 0.1, 0.6, 0.3)
-                    wl = lin5(c0, c1, c2, c3, c4);
-                    wr = lin5(c5, c4, c3, c2, c1);
+                    lin5_pair(c0, c1, c2, c3, c4, c5, wl, wr);
                 } else {
-                    wl = weno5z(c0, c1, c2, c3, c4, weps);
-                    wr = weno5z(c5, c4, c3, c2, c1, weps);
+                    weno5z_pair(c0, c1, c2, c3, c4, c5, weps, wl, wr);
                 }
             }
             WL[q * S::NF + f] = wl;
@@ -229,8 +336,7 @@ __device__ __forceinline__ void mixed_axis(const StageArgs& a, const Eos<float>&
                         wl = weno3z(c1, c2, c3, weps);
                         wr = weno3z(c4, c3, c2, weps);
                     } else {
-                        wl = weno5z(c0, c1, c2, c3, c4, weps);
-                        wr = weno5z(c5, c4, c3, c2, c1, weps);
+                        weno5z_pair(c0, c1, c2, c3, c4, c5, weps, wl, wr);
                     }
                     WL[q * S::NF + f] = wl;
                     WR[q * S::NF + f] = wr;
@@ -342,7 +448,7 @@ __global__ void __launch_bounds__(NT) mixed_stage_kernel(const StageArgs a) {
     unsigned char* Sf = reinterpret_cast<unsigned char*>(acc + NV * NC);   // [EXT]
     if (!*a.gate) return;
     const Mesh& m = a.m;
-    const Eos<float> ef{a.eos.type, (float)a.eos.gamma, (float)a.eos.p_inf};
+    const GasF ef = gas_f(a.eos);
     const float sb = (float)a.shock_blend, weps = (float)a.weno_eps;
     const int tid = threadIdx.x, b = blockIdx.x + a.b0;
     const int o3[3] = {(b % a.tiles[0]) * TX, ((b / a.tiles[0]) % a.tiles[1]) * TY, (b / (a.tiles[0] * a.tiles[1])) * TZ};
@@ -668,7 +774,7 @@ __device__ __forceinline__ int cross_cell(int e, int l3[3]) {
 // One face of axis A in the cross (linear face values): item r of the axis (the 448 faces inside the tile, t = 1 .. 7,
 // then the two seam layers t = 0 and 8); its flux goes to Fs at the face's index in mixed_axis's numbering.
 template <int A, int RIEMANN>
-__device__ __forceinline__ void cross_face(const StageArgs& a, const Eos<float>& ef, float sb, const float* __restrict__ P, float* __restrict__ Fs,
+__device__ __forceinline__ void cross_face(const StageArgs& a, const GasF& ef, float sb, const float* __restrict__ P, float* __restrict__ Fs,
                                            int r, const int o3[3], float& smax) {
     constexpr int NV = 5, NPC = CrossShape::NPC;
     int t, u, v;
@@ -701,8 +807,7 @@ __device__ __forceinline__ void cross_face(const StageArgs& a, const Eos<float>&
     for (int q = 0; q < NV; ++q) {
         const float* c = P + q * NPC;
         const float c0 = c[sl[0]], c1 = c[sl[1]], c2 = c[sl[2]], c3 = c[sl[3]], c4 = c[sl[4]], c5 = c[sl[5]];
-        wl[q] = lin5(c0, c1, c2, c3, c4);
-        wr[q] = lin5(c5, c4, c3, c2, c1);
+        lin5_pair(c0, c1, c2, c3, c4, c5, wl[q], wr[q]);
     }
     const Mesh& m = a.m;
     const int n3[3] = {m.nx, m.ny, m.nz};
@@ -751,7 +856,7 @@ __device__ __forceinline__ void cross_tile(const StageArgs& a, const TmaMaps& ma
     float* Fs = reinterpret_cast<float*>(smem_b + L::STG_OFF);
     const Mesh& m = a.m;
     const int n3[3] = {m.nx, m.ny, m.nz};
-    const Eos<float> ef{a.eos.type, (float)a.eos.gamma, (float)a.eos.p_inf};
+    const GasF ef = gas_f(a.eos);
     const float sb = (float)a.shock_blend;
     const int tid = threadIdx.x;
     const bool aligned = (tma::su32(stg) & 127u) == 0;
@@ -924,7 +1029,7 @@ __global__ void __launch_bounds__(NT, 3) mixed_stage_kernel_tma(const StageArgs 
         unsigned char* Sf = smem_b + LO::SF_OFF;
         float* WL = reinterpret_cast<float*>(smem_b + LO::STG_OFF);
         float* WR = WL + NV * S::NF;
-        const Eos<float> ef{a.eos.type, (float)a.eos.gamma, (float)a.eos.p_inf};
+        const GasF ef = gas_f(a.eos);
         const float sb = (float)a.shock_blend, weps = (float)a.weno_eps;
         mixed_axis<0, 3, kWeno5, RIEMANN, 8, 8, 8, NT, GATED, false, true>(a, ef, sb, weps, P, WL, WR, acc, Sf, o3, smax, maps.m, bar, &phase);
         mixed_axis<1, 3, kWeno5, RIEMANN, 8, 8, 8, NT, GATED, false, true>(a, ef, sb, weps, P, WL, WR, acc, Sf, o3, smax, maps.m, bar, &phase);

@@ -164,32 +164,79 @@ template <typename T> __device__ __forceinline__ T weno5z(T c0, T c1, T c2, T c3
     const T a0 = T(0.1) * (T(1) + tau / (b0 + eps)), a1 = T(0.6) * (T(1) + tau / (b1 + eps)), a2 = T(0.3) * (T(1) + tau / (b2 + eps));
     return (a0 * p0 + a1 * p1 + a2 * p2) / (a0 + a1 + a2);
 }
-// The single-precision WENO5-Z of the mixed form: the same weights, with every product and sum rounded by an explicit
-// intrinsic (FMAs placed by hand) and the candidates' common 1/6 folded into the last division, so that no compiler pass
-// contracts it one way in one kernel and another way in the next: every kernel that solves a face gets the same bits.
-__device__ __forceinline__ float weno5z(float c0, float c1, float c2, float c3, float c4, float eps_rel) {
-    float ss = __fmul_rn(c0, c0);
-    ss = __fmaf_rn(c1, c1, ss);
-    ss = __fmaf_rn(c2, c2, ss);
-    ss = __fmaf_rn(c3, c3, ss);
-    ss = __fmaf_rn(c4, c4, ss);
-    const float eps = __fmaf_rn(__fmul_rn(eps_rel, ss), 0.2f, Num<float>::weno_floor);
-    const float p0 = __fmaf_rn(11.0f, c2, __fmaf_rn(-7.0f, c1, __fmul_rn(2.0f, c0)));   // 6 x the three candidates
-    const float p1 = __fmaf_rn(2.0f, c3, __fmaf_rn(5.0f, c2, -c1));
-    const float p2 = __fmaf_rn(5.0f, c3, __fmaf_rn(2.0f, c2, -c4));
-    const float s0 = __fadd_rn(__fmaf_rn(-2.0f, c1, c0), c2), t0 = __fmaf_rn(3.0f, c2, __fmaf_rn(-4.0f, c1, c0));
-    const float s1 = __fadd_rn(__fmaf_rn(-2.0f, c2, c1), c3), t1 = __fsub_rn(c1, c3);
-    const float s2 = __fadd_rn(__fmaf_rn(-2.0f, c3, c2), c4), t2 = __fadd_rn(__fmaf_rn(-4.0f, c3, __fmul_rn(3.0f, c2)), c4);
-    constexpr float k = 13.0f / 12.0f;
-    const float b0 = __fmaf_rn(__fmul_rn(k, s0), s0, __fmul_rn(__fmul_rn(0.25f, t0), t0));
-    const float b1 = __fmaf_rn(__fmul_rn(k, s1), s1, __fmul_rn(__fmul_rn(0.25f, t1), t1));
-    const float b2 = __fmaf_rn(__fmul_rn(k, s2), s2, __fmul_rn(__fmul_rn(0.25f, t2), t2));
-    const float tau = fabsf(__fsub_rn(b0, b2));
-    const float a0 = __fmul_rn(0.1f, __fadd_rn(1.0f, tau / __fadd_rn(b0, eps)));
-    const float a1 = __fmul_rn(0.6f, __fadd_rn(1.0f, tau / __fadd_rn(b1, eps)));
-    const float a2 = __fmul_rn(0.3f, __fadd_rn(1.0f, tau / __fadd_rn(b2, eps)));
-    const float num = __fmaf_rn(a2, p2, __fmaf_rn(a1, p1, __fmul_rn(a0, p0)));
-    return num / __fmul_rn(6.0f, __fadd_rn(__fadd_rn(a0, a1), a2));
+// Two FP32 values in one 64-bit register pair: sm_100a's packed add, multiply and FMA round each lane as the scalar
+// operation does, at one issue slot for both.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f2_get(F2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// the hardware's approximate reciprocal and square root (each within about one unit in the last place)
+__device__ __forceinline__ float rcp_f(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_f(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ F2 f2_rcp(F2 v) {
+    float a, b;
+    f2_get(v, a, b);
+    return f2(rcp_f(a), rcp_f(b));
+}
+
+// The single-precision WENO5-Z of the mixed form, both values of a face at once: wl right of c2 from c0 .. c4 in the low
+// lane, wr left of c3 from c5 .. c1 in the high lane. The same weights, with every product and sum rounded by an explicit
+// packed operation (FMAs placed by hand) and the candidates' common 1/6 folded into the last division, so that no compiler
+// pass contracts it one way in one kernel and another way in the next: every kernel that solves a face gets the same bits.
+__device__ __forceinline__ void weno5z_pair(float c0, float c1, float c2, float c3, float c4, float c5, float eps_rel, float& wl, float& wr) {
+    const auto k = [](float v) { return f2(v, v); };
+    const F2 a = f2(c0, c5), b = f2(c1, c4), c = f2(c2, c3), d = f2(c3, c2), e = f2(c4, c1);
+    F2 ss = f2_mul(a, a);
+    ss = f2_fma(b, b, ss);
+    ss = f2_fma(c, c, ss);
+    ss = f2_fma(d, d, ss);
+    ss = f2_fma(e, e, ss);
+    const F2 eps = f2_fma(f2_mul(k(eps_rel), ss), k(0.2f), k(Num<float>::weno_floor));
+    const F2 p0 = f2_fma(k(11.0f), c, f2_fma(k(-7.0f), b, f2_mul(k(2.0f), a)));   // 6 x the three candidates
+    const F2 p1 = f2_fma(k(2.0f), d, f2_fma(k(5.0f), c, f2_mul(k(-1.0f), b)));
+    const F2 p2 = f2_fma(k(5.0f), d, f2_fma(k(2.0f), c, f2_mul(k(-1.0f), e)));
+    const F2 s0 = f2_add(f2_fma(k(-2.0f), b, a), c), t0 = f2_fma(k(3.0f), c, f2_fma(k(-4.0f), b, a));
+    const F2 s1 = f2_add(f2_fma(k(-2.0f), c, b), d), t1 = f2_fma(k(-1.0f), d, b);
+    const F2 s2 = f2_add(f2_fma(k(-2.0f), d, c), e), t2 = f2_add(f2_fma(k(-4.0f), d, f2_mul(k(3.0f), c)), e);
+    const F2 w = k(13.0f / 12.0f), h = k(0.25f);
+    const F2 b0 = f2_fma(f2_mul(w, s0), s0, f2_mul(f2_mul(h, t0), t0));
+    const F2 b1 = f2_fma(f2_mul(w, s1), s1, f2_mul(f2_mul(h, t1), t1));
+    const F2 b2 = f2_fma(f2_mul(w, s2), s2, f2_mul(f2_mul(h, t2), t2));
+    float dl, dr;
+    f2_get(f2_fma(k(-1.0f), b2, b0), dl, dr);
+    const F2 tau = f2(fabsf(dl), fabsf(dr));
+    const F2 a0 = f2_mul(k(0.1f), f2_fma(tau, f2_rcp(f2_add(b0, eps)), k(1.0f)));
+    const F2 a1 = f2_mul(k(0.6f), f2_fma(tau, f2_rcp(f2_add(b1, eps)), k(1.0f)));
+    const F2 a2 = f2_mul(k(0.3f), f2_fma(tau, f2_rcp(f2_add(b2, eps)), k(1.0f)));
+    const F2 num = f2_fma(a2, p2, f2_fma(a1, p1, f2_mul(a0, p0)));
+    const F2 den = f2_mul(k(6.0f), f2_add(f2_add(a0, a1), a2));
+    f2_get(f2_mul(num, f2_rcp(den)), wl, wr);
 }
 
 // ------------------------------------------------------------------ HLLC (Toro) with Einfeldt bounds (Schemes.cpp:116-200)
