@@ -23,7 +23,6 @@ using namespace fvg;
 
 namespace {
 
-constexpr double kDtEps = 1e-10;   // TimeScheme.cpp:19
 
 // ------------------------------------------------------------------------------------------------ control kernels
 __global__ void k_batch_begin(BatchCtl* c, int n, double t_end, int max_steps) {

@@ -24,6 +24,7 @@ constexpr int kHaloNone = 0, kHaloWrap = 1, kHaloSlab = 2, kHaloPeer = 3;
 // host round trip (and can be captured in a CUDA graph).
 struct Ctl {
     double t, t_end, dt, dt_max, cfl, L;
+    double dt_step;     // the length of the last step taken
     double s_lag;       // MUSCL-Hancock: wave speed of the previous step (0: none yet)
     double s_step;      // largest wave speed of the current step
     double s_stage[3];  // wave speed of each stage of the step
@@ -36,7 +37,81 @@ struct Ctl {
     int status;         // 0 ok; 1 the solution diverged (non-finite speed or dt, or t no longer advances); 3 a
                         // time-dependent boundary value was not finite, or rho_in or p_out not positive, at a stage time;
                         // 5 a TMA copy of a stage tile, 6 a tensor-core step of the sensor did not complete (a bounded wait gave up)
+    unsigned ticket;    // CTAs of the running stage launch that are done (stage_finish)
+    unsigned long long s_bits;   // the largest speed so far, as the bits of a non-negative double
 };
+
+constexpr double kDtEps = 1e-10;   // TimeScheme.cpp:19
+
+__device__ __forceinline__ void set_next_active(Ctl* c) {
+    c->active = (c->t < c->t_end) && (c->max_steps <= 0 || c->steps < c->max_steps) && c->status == 0;
+}
+// the step length from a wave speed, clamped to t_end and dt_max
+__device__ __forceinline__ double step_length(const Ctl* c, double s) {
+    double dt = __ddiv_rn(__dmul_rn(c->cfl, c->L), __dadd_rn(s, kDtEps));
+    dt = vmin(dt, __dsub_rn(c->t_end, c->t));
+    if (c->dt_max > 0.0) dt = vmin(dt, c->dt_max);
+    return dt;
+}
+// check_progress (cpp/src/SimulationInternal.hpp:259-267), t += dt, and whether the next step runs
+__device__ __forceinline__ void finish_step(Ctl* c, double s) {
+    c->s_step = s;
+    c->dt_step = c->dt;
+    if (!(isfinite(s) && isfinite(c->dt) && __dadd_rn(c->t, c->dt) > c->t)) {
+        c->status = 1;
+        c->active = 0;
+        return;
+    }
+    c->t = __dadd_rn(c->t, c->dt);
+    c->steps += 1;
+    set_next_active(c);
+}
+// the step of MUSCL-Hancock that starts now: dt from the lagged speed (MusclHancock::step, TimeScheme.cpp:296-319)
+__device__ __forceinline__ void hancock_dt(Ctl* c) {
+    c->dt = step_length(c, c->s_lag);
+    c->half_dt = __dmul_rn(0.5, c->dt);
+}
+
+// What a stage (or viscous) launch does with its CTAs' largest wave speeds. kFinNone: each CTA writes its own to the
+// launch's blockmax array, for a kernel that follows. The others fold it into Ctl::s_bits by atomicMax (the bits of
+// non-negative doubles order as the doubles do, and a maximum does not depend on the order, so the result has the same
+// bits), and the last CTA to finish, found by a ticket, does what a control kernel after the launch would: kFinDt the
+// step length after a step's first stage, kFinStep the end of a Runge-Kutta step, kFinHancock the end of a MUSCL-Hancock
+// step and the length of the next one. A control kernel costs about 4 us of a step at every size (131 x 97 cells, SSP-RK2:
+// seven launches and 36 us per step before).
+constexpr int kFinNone = 0, kFinMax = 1, kFinDt = 2, kFinStep = 3, kFinHancock = 4;
+struct Fin {
+    Ctl* ctl;
+    int kind;
+    int ctas;   // of the launch
+};
+// by one thread of each CTA, its last act (every other thread's reads of the control block lie before the block
+// reduction that gave bm)
+__device__ __forceinline__ void stage_finish(const Fin& f, double* blockmax, int b, double bm) {
+    if (f.kind == kFinNone) {
+        blockmax[b] = bm;
+        return;
+    }
+    Ctl* c = f.ctl;
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(bm);
+    if (bits > *(volatile unsigned long long*)&c->s_bits) atomicMax(&c->s_bits, bits);
+    if (f.kind == kFinMax) return;
+    __threadfence();
+    if (atomicAdd(&c->ticket, 1u) != (unsigned)f.ctas - 1u) return;
+    __threadfence();
+    c->ticket = 0;
+    const double s = __longlong_as_double((long long)atomicExch(&c->s_bits, 0ull));
+    if (f.kind == kFinDt) {
+        c->s_stage[0] = s;
+        c->dt = step_length(c, s);
+    } else if (f.kind == kFinStep) {
+        finish_step(c, vmax(c->s_stage[0], s));
+    } else {
+        c->s_lag = s;
+        finish_step(c, s);
+        if (c->active) hancock_dt(c);
+    }
+}
 
 struct Mesh {
     int nx, ny, nz;

@@ -32,6 +32,7 @@ struct HancockArgs {
     const double* Rv;  // the viscous residual of U (null: inviscid); it joins the balance, not the predictor
     double* out;
     double* blockmax;
+    Fin fin;           // kFinNone: the CTAs' speeds to blockmax
     const Ctl* ctl;    // dt and half_dt
     const int* gate;
     int tiles[3];
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(NT) hancock_kernel(const HancockArgs a) {
         }
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 }   // namespace fvg
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(NT) hancock3d_kernel(const HancockArgs a) {
         }
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 }   // namespace fvg

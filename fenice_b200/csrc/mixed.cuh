@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(NT) mixed_stage_kernel(const StageArgs a) {
         for (int q = 0; q < NV; ++q) a.out[q * m.plane + cell] = cell_out(a, in, q, acc[q * NC + c], dt);
     }
     const double bm = block_max<NT>((double)smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 template <int TX, int TY, int TZ> struct MixedViscShape {
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
         if (s > smax) smax = s;
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 // The per-axis sweep's shared memory with TMA boxes (mixed_axis with TMA): red [32 doubles] | the barrier | P | acc | Sf |
@@ -1047,7 +1047,7 @@ __global__ void __launch_bounds__(NT, 3) mixed_stage_kernel_tma(const StageArgs 
         }
     }
     const double bm = block_max<NT>((double)smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 }   // namespace fvg

@@ -45,7 +45,6 @@ using namespace fvg;
 
 namespace {
 
-constexpr double kDtEps = 1e-10;   // TimeScheme.cpp:19
 thread_local std::string g_create_error;
 
 // ------------------------------------------------------------------------------------------------ control kernels
@@ -66,15 +65,13 @@ __device__ double block_reduce_max(const double* a, int n, const double* b, int 
     return r;
 }
 
-__device__ __forceinline__ void set_next_active(Ctl* c) {
-    c->active = (c->t < c->t_end) && (c->max_steps <= 0 || c->steps < c->max_steps) && c->status == 0;
-}
-
 __global__ void k_begin(Ctl* c, double t_end, int max_steps) {
     c->t_end = t_end;
     c->max_steps = max_steps;
     c->steps = 0;
     c->status = 0;
+    c->ticket = 0;
+    c->s_bits = 0;
     set_next_active(c);
 }
 
@@ -84,10 +81,7 @@ __global__ void k_stage1_dt(Ctl* c, const double* bm, int nb, const double* bmv,
     const double s = block_reduce_max(bm, nb, bmv, nbv);
     if (threadIdx.x == 0) {
         c->s_stage[0] = s;
-        double dt = c->cfl * c->L / (s + kDtEps);
-        dt = vmin(dt, c->t_end - c->t);
-        if (c->dt_max > 0.0) dt = vmin(dt, c->dt_max);
-        c->dt = dt;
+        c->dt = step_length(c, s);
     }
 }
 
@@ -95,19 +89,6 @@ __global__ void k_stage_max(Ctl* c, const int* gate, int stage, const double* bm
     if (!*gate) return;
     const double s = block_reduce_max(bm, nb, bmv, nbv);
     if (threadIdx.x == 0) c->s_stage[stage] = s;
-}
-
-// check_progress (cpp/src/SimulationInternal.hpp:259-267), t += dt, and whether the next step runs
-__device__ void finish_step(Ctl* c, double s) {
-    c->s_step = s;
-    if (!(isfinite(s) && isfinite(c->dt) && c->t + c->dt > c->t)) {
-        c->status = 1;
-        c->active = 0;
-        return;
-    }
-    c->t = c->t + c->dt;
-    c->steps += 1;
-    set_next_active(c);
 }
 
 // end of a Runge-Kutta / Euler step with `nstages` stages: S = max(s1, max(s2, s3))
@@ -128,11 +109,7 @@ __global__ void k_hancock_seed(Ctl* c, const double* bm, int nb, const double* b
 }
 __global__ void k_hancock_dt(Ctl* c) {
     if (!c->active) return;
-    double dt = c->cfl * c->L / (c->s_lag + kDtEps);
-    dt = vmin(dt, c->t_end - c->t);
-    if (c->dt_max > 0.0) dt = vmin(dt, c->dt_max);
-    c->dt = dt;
-    c->half_dt = 0.5 * dt;
+    hancock_dt(c);
 }
 // the step's speed: the Hancock residual's, max the viscous bound (Simulation.cpp:1038-1041), lagged to the next step
 __global__ void k_hancock_end(Ctl* c, const double* bm, int nb, const double* bmv, int nbv) {
@@ -142,6 +119,17 @@ __global__ void k_hancock_end(Ctl* c, const double* bm, int nb, const double* bm
         c->s_lag = s;
         finish_step(c, s);
     }
+}
+
+// the end of a step whose stages folded their speeds into the control block, where another kernel runs between the last
+// stage and it (the immersed body's reset)
+__global__ void k_end_folded(Ctl* c, int hancock) {
+    if (!c->active) return;
+    const double s = __longlong_as_double((long long)c->s_bits);
+    c->s_bits = 0;
+    if (hancock) c->s_lag = s;
+    finish_step(c, hancock ? s : vmax(c->s_stage[0], s));
+    if (hancock && c->active) hancock_dt(c);
 }
 
 // BoundaryManager::apply_side's mass-flow target (Boundaries.cpp:284-294), one block per side: the mean over the side's
@@ -622,6 +610,7 @@ struct fvg_run {
     StageLauncher stage;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};   // two steps, by the buffer the state starts in (MUSCL-Hancock ping-pong)
     int cur = 0;   // MUSCL-Hancock ping-pong: 0 the state is in U, 1 in Ut
+    double clock_t = 0.0, clock_dt = 0.0;   // the clock as fvg_run_until read it last (only how many graphs to launch depends on it)
     // kernel timing (fvg_set_timing): CUDA events around each launch of the stage (or predictor) kernel and of the
     // viscous kernel, on the run's stream; the steps are then launched one by one instead of as graphs
     struct EvTimer {
@@ -1059,11 +1048,14 @@ cudaError_t massflow_targets(fvg_run* r, const double* Uin, const int* gate) {
 }
 
 // The viscous residual of Uin into Rv and its per-CTA speed bounds into bmv.
-cudaError_t launch_visc(fvg_run* r, const double* Uin, double* bmv, const int* gate, bool timed = true) {
+// With `fold` they go to the control block instead (the stage launch that follows finishes with them).
+cudaError_t launch_visc(fvg_run* r, const double* Uin, double* bmv, const int* gate, bool timed = true, bool fold = false) {
     if (timed) timer_mark(r, r->t_visc);
-    const cudaError_t e = r->dim == 2 ? launch_viscous2d(visc_args(r, Uin, bmv, gate), r->nbv, r->stream)
-                          : r->cfg.precision == FVG_PREC_MIXED ? mixed_viscous_launch(visc_args(r, Uin, bmv, gate), r->nbv, r->stream)
-                                                               : launch_viscous(visc_args(r, Uin, bmv, gate), r->nbv, r->stream);
+    ViscArgs a = visc_args(r, Uin, bmv, gate);
+    if (fold) a.fin = Fin{r->ctl, kFinMax, r->nbv};
+    const cudaError_t e = r->dim == 2 ? launch_viscous2d(a, r->nbv, r->stream)
+                          : r->cfg.precision == FVG_PREC_MIXED ? mixed_viscous_launch(a, r->nbv, r->stream)
+                                                               : launch_viscous(a, r->nbv, r->stream);
     if (timed) timer_mark(r, r->t_visc);
     return e;
 }
@@ -1141,15 +1133,16 @@ cudaError_t stage_values(fvg_run* r, int kind, const int* gate) {
 // One residual stage of Uin: the immersed body's forced states, the viscous sweep (viscous runs), then the inviscid
 // stage kernel.
 cudaError_t residual_stage(fvg_run* r, const double* Uin, const double* U0, double* out, int mode, double ca, double cb, int stage, const int* gate,
-                           const unsigned char* fb = nullptr) {
+                           const unsigned char* fb = nullptr, int fin = kFinNone) {
     cudaError_t e;
     if ((e = stage_values(r, r->res_kind >= 0 ? r->res_kind : stage, gate)) != cudaSuccess) return e;
     if (r->ibm && (e = ibm_fill(r, Uin, nullptr, 0, gate)) != cudaSuccess) return e;
     if ((e = massflow_targets(r, Uin, gate)) != cudaSuccess) return e;
-    if (r->cfg.use_viscous && (e = launch_visc(r, Uin, r->bmv[stage], gate)) != cudaSuccess) return e;
+    if (r->cfg.use_viscous && (e = launch_visc(r, Uin, r->bmv[stage], gate, true, fin != kFinNone)) != cudaSuccess) return e;
     timer_mark(r, r->t_stage);
     StageArgs sa = stage_args(r, Uin, U0, out, mode, ca, cb, r->cfg.use_viscous ? r->Rv : nullptr, r->bm[stage], gate);
     sa.fb = fb;
+    sa.fin = Fin{r->ctl, fin, r->nb};
     e = r->fourth ? fourth_stage(r, sa) : r->stage.launch(sa, r->nb, r->stream);
     timer_mark(r, r->t_stage);
     return e;
@@ -1247,36 +1240,32 @@ cudaError_t enqueue_step(fvg_run* r, bool refresh = true) {
     const int* act = &c->active;
     const int nbv = r->cfg.use_viscous ? r->nbv : 0;
     const int ts = r->cfg.time_scheme;
-    if (ts == FVG_TS_HANCOCK) {
+    if (ts == FVG_TS_HANCOCK) {   // (its dt was set by hancock_start, or at the end of the step before)
         double* Uin = r->Ucur();
         double* Uout = r->cur ? r->U : r->Ut;
-        k_hancock_begin<<<1, 1, 0, r->stream>>>(c);
-        // the seed (first step only; untimed): one plain residual for the speed, its viscous bound included
-        if ((e = stage_values(r, 0, &c->seed))) return e;
-        if (r->ibm && (e = ibm_fill(r, Uin, nullptr, 0, &c->seed))) return e;
-        if ((e = massflow_targets(r, Uin, &c->seed))) return e;
-        if (r->cfg.use_viscous && (e = launch_visc(r, Uin, r->bmv[1], &c->seed, false))) return e;
-        if ((e = r->stage.launch(stage_args(r, Uin, nullptr, r->R, kStoreR, 0, 0, r->cfg.use_viscous ? r->Rv : nullptr, r->bm_seed, &c->seed), r->nb,
-                                 r->stream)))
-            return e;
-        k_hancock_seed<<<1, 1024, 0, r->stream>>>(c, r->bm_seed, r->nb, r->bmv[1], nbv);
-        k_hancock_dt<<<1, 1, 0, r->stream>>>(c);
         if ((e = stage_values(r, 2, act))) return e;   // t + dt / 2: the sources centred in the step
         if (r->ibm && (e = ibm_fill(r, Uin, nullptr, 0, act))) return e;
         if ((e = massflow_targets(r, Uin, act))) return e;
-        if (r->cfg.use_viscous && (e = launch_visc(r, Uin, r->bmv[0], act))) return e;
+        if (r->cfg.use_viscous && (e = launch_visc(r, Uin, r->bmv[0], act, true, true))) return e;
         timer_mark(r, r->t_stage);
-        e = launch_hancock(r, hancock_args(r, Uin, Uout, kAxpy, r->bm[0], act));
+        HancockArgs ha = hancock_args(r, Uin, Uout, kAxpy, r->bm[0], act);
+        ha.fin = Fin{c, r->ibm ? kFinMax : kFinHancock, r->nbh};
+        e = launch_hancock(r, ha);
         timer_mark(r, r->t_stage);
         if (e) return e;
-        if (r->ibm && (e = ibm_fill(r, Uout, Uout, 1, act))) return e;
-        k_hancock_end<<<1, 1024, 0, r->stream>>>(c, r->bm[0], r->nbh, r->bmv[0], nbv);
+        if (r->ibm) {
+            if ((e = ibm_fill(r, Uout, Uout, 1, act))) return e;
+            k_end_folded<<<1, 1, 0, r->stream>>>(c, 1);
+        }
         r->cur ^= 1;
         return cudaGetLastError();
     }
     if (refresh && (e = refresh_gate(r, r->U, c))) return e;
-    if ((e = residual_stage(r, r->U, nullptr, r->R, kStoreR, 0, 0, 0, act))) return e;
-    k_stage1_dt<<<1, 1024, 0, r->stream>>>(c, r->bm[0], r->nb, r->bmv[0], nbv);
+    // the stage launches fold their speeds into the control block and the last CTAs of the first and the last one do the
+    // control work (the fourth-order face passes: control kernels after them)
+    const bool fold = !r->fourth;
+    if ((e = residual_stage(r, r->U, nullptr, r->R, kStoreR, 0, 0, 0, act, nullptr, fold ? kFinDt : kFinNone))) return e;
+    if (!fold) k_stage1_dt<<<1, 1024, 0, r->stream>>>(c, r->bm[0], r->nb, r->bmv[0], nbv);
     if (r->dynamic) {   // a body driven by the flow: the loads of this first stage, about the pivot of the step
         const double vol = r->dim == 3 ? r->m.dx * r->m.dy * r->m.dz : r->m.dx * r->m.dy;
         k_body_loads<<<1, 32, 0, r->stream>>>(act, r->R, r->U, r->m.plane, r->d_solid, r->nsolid, vol, r->m.nx, r->m.ny, r->m.dx, r->m.dy, r->m.dz,
@@ -1290,19 +1279,42 @@ cudaError_t enqueue_step(fvg_run* r, bool refresh = true) {
         return cudaGetLastError();
     }
     k_axpy<<<axpy_blocks(r), 256, 0, r->stream>>>(c, r->Ut, r->U, r->R, r->m.plane, r->m.ncells, r->nvar);
+    const int last = !fold ? kFinNone : (r->ibm ? kFinMax : kFinStep);
+    const int nstages = ts == FVG_TS_SSPRK2 ? 2 : 3;
     if (ts == FVG_TS_SSPRK2) {
-        if ((e = residual_stage(r, r->Ut, r->U, r->U, kCombine, 0.5, 0.5, 1, act))) return e;
-        k_stage_max<<<1, 1024, 0, r->stream>>>(c, act, 1, r->bm[1], r->nb, r->bmv[1], nbv);
-        if (r->ibm && (e = ibm_fill(r, r->U, r->U, 1, act))) return e;
-        k_end_rk<<<1, 1, 0, r->stream>>>(c, 2);
-        return cudaGetLastError();
+        if ((e = residual_stage(r, r->Ut, r->U, r->U, kCombine, 0.5, 0.5, 1, act, nullptr, last))) return e;
+        if (!fold) k_stage_max<<<1, 1024, 0, r->stream>>>(c, act, 1, r->bm[1], r->nb, r->bmv[1], nbv);
+    } else {
+        if ((e = residual_stage(r, r->Ut, r->U, r->R, kCombine, 0.75, 0.25, 1, act, nullptr, fold ? kFinMax : kFinNone))) return e;
+        if (!fold) k_stage_max<<<1, 1024, 0, r->stream>>>(c, act, 1, r->bm[1], r->nb, r->bmv[1], nbv);
+        if ((e = residual_stage(r, r->R, r->U, r->U, kCombine, 1.0 / 3.0, 2.0 / 3.0, 2, act, nullptr, last))) return e;
+        if (!fold) k_stage_max<<<1, 1024, 0, r->stream>>>(c, act, 2, r->bm[2], r->nb, r->bmv[2], nbv);
     }
-    if ((e = residual_stage(r, r->Ut, r->U, r->R, kCombine, 0.75, 0.25, 1, act))) return e;
-    k_stage_max<<<1, 1024, 0, r->stream>>>(c, act, 1, r->bm[1], r->nb, r->bmv[1], nbv);
-    if ((e = residual_stage(r, r->R, r->U, r->U, kCombine, 1.0 / 3.0, 2.0 / 3.0, 2, act))) return e;
-    k_stage_max<<<1, 1024, 0, r->stream>>>(c, act, 2, r->bm[2], r->nb, r->bmv[2], nbv);
     if (r->ibm && (e = ibm_fill(r, r->U, r->U, 1, act))) return e;
-    k_end_rk<<<1, 1, 0, r->stream>>>(c, 3);
+    if (!fold)
+        k_end_rk<<<1, 1, 0, r->stream>>>(c, nstages);
+    else if (r->ibm)
+        k_end_folded<<<1, 1, 0, r->stream>>>(c, 0);
+    return cudaGetLastError();
+}
+
+// Before the first MUSCL-Hancock step of a call: the lagged speed, seeded with one plain residual (its viscous bound
+// included) when there is none yet, and the step's dt; each step then sets the next one's.
+cudaError_t hancock_start(fvg_run* r) {
+    cudaError_t e;
+    Ctl* c = r->ctl;
+    double* Uin = r->Ucur();
+    const int nbv = r->cfg.use_viscous ? r->nbv : 0;
+    k_hancock_begin<<<1, 1, 0, r->stream>>>(c);
+    if ((e = stage_values(r, 0, &c->seed))) return e;
+    if (r->ibm && (e = ibm_fill(r, Uin, nullptr, 0, &c->seed))) return e;
+    if ((e = massflow_targets(r, Uin, &c->seed))) return e;
+    if (r->cfg.use_viscous && (e = launch_visc(r, Uin, r->bmv[1], &c->seed, false))) return e;
+    if ((e = r->stage.launch(stage_args(r, Uin, nullptr, r->R, kStoreR, 0, 0, r->cfg.use_viscous ? r->Rv : nullptr, r->bm_seed, &c->seed), r->nb,
+                             r->stream)))
+        return e;
+    k_hancock_seed<<<1, 1024, 0, r->stream>>>(c, r->bm_seed, r->nb, r->bmv[1], nbv);
+    k_hancock_dt<<<1, 1, 0, r->stream>>>(c);
     return cudaGetLastError();
 }
 
@@ -2366,7 +2378,7 @@ static int ctl_status(fvg_run* run, const Ctl& h, int done) {
     }
     if (h.status) {
         char msg[256];
-        std::snprintf(msg, sizeof msg, "the solution diverged at step %d (t = %.6g, dt = %.3g, largest wave speed = %.3g)", done + 1, h.t, h.dt,
+        std::snprintf(msg, sizeof msg, "the solution diverged at step %d (t = %.6g, dt = %.3g, largest wave speed = %.3g)", done + 1, h.t, h.dt_step,
                       h.s_step);
         return fail(run, FVG_ERR_DIVERGED, msg);
     }
@@ -2381,13 +2393,20 @@ static int run_steps(fvg_run* run, double t_end, int max_steps, int use_graph, i
     int rc;
     const bool hancock = run->cfg.time_scheme == FVG_TS_HANCOCK;
     int done = 0;
+    // (a moving body is placed before the first residual is taken)
+    auto start = [&]() -> int {
+        if (!hancock) return FVG_OK;
+        const cudaError_t e = hancock_start(run);
+        return e == cudaSuccess ? FVG_OK : fail(run, FVG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
+    };
+    if (!run->moving && (rc = start())) return rc;
     if (run->moving) {
         // a moving body: step by step, the body placed at the start of each step from the device's clock, the distance
         // it travelled checked after it (at most one cell per step, SimulationRun.cpp:449-458)
         while (true) {
             if ((rc = read_ctl(run, &h))) return rc;
             if (!h.active) break;
-            if ((rc = place_body(run, h.t))) return rc;
+            if ((rc = place_body(run, h.t)) || (h.steps == 0 && (rc = start()))) return rc;
             cudaError_t e = enqueue_step(run);
             if (e != cudaSuccess) return fail(run, FVG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
             Ctl h2;
@@ -2399,10 +2418,10 @@ static int run_steps(fvg_run* run, double t_end, int max_steps, int use_graph, i
             }
             const fvg_config& c = run->cfg;
             const double wv[3] = {run->dynamic ? run->body.u : c.ibm_vx, run->dynamic ? run->body.v : c.ibm_vy, run->dynamic ? run->body.w : c.ibm_vz};
-            double travel = h2.dt * vmax(fabs(wv[0]) / run->m.dx, fabs(wv[1]) / run->m.dy);
-            if (run->dim == 3) travel = vmax(travel, h2.dt * fabs(wv[2]) / run->m.dz);
+            double travel = h2.dt_step * vmax(fabs(wv[0]) / run->m.dx, fabs(wv[1]) / run->m.dy);
+            if (run->dim == 3) travel = vmax(travel, h2.dt_step * fabs(wv[2]) / run->m.dz);
             if (c.ibm_inertia > 0.0) {   // a driven rotation: how far the section's farthest vertex moves (0 for a circle or sphere)
-                const double turn = h2.dt * fabs(run->body.om) * run->reach / vmin(run->m.dx, run->m.dy);
+                const double turn = h2.dt_step * fabs(run->body.om) * run->reach / vmin(run->m.dx, run->m.dy);
                 travel = (c.ibm_cm_x != 0.0 || c.ibm_cm_y != 0.0) ? travel + turn : vmax(travel, turn);
             }
             if (travel > 1.0) {
@@ -2419,7 +2438,7 @@ static int run_steps(fvg_run* run, double t_end, int max_steps, int use_graph, i
                 b.fz = L[3];
                 b.mx = L[4];
                 b.my = L[5];
-                advance_body(run, h2.dt);
+                advance_body(run, h2.dt_step);
             }
             h = h2;
         }
@@ -2478,9 +2497,15 @@ static int run_steps(fvg_run* run, double t_end, int max_steps, int use_graph, i
         const int per_graph = run->sens ? run->sens_every : 2;
         int chunk = 4, ran = 0;
         while (true) {
-            const int n = max_steps > 0 ? std::max(1, std::min(chunk, (max_steps - ran + per_graph - 1) / per_graph)) : chunk;
+            // the last clock read says how far t_end is, in steps of its length: with a step limit nearer than that,
+            // everything up to the limit is launched at once (a 20-step call of a 256^2 run waited twice for the clock)
+            const int need = max_steps > 0 ? (max_steps - ran + per_graph - 1) / per_graph : chunk;
+            const bool far = max_steps > 0 && run->clock_dt > 0.0 && t_end - run->clock_t > 2.0 * (max_steps - ran) * run->clock_dt;
+            const int n = std::max(1, std::min(far ? 64 : chunk, need));
             for (int k = 0; k < n; ++k) CK(cudaGraphLaunch(graph, run->stream));
             if ((rc = read_ctl(run, &h))) return rc;
+            run->clock_t = h.t;
+            run->clock_dt = h.dt_step;
             if (!h.active) break;
             ran = h.steps;
             if (chunk < 64) chunk *= 2;
@@ -2501,7 +2526,7 @@ int fvg_step(fvg_run* run, double t_end, double* dt, double* smax) {
     Ctl h;
     int r2 = read_ctl(run, &h);
     if (r2) return r2;
-    if (dt) *dt = n ? h.dt : 0.0;
+    if (dt) *dt = n ? h.dt_step : 0.0;
     if (smax) *smax = n ? h.s_step : 0.0;
     return FVG_OK;
 }

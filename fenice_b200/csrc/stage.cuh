@@ -40,7 +40,8 @@ struct StageArgs {
     // the 3-D mixed form's viscous balance sums instead (FP32, the planes rho u .. rho w after the density's, whose
     // viscous term is 0): the viscous residual is each sum widened to FP64 times 1 / volume (null: none)
     const float* Rvf;
-    double* blockmax;           // per-CTA largest wave speed
+    double* blockmax;           // per-CTA largest wave speed (fin.kind == kFinNone)
+    Fin fin;                    // or what is done with it
     const Ctl* ctl;             // dt
     const int* gate;            // the kernel does nothing unless *gate (the control block's `active` or `seed`)
     int tiles[3];               // tiles per axis
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
         }
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 }   // namespace fvg

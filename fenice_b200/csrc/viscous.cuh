@@ -33,7 +33,8 @@ struct ViscArgs {
     const double* U;
     double* Rv;
     float* Rvf;        // the 3-D mixed form: the FP32 viscous balance sums of the planes 1 .. 4 (StageArgs::Rvf)
-    double* blockmax;
+    double* blockmax;  // per-CTA largest speed bound, or
+    Fin fin;           // folded into the control block (kFinMax)
     const int* gate;   // the kernel does nothing unless *gate
     int tiles[3];
     int b0;            // the tile of the launch's first CTA (a launch over a range of tiles; 0: all)
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
         if (s > smax) smax = s;
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 }   // namespace fvg
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(NT) viscous2d_kernel(const ViscArgs a) {
         if (s > smax) smax = s;
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) a.blockmax[b] = bm;
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
 }   // namespace fvg
