@@ -443,9 +443,7 @@ int fvg_batch_create(const fvg_config* cfgs, int n, fvg_batch** out) {
         pr.bc.u_in = c.u_in;
         pr.bc.v_in = c.v_in;
         pr.bc.p_out = c.p_out;
-        pr.eos.type = c.eos_type;
-        pr.eos.gamma = c.gamma;
-        pr.eos.p_inf = c.p_inf;
+        set_eos(pr.eos, c.eos_type, c.gamma, c.p_inf);
         pr.shock_blend = c.shock_blend;
         pr.weno_eps = c.weno_epsilon;
         pr.limiter = c.limiter;

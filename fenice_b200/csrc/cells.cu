@@ -974,9 +974,7 @@ int fvg_cells_create(const fvg_config* cfg, int nleaf, const int* level, const i
     }
     e->nface = t.nface;
     e->fplane = (t.nface + 31) / 32 * 32;
-    e->eos.type = c.eos_type;
-    e->eos.gamma = c.gamma;
-    e->eos.p_inf = c.p_inf;
+    set_eos(e->eos, c.eos_type, c.gamma, c.p_inf);
     for (int s = 0; s < 6; ++s) e->bc.type[s] = c.bc[s];
     e->bc.u_in = c.u_in;
     e->bc.v_in = c.v_in;

@@ -43,7 +43,20 @@ template <typename T> __host__ __device__ __forceinline__ T vmin(T a, T b) { ret
 template <typename T> struct Eos {
     int type;
     T gamma, p_inf;
+    T rgm1;   // 1 / (gamma - 1), correctly rounded (0: divide); set by set_eos
 };
+// The gas of a run, on the host. The reciprocal is left out where Markstein's theorem does not cover it (a divisor whose
+// significand is all ones).
+inline void set_eos(Eos<double>& e, int type, double gamma, double p_inf) {
+    e.type = type;
+    e.gamma = gamma;
+    e.p_inf = p_inf;
+    const double d = gamma - 1.0;
+    int ex = 0;
+    const double m = frexp(d, &ex);
+    const bool covered = d > 1e-100 && d < 1e100 && m != 1.0 - 0x1p-53;
+    e.rgm1 = covered ? 1.0 / d : 0.0;
+}
 
 // State of NV components: [rho, rho u, rho v, rho E (, rho w)] or primitive [rho, u, v, p (, w)].
 template <typename T, int NV> struct St {
@@ -52,8 +65,23 @@ template <typename T, int NV> struct St {
     __device__ __forceinline__ const T& operator[](int q) const { return v[q]; }
 };
 
+// x / (gamma - 1), correctly rounded as the division is: the product with the rounded reciprocal, corrected twice by its
+// exact residual (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990: with the
+// correctly rounded reciprocal, one correction of a quotient within one unit in the last place gives the rounded quotient;
+// the first correction brings the product there). Five dependent operations and no branch taken instead of a division; a
+// zero, an infinity, a NaN or a quotient near the limits of the range is divided.
+__device__ __forceinline__ double over_gm1(const Eos<double>& e, double x) {
+    const double d = e.gamma - 1.0;
+    const double q0 = __dmul_rn(x, e.rgm1);
+    const unsigned ex = ((unsigned)__double2hiint(q0) >> 20) & 0x7ffu;
+    if (ex - 123u > 1800u) return x / d;   // |q0| outside 2^-900 .. 2^900 (or no reciprocal: q0 = 0)
+    const double q1 = __fma_rn(__fma_rn(-d, q0, x), e.rgm1, q0);
+    return __fma_rn(__fma_rn(-d, q1, x), e.rgm1, q1);
+}
+template <typename T> __device__ __forceinline__ T over_gm1(const Eos<T>& e, T x) { return x / (e.gamma - T(1)); }
+
 template <typename T> __device__ __forceinline__ T internal_energy(const Eos<T>& e, T p) {
-    return e.type == kIdeal ? p / (e.gamma - T(1)) : (p + e.gamma * e.p_inf) / (e.gamma - T(1));
+    return e.type == kIdeal ? over_gm1(e, p) : over_gm1(e, p + e.gamma * e.p_inf);
 }
 template <typename T> __device__ __forceinline__ T pressure(const Eos<T>& e, T rho_e) {
     return e.type == kIdeal ? (e.gamma - T(1)) * rho_e : (e.gamma - T(1)) * rho_e - e.gamma * e.p_inf;
@@ -242,74 +270,79 @@ __device__ __forceinline__ void weno5z_pair(float c0, float c1, float c2, float 
 // ------------------------------------------------------------------ HLLC (Toro) with Einfeldt bounds (Schemes.cpp:116-200)
 template <typename T> __device__ __forceinline__ T safe_denom(T x) { return copysign(vmax(fabs(x), Num<T>::denom_eps), x); }
 
+// One side's Euler flux along `axis`.
+template <typename T, int NV>
+__device__ __forceinline__ void hllc_side_flux(const St<T, NV>& W, T E, int axis, St<T, NV>& F) {
+    constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
+    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
+    const T rho = W[0], p = W[3], Vn = W[mn];
+    F[0] = rho * Vn;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
+        F[m] = rho * W[m] * Vn;
+    }
+    F[mn] = F[mn] + p;
+    F[3] = Vn * (rho * E + p);
+}
+
 // The flux along `axis` (0, 1, 2) from the primitive (floored) and conservative states of both sides; returns max(|S_L|, |S_R|).
+// The reference forms both sides' fluxes and star states and then takes one of the four by the order of the waves; here the
+// side is chosen first and only its flux and star state are formed, with the same operations (the same bits, three
+// divisions instead of five).
 template <typename T, int NV>
 __device__ __forceinline__ T hllc_core(const St<T, NV>& WL, const St<T, NV>& WR, const St<T, NV>& UL, const St<T, NV>& UR, T inv_L,
                                        T inv_R, T c_L, T c_R, int axis, T shock_blend, St<T, NV>& F) {
     constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
+    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
     const T rho_L = WL[0], p_L = WL[3];
     const T rho_R = WR[0], p_R = WR[3];
-    T vel_L[NA], vel_R[NA];
-    vel_L[0] = WL[1];
-    vel_L[1] = WL[2];
-    vel_R[0] = WR[1];
-    vel_R[1] = WR[2];
-    if constexpr (NA == 3) {
-        vel_L[2] = WL[4];
-        vel_R[2] = WR[4];
-    }
-    const T E_L = UL[3] * inv_L, E_R = UR[3] * inv_R;
-    const T Vn_L = vel_L[axis], Vn_R = vel_R[axis];
-    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
-    St<T, NV> FL, FR;
-    FL[0] = rho_L * Vn_L;
-    FR[0] = rho_R * Vn_R;
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-        FL[m] = rho_L * vel_L[a] * Vn_L;
-        FR[m] = rho_R * vel_R[a] * Vn_R;
-    }
-    FL[mn] = FL[mn] + p_L;
-    FR[mn] = FR[mn] + p_R;
-    FL[3] = Vn_L * (rho_L * E_L + p_L);
-    FR[3] = Vn_R * (rho_R * E_R + p_R);
+    const T Vn_L = WL[mn], Vn_R = WR[mn];
     const T S_L = vmin(Vn_L - c_L, Vn_R - c_R);
     const T S_R = vmax(Vn_L + c_L, Vn_R + c_R);
     const T num = rho_R * Vn_R * (S_R - Vn_R) - rho_L * Vn_L * (S_L - Vn_L) + p_L - p_R;
     const T den = rho_R * (S_R - Vn_R) - rho_L * (S_L - Vn_L);
     const T S_M = num / safe_denom(den);
-    const T den_star_L = safe_denom(S_L - S_M);
-    const T den_star_R = safe_denom(S_R - S_M);
-    const T den_pL = safe_denom(S_L - Vn_L);
-    const T den_pR = safe_denom(S_R - Vn_R);
-    const T fL = rho_L * (S_L - Vn_L) / den_star_L;
-    const T fR = rho_R * (S_R - Vn_R) / den_star_R;
-    St<T, NV> UsL, UsR;
-    UsL[0] = fL;
-    UsR[0] = fR;
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-        UsL[m] = fL * (a == axis ? S_M : vel_L[a]);
-        UsR[m] = fR * (a == axis ? S_M : vel_R[a]);
-    }
-    UsL[3] = fL * (E_L + (S_M - Vn_L) * (S_M + p_L / (rho_L * den_pL)));
-    UsR[3] = fR * (E_R + (S_M - Vn_R) * (S_M + p_R / (rho_R * den_pR)));
-    // flux selection by wave ordering: the four tests in the reference's sequence (a NaN speed leaves F = 0)
+    // flux selection by wave ordering: the last true one of the reference's four tests (a NaN speed leaves F = 0)
+    const bool star_R = S_M < T(0) && S_R >= T(0), star_L = S_L < T(0) && S_M >= T(0);
+    const bool right = S_R < T(0) || star_R;
+    const bool star = !(S_R < T(0)) && (star_R || star_L);
+    const bool none = !right && !star && !(S_L >= T(0));
+    St<T, NV> W, U;
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
-        T f = T(0);
-        if (S_L >= T(0)) f = FL[q];
-        if (S_L < T(0) && S_M >= T(0)) f = FL[q] + S_L * (UsL[q] - UL[q]);
-        if (S_M < T(0) && S_R >= T(0)) f = FR[q] + S_R * (UsR[q] - UR[q]);
-        if (S_R < T(0)) f = FR[q];
-        F[q] = f;
+        W[q] = right ? WR[q] : WL[q];
+        U[q] = right ? UR[q] : UL[q];
     }
+    const T E = U[3] * (right ? inv_R : inv_L);
+    hllc_side_flux(W, E, axis, F);
+    if (star) {
+        const T S = right ? S_R : S_L;
+        const T rho = W[0], p = W[3], Vn = W[mn];
+        const T den_star = safe_denom(S - S_M);
+        const T den_p = safe_denom(S - Vn);
+        const T f = rho * (S - Vn) / den_star;
+        St<T, NV> Us;
+        Us[0] = f;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
+            Us[m] = f * (a == axis ? S_M : W[m]);
+        }
+        Us[3] = f * (E + (S_M - Vn) * (S_M + p / (rho * den_p)));
+#pragma unroll
+        for (int q = 0; q < NV; ++q) F[q] = F[q] + S * (Us[q] - U[q]);
+    }
+    if (none)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) F[q] = T(0);
     if (shock_blend > T(0)) {
         const T s = fabs(p_R - p_L) / vmin(p_L, p_R);
         if (s > shock_blend) {
             const T phi = vmin((s - shock_blend) / shock_blend, T(1));
+            St<T, NV> FL, FR;
+            hllc_side_flux(WL, UL[3] * inv_L, axis, FL);
+            hllc_side_flux(WR, UR[3] * inv_R, axis, FR);
             if (S_L >= T(0)) {
 #pragma unroll
                 for (int q = 0; q < NV; ++q) F[q] = (T(1) - phi) * F[q] + phi * FL[q];

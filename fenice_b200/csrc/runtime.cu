@@ -2043,9 +2043,7 @@ int create_run(const fvg_config* cfg, int nparts, int part, bool as_part, fvg_ru
         m.inv_cell = 1.0 / (m.dx * m.dy);
         run->L = vmin(g.Lx / g.nx, g.Ly / g.ny);
     }
-    run->eos.type = c.eos_type;
-    run->eos.gamma = c.gamma;
-    run->eos.p_inf = c.p_inf;
+    set_eos(run->eos, c.eos_type, c.gamma, c.p_inf);
     for (int s = 0; s < 6; ++s) run->bc.type[s] = c.bc[s];
     halo_kinds(c, c.reconstruction == FVG_RECON_WENO5 ? 3 : 2, run->bc.halo);
     for (int h = 0; h < 2; ++h)
@@ -3334,9 +3332,7 @@ extern "C" int fvg_residual_noalloc(const fvg_config* cfg, const double* U, long
     a.bc.p_out = c.p_out;
     set_body_force(c, a.bc);
     set_nrbc(c, a.bc);
-    a.eos.type = c.eos_type;
-    a.eos.gamma = c.gamma;
-    a.eos.p_inf = c.p_inf;
+    set_eos(a.eos, c.eos_type, c.gamma, c.p_inf);
     a.shock_blend = c.shock_blend;
     a.weno_eps = c.weno_epsilon;
     a.limiter = c.limiter;
