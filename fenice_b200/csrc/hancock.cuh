@@ -38,14 +38,26 @@ struct HancockArgs {
     int tiles[3];
 };
 
+// Tile and threads: 14 x 14 cells and 256 threads, three CTAs per SM. The ring of predicted cells (16 x 16 with its
+// corners) is then one round of the block, the 420 faces of both axes, solved in one pass, are two, and the box of 18 x 18
+// cells two: the kernel is bound by the latency of long FP64 chains, so rounds that leave most of the block idle cost as
+// much as full ones (a 16 x 16 tile with an axis at a time took two rounds for the ring and four for the faces).
 template <int TX, int TY> struct HancockShape {
     static constexpr int PX = TX + 4, PY = TY + 4;   // primitive box
     static constexpr int BX = TX + 2, BY = TY + 2;   // predicted-state box
-    static constexpr int NF = (TX + 1) * TY > TX * (TY + 1) ? (TX + 1) * TY : TX * (TY + 1);
-    // P [4][PX*PY], S [4 states][4][BX*BY], F [4][NF], acc [4][TX*TY], red [32]
-    static constexpr int SMEM_DOUBLES = 4 * PX * PY + 16 * BX * BY + 4 * NF + 4 * TX * TY + 32;
+    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1), NF = NFX + NFY;
+    // P [4][PX*PY], then in its place the fluxes F [4][NF] (x faces, then y faces); S [4 states][4][BX*BY], red [32]
+    static constexpr int PF = PX * PY > NF ? PX * PY : NF;
+    static constexpr int SMEM_DOUBLES = 4 * PF + 16 * BX * BY + 32;
     static constexpr size_t SMEM_BYTES = sizeof(double) * SMEM_DOUBLES;
 };
+
+// phi(a, b) and phi(b, a) of a limiter. Van Leer's and MC are symmetric to the last bit (products, sums and minima of the
+// same operands; a NaN gives 0 both ways); Minmod's minimum orders a NaN and Koren's is not symmetric.
+__device__ __forceinline__ void limiter_both(int l, double a, double b, double& ab, double& ba) {
+    ab = limiter(l, a, b);
+    ba = (l == kVanLeer || l == kMC) ? ab : limiter(l, b, a);
+}
 
 // euler_flux_axis (Schemes.cpp:2137-2141) of a planar state
 __device__ __forceinline__ St<double, 4> euler_flux2(const Eos<double>& e, const St<double, 4>& U, int a) {
@@ -79,15 +91,14 @@ template <int NV> __device__ __forceinline__ St<double, NV> body_source(const Bc
 
 // FULL = false: a run without part interfaces, non-reflecting sides or the body force (their code compiled out)
 template <int RIEMANN, int TX, int TY, int NT, bool FULL = true>
-__global__ void __launch_bounds__(NT) hancock_kernel(const HancockArgs a) {
+__global__ void __launch_bounds__(NT, 3) hancock_kernel(const HancockArgs a) {
     using S = HancockShape<TX, TY>;
     constexpr int PX = S::PX, PY = S::PY, BX = S::BX, BY = S::BY, NB = BX * BY, NP = PX * PY, NC = TX * TY;
     extern __shared__ double smem[];
     double* P = smem;                  // [4][NP]
-    double* Sx = P + 4 * NP;           // [state 0..3: xl, xr, yb, yt][4][NB]
-    double* Fl = Sx + 16 * NB;         // [4][NF]
-    double* acc = Fl + 4 * S::NF;      // [4][NC]
-    double* red = acc + 4 * NC;
+    double* Fl = smem;                 // [4][NF], once the states are formed
+    double* Sx = smem + 4 * S::PF;     // [state 0..3: xl, xr, yb, yt][4][NB]
+    double* red = Sx + 16 * NB;
     if (!*a.gate) return;
     const Mesh& m = a.m;
     const Eos<double>& e = a.eos;
@@ -121,8 +132,10 @@ __global__ void __launch_bounds__(NT) hancock_kernel(const HancockArgs a) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const double cm = P[q * NP + pc - s], c = P[q * NP + pc], cp = P[q * NP + pc + s];
-                wl[q] = c + 0.5 * limiter(a.limiter, c - cm, cp - c);
-                wr[q] = c - 0.5 * limiter(a.limiter, cp - c, c - cm);
+                double up, down;
+                limiter_both(a.limiter, c - cm, cp - c, up, down);
+                wl[q] = c + 0.5 * up;
+                wr[q] = c - 0.5 * down;
             }
             st[2 * ax + 1] = p2c(e, wl);
             st[2 * ax] = p2c(e, wr);
@@ -179,75 +192,73 @@ __global__ void __launch_bounds__(NT) hancock_kernel(const HancockArgs a) {
     }
     __syncthreads();
     double smax = 0.0;
-    // ---- 3. faces: axis 0 (x), then axis 1 (y)
-#pragma unroll 1
-    for (int axis = 0; axis < 2; ++axis) {
-        const int FX = TX + (axis == 0), FY = TY + (axis == 1);
-        const int nF = FX * FY;
+    // ---- 3. the faces of both axes. The velocity normal to the face is put in slot 1, so that one code serves both axes
+    // (u u + v v does not depend on the order of its two terms).
+    for (int f = tid; f < S::NF; f += NT) {
+        const int axis = f < S::NFX ? 0 : 1;
+        const int r = axis == 0 ? f : f - S::NFX, FX = axis == 0 ? TX + 1 : TX;
+        const int fi = r % FX, fj = r / FX;
         const int lo_side = 2 * axis, hi_side = lo_side + 1;
-        const bool wall_lo = a.bc.type[lo_side] == kBcWall || a.bc.type[lo_side] == kBcNoSlip || a.bc.type[lo_side] == kBcMovingWall;
-        const bool wall_hi = a.bc.type[hi_side] == kBcWall || a.bc.type[hi_side] == kBcNoSlip || a.bc.type[hi_side] == kBcMovingWall;
-        for (int f = tid; f < nF; f += NT) {
-            const int fi = f % FX, fj = f / FX;
-            const int gi = ox + fi, gj = oy + fj;
-            const int n_a = axis == 0 ? nx : ny, t = axis == 0 ? gi : gj;
-            const bool inside = axis == 0 ? (gi <= nx && gj < ny) : (gi < nx && gj <= ny);
-            St<double, 4> F;
+        const int gi = ox + fi, gj = oy + fj;
+        const int n_a = axis == 0 ? nx : ny, t = axis == 0 ? gi : gj;
+        const bool inside = axis == 0 ? (gi <= nx && gj < ny) : (gi < nx && gj <= ny);
+        St<double, 4> F;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) F[q] = 0.0;
-            if (inside) {
-                // the cells before and after the face in the state box
-                const int pR = (fj + 1) * BX + (fi + 1);
-                const int pL = axis == 0 ? pR - 1 : pR - BX;
-                const int sL = axis == 0 ? 1 : 3, sR = axis == 0 ? 0 : 2;   // high-side state of L, low-side state of R
-                St<double, 4> UL, UR;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    UL[q] = Sx[(sL * 4 + q) * NB + pL];
-                    UR[q] = Sx[(sR * 4 + q) * NB + pR];
-                }
-                if (t == 0) {
-                    if (wall_lo)
-                        UL = ghost_state(e, a.bc, lo_side, UR);
-                    else if (a.bc.halo[lo_side] == kHaloNone)
-                        UL = round_trip(e, side_ghost<4, FULL>(m, a.bc, e, a.U, lo_side, gi, gj, 0));
-                }
-                if (t == n_a) {
-                    const int ci = axis == 0 ? nx - 1 : gi, cj = axis == 0 ? gj : ny - 1;
-                    if (wall_hi)
-                        UR = ghost_state(e, a.bc, hi_side, UL);
-                    else if (a.bc.halo[hi_side] == kHaloNone)
-                        UR = round_trip(e, side_ghost<4, FULL>(m, a.bc, e, a.U, hi_side, ci, cj, 0));
-                }
-                const double s = face_flux<RIEMANN>(e, a.shock_blend, UL, UR, axis, F);
-                if (s > smax) smax = s;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) Fl[q * S::NF + f] = F[q];
-        }
-        __syncthreads();
-        const double A = m.area[axis];
-        for (int c = tid; c < NC; c += NT) {
-            const int ci = c % TX, cj = c / TX;
-            const int fl = cj * FX + ci, fr = fl + (axis == 0 ? 1 : FX);
+        for (int q = 0; q < 4; ++q) F[q] = 0.0;
+        if (inside) {
+            // the cells before and after the face in the state box
+            const int pR = (fj + 1) * BX + (fi + 1);
+            const int pL = axis == 0 ? pR - 1 : pR - BX;
+            const int sL = axis == 0 ? 1 : 3, sR = axis == 0 ? 0 : 2;   // high-side state of L, low-side state of R
+            St<double, 4> UL, UR;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const double dd = Fl[q * S::NF + fr] * A - Fl[q * S::NF + fl] * A;
-                acc[q * NC + c] = axis == 0 ? 0.0 - dd : acc[q * NC + c] - dd;
+                UL[q] = Sx[(sL * 4 + q) * NB + pL];
+                UR[q] = Sx[(sR * 4 + q) * NB + pR];
             }
+            if (t == 0) {
+                if (a.bc.type[lo_side] == kBcWall || a.bc.type[lo_side] == kBcNoSlip || a.bc.type[lo_side] == kBcMovingWall)
+                    UL = ghost_state(e, a.bc, lo_side, UR);
+                else if (a.bc.halo[lo_side] == kHaloNone)
+                    UL = round_trip(e, side_ghost<4, FULL>(m, a.bc, e, a.U, lo_side, gi, gj, 0));
+            }
+            if (t == n_a) {
+                const int ci = axis == 0 ? nx - 1 : gi, cj = axis == 0 ? gj : ny - 1;
+                if (a.bc.type[hi_side] == kBcWall || a.bc.type[hi_side] == kBcNoSlip || a.bc.type[hi_side] == kBcMovingWall)
+                    UR = ghost_state(e, a.bc, hi_side, UL);
+                else if (a.bc.halo[hi_side] == kHaloNone)
+                    UR = round_trip(e, side_ghost<4, FULL>(m, a.bc, e, a.U, hi_side, ci, cj, 0));
+            }
+            if (axis == 1) {
+                const double l = UL[1], r1 = UR[1];
+                UL[1] = UL[2];
+                UL[2] = l;
+                UR[1] = UR[2];
+                UR[2] = r1;
+            }
+            const double s = face_flux<RIEMANN>(e, a.shock_blend, UL, UR, 0, F);
+            if (s > smax) smax = s;
         }
-        __syncthreads();
+        Fl[f] = F[0];
+        Fl[(1 + axis) * S::NF + f] = F[1];
+        Fl[(2 - axis) * S::NF + f] = F[2];
+        Fl[3 * S::NF + f] = F[3];
     }
-    // ---- 4. the residual and the update
-    const double dt = a.ctl->dt;
+    __syncthreads();
+    // ---- 4. the balance, the residual and the update
+    const double dt = a.ctl->dt, Ax = m.area[0], Ay = m.area[1];
     for (int c = tid; c < NC; c += NT) {
-        const int gi = ox + c % TX, gj = oy + c / TX;
+        const int ci = c % TX, cj = c / TX;
+        const int gi = ox + ci, gj = oy + cj;
         if (gi >= nx || gj >= ny) continue;
         const long long cell = (long long)gj * nx + gi;
+        const int fx = cj * (TX + 1) + ci, fy = S::NFX + c;
         St<double, 4> r;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            r[q] = acc[q * NC + c] * m.inv_cell;
+            const double* Fq = Fl + q * S::NF;
+            const double dx = Fq[fx + 1] * Ax - Fq[fx] * Ax, dy = Fq[fy + TX] * Ay - Fq[fy] * Ay;
+            r[q] = ((0.0 - dx) - dy) * m.inv_cell;
             if (a.Rv) r[q] = r[q] + a.Rv[q * m.plane + cell];
         }
         if (FULL && (a.bc.grav_on || a.bc.src)) {

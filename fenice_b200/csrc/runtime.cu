@@ -569,19 +569,20 @@ cudaError_t launch_viscous2d(const ViscArgs& a, int nblocks, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// MUSCL-Hancock tiles: 16 x 16 in 2-D, 8 x 8 x 4 in 3-D (93 KB of shared memory: two CTAs per SM); FULL as the stage kernels
+// MUSCL-Hancock tiles: 14 x 14 in 2-D, 8 x 8 x 4 in 3-D (93 KB of shared memory: two CTAs per SM); FULL as the stage kernels
+constexpr int kHancock2T = 14;
 template <int RIEMANN, bool FULL> cudaError_t prepare_hancock_t(int dim) {
     if (dim == 3)
         return cudaFuncSetAttribute(hancock3d_kernel<RIEMANN, 8, 8, 4, 256, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)Hancock3Shape<8, 8, 4>::SMEM_BYTES);
-    return cudaFuncSetAttribute(hancock_kernel<RIEMANN, 16, 16, 256, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)HancockShape<16, 16>::SMEM_BYTES);
+    return cudaFuncSetAttribute(hancock_kernel<RIEMANN, kHancock2T, kHancock2T, 256, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)HancockShape<kHancock2T, kHancock2T>::SMEM_BYTES);
 }
 template <int RIEMANN, bool FULL> cudaError_t launch_hancock_t(int dim, const HancockArgs& a, int nblocks, cudaStream_t s) {
     if (dim == 3)
         hancock3d_kernel<RIEMANN, 8, 8, 4, 256, FULL><<<nblocks, 256, Hancock3Shape<8, 8, 4>::SMEM_BYTES, s>>>(a);
     else
-        hancock_kernel<RIEMANN, 16, 16, 256, FULL><<<nblocks, 256, HancockShape<16, 16>::SMEM_BYTES, s>>>(a);
+        hancock_kernel<RIEMANN, kHancock2T, kHancock2T, 256, FULL><<<nblocks, 256, HancockShape<kHancock2T, kHancock2T>::SMEM_BYTES, s>>>(a);
     return cudaGetLastError();
 }
 cudaError_t prepare_hancock(int riemann, bool full, int dim) {
@@ -2068,7 +2069,7 @@ int create_run(const fvg_config* cfg, int nparts, int part, bool as_part, fvg_ru
     run->ntiles_v[1] = (c.ny + vt - 1) / vt;
     run->ntiles_v[2] = run->dim == 3 ? (c.nz + 7) / 8 : 1;
     run->nbv = run->ntiles_v[0] * run->ntiles_v[1] * run->ntiles_v[2];
-    const int hx = run->dim == 3 ? 8 : 16, hz = run->dim == 3 ? 4 : 1;   // MUSCL-Hancock tiles
+    const int hx = run->dim == 3 ? 8 : kHancock2T, hz = run->dim == 3 ? 4 : 1;   // MUSCL-Hancock tiles
     run->ntiles_h[0] = (c.nx + hx - 1) / hx;
     run->ntiles_h[1] = (c.ny + hx - 1) / hx;
     run->ntiles_h[2] = (c.nz + hz - 1) / hz;
