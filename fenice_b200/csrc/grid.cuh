@@ -36,7 +36,7 @@ struct Ctl {
     int steps, max_steps;
     int status;         // 0 ok; 1 the solution diverged (non-finite speed or dt, or t no longer advances); 3 a
                         // time-dependent boundary value was not finite, or rho_in or p_out not positive, at a stage time;
-                        // 5 a TMA copy of a stage tile, 6 a tensor-core step of the sensor did not complete (a bounded wait gave up)
+                        // 6 a tensor-core step of the sensor did not complete (a bounded wait gave up)
     unsigned ticket;    // CTAs of the running stage launch that are done (stage_finish)
     unsigned long long s_bits;   // the largest speed so far, as the bits of a non-negative double
 };

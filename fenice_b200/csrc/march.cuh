@@ -1,0 +1,361 @@
+// The mixed-precision WENO5-Z stage kernel of a 3-D mesh: a CTA owns 32 x 8 columns of cells and marches along z.
+//
+// The arithmetic of mixed.cuh (the same functions, so the same bits as mixed_stage_kernel, which parts of a decomposed
+// mesh and meshes with first-order sides keep), in an order that forms each thing once:
+// - the primitive state of a cell is recovered once as its plane arrives and once more where the cell lies beside another
+//   CTA's columns (1.9 recoveries per cell; an 8x8x8 tile with its three halos takes 3.25);
+// - a thread keeps the six planes of its column around its z face in registers; the plane being solved lies in shared
+//   memory with three cells around the columns, for the x and y faces (rows of 40 floats: a warp reads 32 neighbours of
+//   one row, no two on a bank);
+// - per plane a thread solves its low x, its low y and its high z face in one loop whose body is the only copy of the
+//   reconstruction and the Riemann solver (a copy per axis would not fit the instruction cache); a ninth warp solves the
+//   40 faces on the high sides of the columns;
+// - fluxes meet in shared memory, and the balance ((0 - x) - y) - z and the FP64 update finish the plane.
+// All global operands of a plane (the raw state three planes ahead, the raw halo of the next plane, U, U0 and the viscous
+// sums of the cell) are on their way to shared memory (cp.async, each thread its own values, so no barrier) while the plane
+// before is solved. Two CTAs per SM (288 threads, at most 112 registers, 87 KB of shared memory).
+//
+// What bounds it: instruction issue at 16 to 18 warps per SM (ncu at 192^3: 58 warp instructions per cell, issue 59 %, DRAM 18 %;
+// the tiled form with boxes by TMA took 80). Against that form, mixed + sensor at 256^3: 7.29 -> 7.17 ms per step; mixed at 64^3:
+// 225 -> 209 us per step.
+#pragma once
+
+#include "mixed.cuh"
+
+namespace fvg {
+
+struct MarchShape {
+    static constexpr int W = 32, H = 8, NT = 288, NCOL = W * H;
+    static constexpr int PITCH = 40, PL = 14 * PITCH;             // a plane of P: rows y = -3 .. 10, x = -3 .. 34
+    static constexpr int NHALO = 6 * W + 6 * H;                    // cells around the columns
+    static constexpr int FXP = 36, NFX = H * FXP, NFY = (H + 1) * W;
+    // doubles: red [32], the raw values on their way: core [5][256], halo [5][256], u [5][256], u0 [5][256]; then floats:
+    // the viscous sums [4][256], P [5][PL], FX [5][NFX], FY [5][NFY], FZ [2][5][256]
+    static constexpr size_t SMEM_BYTES = 8 * (32 + 20 * NCOL) + 4 * (4 * NCOL + 5 * PL + 5 * NFX + 5 * NFY + 10 * NCOL);
+};
+
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The cell a stencil position g along an axis reads, and the side whose ghost-slab rule applies to it (-1: none); the rules
+// of stencil_cons for one axis.
+__device__ __forceinline__ int march_cell(const Bc& bc, int axis, int g, int n, int& side) {
+    side = -1;
+    if (g >= 0 && g < n) return g;
+    const bool hi = g >= n;
+    const int kind = bc.halo[2 * axis + (hi ? 1 : 0)];
+    if (kind == kHaloWrap) return ((g % n) + n) % n;
+    if (kind == kHaloSlab) {
+        side = 2 * axis + (hi ? 1 : 0);
+        const int l0 = hi ? g - n : -1 - g, l = l0 < n ? l0 : n - 1;
+        return hi ? n - 1 - l : l;
+    }
+    return hi ? n - 1 : 0;
+}
+
+// z0 .. z1: the planes of the launch; lz: planes per CTA (a multiple of 8 where the CTAs write blockmax). GATED: a face is
+// linear when the tiles of both its cells are linear along its axis (inside a tile: when the tile is), which is the seam
+// rule of mixed_axis face by face.
+template <int RIEMANN, bool GATED>
+__global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const StageArgs a, const int z0, const int z1, const int lz, const int nslots) {
+    using S = MarchShape;
+    constexpr int NV = 5, PL = S::PL, NCOL = S::NCOL;
+    extern __shared__ double smem_d[];
+    double* red = smem_d;
+    double* Rc = smem_d + 32;        // raw state of the column, three planes ahead
+    double* Rh = Rc + 5 * NCOL;      // raw halo of the next plane
+    double* Ru = Rh + 5 * NCOL;      // U of the cell
+    double* R0 = Ru + 5 * NCOL;      // U0 of the cell
+    float* Rv = reinterpret_cast<float*>(R0 + 5 * NCOL);
+    float* P = Rv + 4 * NCOL;        // [rho, u, v, p, w][PL]
+    float* FX = P + 5 * PL;          // [5][NFX]
+    float* FY = FX + 5 * S::NFX;     // [5][NFY]
+    float* FZ = FY + 5 * S::NFY;     // [2][5][256]: the z faces below and above the plane, by turns
+    if (!*a.gate) return;
+    const Mesh& m = a.m;
+    const GasF gas = gas_f(a.eos);
+    const float sb = (float)a.shock_blend, weps = (float)a.weno_eps;
+    const int tid = threadIdx.x;
+    const int cx = (m.nx + S::W - 1) / S::W, cy = (m.ny + S::H - 1) / S::H;
+    const int cta = blockIdx.x;
+    const int x0 = (cta % cx) * S::W, y0 = ((cta / cx) % cy) * S::H, za = z0 + (cta / (cx * cy)) * lz;
+    const int zb = za + lz < z1 ? za + lz : z1;
+    const bool col = tid < NCOL;
+    const int tx = tid & 31, ty = tid >> 5;             // (the ninth warp: ty = 8)
+    const int gx = x0 + tx, gy = y0 + ty;
+    const bool cell_in = col && gx < m.nx && gy < m.ny;
+    const long long zs = (long long)m.nx * m.ny;
+
+    // the thread's column and its halo cell: what they read, and the side whose ghost rule they follow
+    int cside, hside = -1, hslot = -1;
+    long long coff, hoff = 0;
+    {
+        int sx, sy;
+        const int ix = march_cell(a.bc, 0, gx, m.nx, sx), iy = march_cell(a.bc, 1, gy, m.ny, sy);
+        coff = (long long)iy * m.nx + ix;
+        cside = sx >= 0 ? sx : sy;
+        if (tid < S::NHALO) {
+            int hx, hy;
+            if (tid < 6 * S::W) {
+                const int r = tid >> 5;
+                hx = tid & 31;
+                hy = r < 3 ? r - 3 : S::H + r - 3;
+            } else {
+                const int r = tid - 6 * S::W, s = r % 6;
+                hy = r / 6;
+                hx = s < 3 ? s - 3 : S::W + s - 3;
+            }
+            const int jx = march_cell(a.bc, 0, x0 + hx, m.nx, sx), jy = march_cell(a.bc, 1, y0 + hy, m.ny, sy);
+            hoff = (long long)jy * m.nx + jx;
+            hside = sx >= 0 ? sx : sy;
+            hslot = (hy + 3) * S::PITCH + hx + 3;
+        }
+    }
+    const int pslot = (ty + 3) * S::PITCH + tx + 3;     // the column in a plane of P
+    auto prim = [&](const double* raw, long long stride, int side) {
+        St<double, NV> u;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) u[q] = raw[q * stride];
+        if (side >= 0) u = ghost_state(a.eos, a.bc, side, u);
+        double inv;
+        return prim_d(a.eos, u, inv);
+    };
+    auto fetch_core = [&](int g) {   // the column's raw state of plane g
+        int sz;
+        const double* src = a.U + march_cell(a.bc, 2, g, m.nz, sz) * zs + coff;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * NCOL + tid, src + q * m.plane);
+    };
+    auto core_side = [&](int g) {
+        int sz;
+        march_cell(a.bc, 2, g, m.nz, sz);
+        return sz >= 0 ? sz : cside;
+    };
+    auto fetch_halo = [&](int g) {
+        const double* src = a.U + g * zs + hoff;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) cp_async8(Rh + q * NCOL + tid, src + q * m.plane);
+    };
+    auto fetch_cell = [&](int g) {   // the operands of the cell's update
+        const long long cell = g * zs + coff;
+        if (a.mode != kStoreR)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(Ru + q * NCOL + tid, a.U + q * m.plane + cell);
+        if (a.mode == kCombine)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(R0 + q * NCOL + tid, a.U0 + q * m.plane + cell);
+        if (a.Rvf)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) cp_async4(Rv + q * NCOL + tid, a.Rvf + q * m.plane + cell);
+    };
+    // GATED: whether the tile of the cell at (x, y, z) is linear along an axis (a cell beyond a wrapped side: the wrapped
+    // cell's; beyond another side no tile, and the tiles beside it are kept WENO5-Z by the gate)
+    auto tile_linear = [&](int axis, int x, int y, int z) -> bool {
+        int p[3] = {x, y, z};
+        const int n3[3] = {m.nx, m.ny, m.nz};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (p[d] >= 0 && p[d] < n3[d]) continue;
+            if (a.bc.halo[2 * d + (p[d] < 0 ? 0 : 1)] != kHaloWrap) return true;
+            p[d] = ((p[d] % n3[d]) + n3[d]) % n3[d];
+        }
+        const long long t = ((long long)(p[2] >> 3) * a.tiles[1] + (p[1] >> 3)) * a.tiles[0] + (p[0] >> 3);
+        return a.sens_flags[(long long)axis * a.tiles[0] * a.tiles[1] * a.tiles[2] + t] == 0;
+    };
+    const int fx = col ? tx : S::W, fy = col ? ty : (tx < S::H ? tx : 0);   // the thread's x face: its low one, or the ninth warp's
+
+    if (col) fetch_core(za + 3);
+    if (hslot >= 0) fetch_halo(za);
+    if (cell_in) fetch_cell(za);
+    // the column's planes k - 2 .. k + 3 in registers ([variable][plane]), from k = za - 1
+    float r[NV][6];
+    if (col) {
+#pragma unroll
+        for (int p = 0; p < 6; ++p) {
+            int sz;
+            const double* src = a.U + march_cell(a.bc, 2, za - 3 + p, m.nz, sz) * zs + coff;
+            const St<double, NV> w = prim(src, m.plane, sz >= 0 ? sz : cside);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) r[q][p] = (float)w[q];
+        }
+    }
+    const float Ax = (float)m.area[0], Ay = (float)m.area[1], Az = (float)m.area[2];
+    const double dt = a.ctl->dt;
+    float smax = 0.0f;
+    int lin = 0;   // bit 0, 1, 2: the thread's x, y and z faces are linear
+    // k = za - 1: only the z faces below the first plane
+#pragma unroll 1
+    for (int k = za - 1; k < zb; ++k) {
+        const bool first = k < za;
+        if (!first) {
+            cp_async_wait();
+            if (col) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q)
+#pragma unroll
+                    for (int p = 0; p < 5; ++p) r[q][p] = r[q][p + 1];
+                const St<double, NV> w = prim(Rc + tid, NCOL, core_side(k + 3));
+#pragma unroll
+                for (int q = 0; q < NV; ++q) {
+                    r[q][5] = (float)w[q];
+                    P[q * PL + pslot] = r[q][2];
+                }
+            }
+            if (hslot >= 0) {
+                const St<double, NV> w = prim(Rh + tid, NCOL, hside);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) P[q * PL + hslot] = (float)w[q];
+            }
+            if (k + 1 < zb) {
+                if (col) fetch_core(k + 4);
+                if (hslot >= 0) fetch_halo(k + 1);
+            }
+        }
+        if constexpr (GATED) {
+            if (k <= za || (k & 7) == 0 || (k & 7) == 7) {
+                const int xf = x0 + fx, yf = y0 + fy;
+                lin = (tile_linear(0, xf - 1, yf, k) && tile_linear(0, xf, yf, k) ? 1 : 0) |
+                      (tile_linear(1, gx, gy - 1, k) && tile_linear(1, gx, gy, k) ? 2 : 0) |
+                      (tile_linear(2, gx, gy, k) && tile_linear(2, gx, gy, k + 1) ? 4 : 0);
+            }
+        }
+        __syncthreads();
+        // ---- the faces: x (the low side of the cell), y (low), z (high)
+#pragma unroll 1
+        for (int it = first ? 2 : 0; it < 3; ++it) {
+            float c[NV][6];   // rho, p, the normal velocity, the other two in cyclic order
+            bool on, inside;
+            if (it == 2) {
+                on = col && gy < m.ny;
+                inside = cell_in;
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    c[0][p] = r[0][p];
+                    c[1][p] = r[3][p];
+                    c[2][p] = r[4][p];
+                    c[3][p] = r[1][p];
+                    c[4][p] = r[2][p];
+                }
+            } else if (it == 1) {
+                on = gy <= m.ny;
+                inside = gx < m.nx && gy <= m.ny;
+                const float* b = P + ty * S::PITCH + tx + 3;
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    c[0][p] = b[p * S::PITCH];
+                    c[1][p] = b[3 * PL + p * S::PITCH];
+                    c[2][p] = b[2 * PL + p * S::PITCH];
+                    c[3][p] = b[4 * PL + p * S::PITCH];
+                    c[4][p] = b[1 * PL + p * S::PITCH];
+                }
+            } else {
+                on = (col || tx < S::H) && y0 + fy < m.ny;
+                inside = x0 + fx <= m.nx && y0 + fy < m.ny;
+                const float* b = P + (fy + 3) * S::PITCH + fx;
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    c[0][p] = b[p];
+                    c[1][p] = b[3 * PL + p];
+                    c[2][p] = b[1 * PL + p];
+                    c[3][p] = b[2 * PL + p];
+                    c[4][p] = b[4 * PL + p];
+                }
+            }
+            if (!on) continue;
+            float L[NV], R[NV];
+            if (GATED && (lin >> it & 1)) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) lin5_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], L[q], R[q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) weno5z_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], weps, L[q], R[q]);
+            }
+            float vL[3] = {L[2], L[3], L[4]}, vR[3] = {R[2], R[3], R[4]}, Fm, Fe, Fv[3];
+            const float s = riemann_f<RIEMANN>(gas, sb, L[0], L[1], vL, R[0], R[1], vR, Fm, Fe, Fv);
+            if (inside && s > smax) smax = s;
+            float* dst = it == 0 ? FX + fy * S::FXP + fx : (it == 1 ? FY + tid : FZ + (k & 1) * 5 * NCOL + tid);
+            const int st = it == 0 ? S::NFX : (it == 1 ? S::NFY : NCOL);
+            const int n = it == 0 ? 1 : (it == 1 ? 2 : 4), t1 = it == 0 ? 2 : (it == 1 ? 4 : 1), t2 = it == 0 ? 4 : (it == 1 ? 1 : 2);
+            dst[0] = Fm;
+            dst[3 * st] = Fe;
+            dst[n * st] = Fv[0];
+            dst[t1 * st] = Fv[1];
+            dst[t2 * st] = Fv[2];
+        }
+        __syncthreads();
+        // ---- the balance, the residual widened to FP64 and the FP64 update of plane k
+        if (!first && cell_in) {
+            const long long cell = k * zs + coff;
+            CellIn<NV> in;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                in.u[q] = a.mode != kStoreR ? Ru[q * NCOL + tid] : 0.0;
+                in.u0[q] = a.mode == kCombine ? R0[q * NCOL + tid] : 0.0;
+                in.rv[q] = a.Rvf && q > 0 ? (double)Rv[(q - 1) * NCOL + tid] : 0.0;
+            }
+            const float *X = FX + ty * S::FXP + tx, *Y = FY + tid, *Zh = FZ + (k & 1) * 5 * NCOL + tid, *Zl = FZ + ((k + 1) & 1) * 5 * NCOL + tid;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                float acc = -__fmul_rn(X[q * S::NFX + 1] - X[q * S::NFX], Ax);
+                acc = __fmaf_rn(-(Y[q * S::NFY + S::W] - Y[q * S::NFY]), Ay, acc);
+                acc = __fmaf_rn(-(Zh[q * NCOL] - Zl[q * NCOL]), Az, acc);
+                a.out[q * m.plane + cell] = cell_out(a, in, q, acc, dt);
+            }
+            if (k + 1 < zb) fetch_cell(k + 1);
+        }
+    }
+    const double bm = block_max<S::NT>((double)smax, red);
+    if (tid == 0) {
+        if (a.fin.kind == kFinNone)   // one entry per tile of the launch is read: this CTA's, and its share of the others empty
+            for (int i = cta; i < nslots; i += gridDim.x) a.blockmax[a.b0 + i] = i == cta ? bm : 0.0;
+        else
+            stage_finish(a.fin, nullptr, 0, bm);
+    }
+}
+
+// Whether a launch can march: a lean WENO5-Z run without an immersed body whose every side wraps or has a ghost slab (no
+// first-order boundary faces).
+inline bool can_march(const StageArgs& a) {
+    bool ok = !a.bc.solid && !a.bc.slot;
+    for (int s = 0; s < 6; ++s) ok = ok && (a.bc.halo[s] == kHaloWrap || a.bc.halo[s] == kHaloSlab);
+    return ok;
+}
+// The planes a CTA marches over, for `cols` column blocks and nz planes: the count that gives the fewest rounds of the
+// `resident` CTAs of 148 SMs times the planes of a round (3 more each for filling the column). 256^3: 32 planes, 7 rounds.
+inline int march_planes(int cols, int nz, int step, int resident) {
+    const int round = 148 * resident;
+    int best = step;
+    long long least = 0;
+    for (int lz = step; lz < nz + step; lz += step) {
+        const long long ctas = (long long)cols * ((nz + lz - 1) / lz), cost = (ctas + round - 1) / round * (lz + 3);
+        if (lz == step || cost < least) {
+            best = lz;
+            least = cost;
+        }
+    }
+    return best;
+}
+template <int RIEMANN, bool GATED> struct MarchK {
+    static cudaError_t prepare() {
+        return cudaFuncSetAttribute(mixed_march_kernel<RIEMANN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MarchShape::SMEM_BYTES);
+    }
+    // `nblocks` 8x8x8 tiles from a.b0, whole layers of tiles
+    static cudaError_t launch(const StageArgs& a0, int nblocks, cudaStream_t s) {
+        StageArgs a = a0;
+        const int layer = a.tiles[0] * a.tiles[1];
+        const int z0 = a.b0 / layer * 8, z_end = (a.b0 + nblocks) / layer * 8, z1 = z_end < a.m.nz ? z_end : a.m.nz;
+        const int cols = ((a.m.nx + MarchShape::W - 1) / MarchShape::W) * ((a.m.ny + MarchShape::H - 1) / MarchShape::H);
+        const int lz = march_planes(cols, z1 - z0, a.fin.kind == kFinNone ? 8 : 4, 2);
+        const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
+        a.fin.ctas = ctas;
+        mixed_march_kernel<RIEMANN, GATED><<<ctas, MarchShape::NT, MarchShape::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
+        return cudaGetLastError();
+    }
+};
+
+}   // namespace fvg

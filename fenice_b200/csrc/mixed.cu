@@ -2,6 +2,7 @@
 // root are the fast approximations and multiplies and adds may contract into FMAs, except where mixed.cuh rounds each
 // operation explicitly (the face values, the balance, the FP64 update); FP64 division and square root stay IEEE.
 #include "mixed.cuh"
+#include "march.cuh"
 #include "mixed_api.h"
 
 namespace fvg {
@@ -12,21 +13,8 @@ template <int DIM> struct MTile;
 template <> struct MTile<3> { static constexpr int X = 8, Y = 8, Z = 8, NT = 384; };
 template <> struct MTile<2> { static constexpr int X = 16, Y = 15, Z = 1, NT = 256; };
 
-// the cross-box kernel whose tiles inside the mesh come in by TMA: the 3-D WENO5-Z lean kernels, when the run passes
-// tensor maps (StageArgs::tma); 8x8x8 tiles of 384 threads
-template <int DIM, int RECON, bool FULL> constexpr bool kHasTma = DIM == 3 && RECON == kWeno5 && !FULL;
-
-template <int RIEMANN, bool GATED> struct TmaK {
-    static constexpr int NT = MTile<3>::NT;
-    static_assert(MTile<3>::X == 8 && MTile<3>::Y == 8 && MTile<3>::Z == 8, "the cross-box kernel's tile");
-    static cudaError_t prepare() {
-        return cudaFuncSetAttribute(mixed_stage_kernel_tma<RIEMANN, NT, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CrossShape::SMEM_BYTES);
-    }
-    static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
-        mixed_stage_kernel_tma<RIEMANN, NT, GATED><<<nblocks, NT, CrossShape::SMEM_BYTES, s>>>(a, *static_cast<const TmaMaps*>(a.tma));
-        return cudaGetLastError();
-    }
-};
+// the marching kernel (march.cuh): the 3-D WENO5-Z lean kernels, where can_march
+template <int DIM, int RECON, bool FULL> constexpr bool kHasMarch = DIM == 3 && RECON == kWeno5 && !FULL;
 
 template <int DIM, int RECON, int RIEMANN, bool FULL> struct MixedK {
     using T = MTile<DIM>;
@@ -34,13 +22,13 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct MixedK {
     static cudaError_t prepare() {
         cudaError_t e = cudaFuncSetAttribute(mixed_stage_kernel<DIM, RECON, RIEMANN, T::X, T::Y, T::Z, T::NT, false, FULL>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
-        if constexpr (kHasTma<DIM, RECON, FULL>)
-            if (e == cudaSuccess) e = TmaK<RIEMANN, false>::prepare();
+        if constexpr (kHasMarch<DIM, RECON, FULL>)
+            if (e == cudaSuccess) e = MarchK<RIEMANN, false>::prepare();
         return e;
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
-        if constexpr (kHasTma<DIM, RECON, FULL>)
-            if (a.tma) return TmaK<RIEMANN, false>::launch(a, nblocks, s);
+        if constexpr (kHasMarch<DIM, RECON, FULL>)
+            if (can_march(a)) return MarchK<RIEMANN, false>::launch(a, nblocks, s);
         mixed_stage_kernel<DIM, RECON, RIEMANN, T::X, T::Y, T::Z, T::NT, false, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
@@ -53,13 +41,13 @@ template <int DIM, int RIEMANN, bool FULL> struct GatedK {
     static cudaError_t prepare() {
         cudaError_t e = cudaFuncSetAttribute(mixed_stage_kernel<DIM, kWeno5, RIEMANN, T::X, T::Y, T::Z, T::NT, true, FULL>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
-        if constexpr (kHasTma<DIM, kWeno5, FULL>)
-            if (e == cudaSuccess) e = TmaK<RIEMANN, true>::prepare();
+        if constexpr (kHasMarch<DIM, kWeno5, FULL>)
+            if (e == cudaSuccess) e = MarchK<RIEMANN, true>::prepare();
         return e;
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
-        if constexpr (kHasTma<DIM, kWeno5, FULL>)
-            if (a.tma) return TmaK<RIEMANN, true>::launch(a, nblocks, s);
+        if constexpr (kHasMarch<DIM, kWeno5, FULL>)
+            if (can_march(a)) return MarchK<RIEMANN, true>::launch(a, nblocks, s);
         mixed_stage_kernel<DIM, kWeno5, RIEMANN, T::X, T::Y, T::Z, T::NT, true, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }

@@ -19,7 +19,6 @@
 
 #include "grid.cuh"
 #include "stage.cuh"
-#include "tma.cuh"
 #include "viscous.cuh"
 
 namespace fvg {
@@ -48,8 +47,10 @@ __device__ __forceinline__ float min_nan(float a, float b) {
     return r;
 }
 
-// HLLC / low-Mach HLLC of a face from its two primitive states (the Riemann solver of the mixed form), every operation
-// rounded explicitly so that each kernel that solves a face gets the same flux.
+// HLLC / low-Mach HLLC of a face from its two primitive states (the Riemann solver of the mixed form): density, pressure
+// and the NA velocity components of each side, the normal one first, the others in cyclic order; every operation rounded
+// explicitly, so that each kernel that solves a face gets the same flux. Fm: the mass flux, Fe: the energy flux, Fv: the
+// momentum fluxes in the order of the velocities; returns max(|S_L|, |S_R|).
 //
 // The star flux is written from the side the contact leaves to the other: with S the wave speed of that side, q =
 // rho (S - u_n) and f = q / (S - S_M), the mass flux is f S_M, the momentum flux f S_M v (+ p* = p + q (S_M - u_n) along
@@ -57,36 +58,36 @@ __device__ __forceinline__ float min_nan(float a, float b) {
 // between the four, in exact arithmetic, with one side's states instead of two, two reciprocals instead of five and no
 // difference of nearly equal products at low Mach numbers. A supersonic face is the same formulas with S_M = u_n, f = rho,
 // p* = p. The Mach number of the low-Mach scaling takes one reciprocal and one square root for both sides.
-template <int RIEMANN, int NV>
-__device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend, St<float, NV> WL, St<float, NV> WR, int axis, St<float, NV>& F) {
-    constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
-    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
-    const float rL = max_nan(WL[0], Num<float>::eos_eps), pL = max_nan(WL[3], Num<float>::eos_eps);
-    const float rR = max_nan(WR[0], Num<float>::eos_eps), pR = max_nan(WR[3], Num<float>::eos_eps);
+template <int RIEMANN, int NA>
+__device__ __forceinline__ float riemann_f(const GasF& e, float shock_blend, float rL, float pL, float (&vL)[NA], float rR, float pR, float (&vR)[NA],
+                                           float& Fm, float& Fe, float (&Fv)[NA]) {
+    rL = max_nan(rL, Num<float>::eos_eps);
+    pL = max_nan(pL, Num<float>::eos_eps);
+    rR = max_nan(rR, Num<float>::eos_eps);
+    pR = max_nan(pR, Num<float>::eos_eps);
     const float iL = rcp_f(rL), iR = rcp_f(rR);
     const float aL = __fmul_rn(__fmul_rn(e.g, __fadd_rn(pL, e.pi)), iL), aR = __fmul_rn(__fmul_rn(e.g, __fadd_rn(pR, e.pi)), iR);   // c^2
     const float cL = sqrt_f(aL), cR = sqrt_f(aR);
+    const auto square = [](const float (&v)[NA]) {
+        float s = __fmul_rn(v[0], v[0]);
+#pragma unroll
+        for (int a = 1; a < NA; ++a) s = __fmaf_rn(v[a], v[a], s);
+        return s;
+    };
     if constexpr (RIEMANN == kLowMach) {
-        float mL = __fmul_rn(WL[1], WL[1]), mR = __fmul_rn(WR[1], WR[1]);
-        mL = __fmaf_rn(WL[2], WL[2], mL);
-        mR = __fmaf_rn(WR[2], WR[2], mR);
-        if constexpr (NV == 5) {
-            mL = __fmaf_rn(WL[4], WL[4], mL);
-            mR = __fmaf_rn(WR[4], WR[4], mR);
-        }
+        const float mL = square(vL), mR = square(vR);
         const bool gl = __fmul_rn(mL, aR) > __fmul_rn(mR, aL);   // the larger Mach number's side
         const float M = sqrt_f(__fmul_rn(gl ? mL : mR, rcp_f(gl ? aL : aR)));
         const float z = min_nan(max_nan(M, 1e-4f), 1.0f);
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
-            const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-            const float avg = __fmul_rn(0.5f, __fadd_rn(WL[m], WR[m]));
-            const float half = __fmul_rn(0.5f, __fsub_rn(WL[m], WR[m]));
-            WL[m] = __fmaf_rn(z, half, avg);
-            WR[m] = __fmaf_rn(-z, half, avg);
+            const float avg = __fmul_rn(0.5f, __fadd_rn(vL[a], vR[a]));
+            const float half = __fmul_rn(0.5f, __fsub_rn(vL[a], vR[a]));
+            vL[a] = __fmaf_rn(z, half, avg);
+            vR[a] = __fmaf_rn(-z, half, avg);
         }
     }
-    const float uL = WL[mn], uR = WR[mn];
+    const float uL = vL[0], uR = vR[0];
     const float SL = min_nan(__fsub_rn(uL, cL), __fsub_rn(uR, cR)), SR = max_nan(__fadd_rn(uL, cL), __fadd_rn(uR, cR));
     const float qL = __fmul_rn(rL, __fsub_rn(SL, uL)), qR = __fmul_rn(rR, __fsub_rn(SR, uR));
     const float num = __fmaf_rn(qR, uR, __fmaf_rn(-qL, uL, __fsub_rn(pL, pR)));
@@ -94,68 +95,72 @@ __device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend
     const bool sup = SL >= 0.0f || SR < 0.0f;
     const bool left = SR >= 0.0f && (SL >= 0.0f || SM >= 0.0f);
     const bool fail = !sup && !(SM >= 0.0f) && !(SM < 0.0f);   // a NaN speed: no flux
-    const float rho = left ? rL : rR, p = left ? pL : pR, un = left ? uL : uR, q = left ? qL : qR;
-    float vt[NA];   // the side's velocity
+    const float rho = left ? rL : rR, p = left ? pL : pR, q = left ? qL : qR;
+    float v[NA];   // the side's velocity
 #pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-        vt[a] = left ? WL[m] : WR[m];
-    }
-    float ke = __fmul_rn(vt[0], vt[0]);
-#pragma unroll
-    for (int a = 1; a < NA; ++a) ke = __fmaf_rn(vt[a], vt[a], ke);
-    const float E = __fmaf_rn(0.5f, ke, __fmul_rn(__fmul_rn(__fadd_rn(p, e.gpi), e.g1), left ? iL : iR));   // per unit mass
-    const float d = __fsub_rn(SM, un);
+    for (int a = 0; a < NA; ++a) v[a] = left ? vL[a] : vR[a];
+    const float E = __fmaf_rn(0.5f, square(v), __fmul_rn(__fmul_rn(__fadd_rn(p, e.gpi), e.g1), left ? iL : iR));   // per unit mass
+    const float d = __fsub_rn(SM, v[0]);
     const float w = __fsub_rn(left ? SL : SR, SM);
     const float rc = rcp_f(copysignf(max_nan(fabsf(w), Num<float>::denom_eps), w));
     float f = __fmul_rn(q, rc), ps = __fmaf_rn(q, d, p);
     float Es = __fmaf_rn(f, __fmaf_rn(d, SM, E), __fmul_rn(__fmul_rn(d, p), rc));
     if (sup) {
-        SM = un;
+        SM = v[0];
         f = rho;
         ps = p;
         Es = __fmul_rn(rho, E);
     }
-    const float G = __fmul_rn(f, SM);
-    F[0] = G;
+    Fm = __fmul_rn(f, SM);
+    Fv[0] = __fmaf_rn(Fm, SM, ps);
 #pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-        F[m] = a == axis ? __fmaf_rn(G, SM, ps) : __fmul_rn(G, vt[a]);
-    }
-    F[3] = __fmul_rn(SM, __fadd_rn(Es, ps));
+    for (int a = 1; a < NA; ++a) Fv[a] = __fmul_rn(Fm, v[a]);
+    Fe = __fmul_rn(SM, __fadd_rn(Es, ps));
     const float jump = fabsf(__fsub_rn(pR, pL)), pm = min_nan(pL, pR);
     if (shock_blend > 0.0f && jump > __fmul_rn(shock_blend, pm) && !sup) {
         // a strong pressure jump: the HLL flux blended in
         const float phi = min_nan(__fmul_rn(__fsub_rn(__fmul_rn(jump, rcp_f(pm)), shock_blend), rcp_f(shock_blend)), 1.0f);
         const float inv = rcp_f(__fsub_rn(SR, SL)), ss = __fmul_rn(SL, SR);
         const float mL = __fmul_rn(rL, uL), mR = __fmul_rn(rR, uR);
-        float kL = __fmul_rn(WL[1], WL[1]), kR = __fmul_rn(WR[1], WR[1]);
-        kL = __fmaf_rn(WL[2], WL[2], kL);
-        kR = __fmaf_rn(WR[2], WR[2], kR);
-        if constexpr (NV == 5) {
-            kL = __fmaf_rn(WL[4], WL[4], kL);
-            kR = __fmaf_rn(WR[4], WR[4], kR);
-        }
-        const float EL = __fmaf_rn(__fmul_rn(0.5f, rL), kL, __fmul_rn(__fadd_rn(pL, e.gpi), e.g1));
-        const float ER = __fmaf_rn(__fmul_rn(0.5f, rR), kR, __fmul_rn(__fadd_rn(pR, e.gpi), e.g1));
+        const float EL = __fmaf_rn(__fmul_rn(0.5f, rL), square(vL), __fmul_rn(__fadd_rn(pL, e.gpi), e.g1));
+        const float ER = __fmaf_rn(__fmul_rn(0.5f, rR), square(vR), __fmul_rn(__fadd_rn(pR, e.gpi), e.g1));
         const auto blend = [&](float f0, float fl, float fr, float ul, float ur) {
             const float h = __fmul_rn(__fmaf_rn(ss, __fsub_rn(ur, ul), __fmaf_rn(SR, fl, -__fmul_rn(SL, fr))), inv);
             return __fmaf_rn(phi, h, __fmul_rn(__fsub_rn(1.0f, phi), f0));
         };
-        F[0] = blend(F[0], mL, mR, rL, rR);
+        Fm = blend(Fm, mL, mR, rL, rR);
 #pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-            F[m] = blend(F[m], a == axis ? __fmaf_rn(mL, WL[m], pL) : __fmul_rn(mL, WL[m]), a == axis ? __fmaf_rn(mR, WR[m], pR) : __fmul_rn(mR, WR[m]),
-                         __fmul_rn(rL, WL[m]), __fmul_rn(rR, WR[m]));
-        }
-        F[3] = blend(F[3], __fmul_rn(uL, __fadd_rn(EL, pL)), __fmul_rn(uR, __fadd_rn(ER, pR)), EL, ER);
+        for (int a = 0; a < NA; ++a)
+            Fv[a] = blend(Fv[a], a == 0 ? __fmaf_rn(mL, uL, pL) : __fmul_rn(mL, vL[a]), a == 0 ? __fmaf_rn(mR, uR, pR) : __fmul_rn(mR, vR[a]),
+                          __fmul_rn(rL, vL[a]), __fmul_rn(rR, vR[a]));
+        Fe = blend(Fe, __fmul_rn(uL, __fadd_rn(EL, pL)), __fmul_rn(uR, __fadd_rn(ER, pR)), EL, ER);
     }
-    if (fail)
+    if (fail) {
+        Fm = Fe = 0.0f;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) F[k] = 0.0f;
+        for (int a = 0; a < NA; ++a) Fv[a] = 0.0f;
+    }
     return max_nan(fabsf(SL), fabsf(SR));
+}
+// riemann_f of two primitive states in the state's order, along a compile-time axis
+template <int RIEMANN, int NV>
+__device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend, const St<float, NV>& WL, const St<float, NV>& WR, int axis,
+                                                St<float, NV>& F) {
+    constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
+    float vL[NA], vR[NA], Fv[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        const int c = (axis + a) % NA, m = c == 0 ? 1 : (c == 1 ? 2 : 4);
+        vL[a] = WL[m];
+        vR[a] = WR[m];
+    }
+    const float s = riemann_f<RIEMANN>(e, shock_blend, WL[0], WL[3], vL, WR[0], WR[3], vR, F[0], F[3], Fv);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        const int c = (axis + a) % NA, m = c == 0 ? 1 : (c == 1 ? 2 : 4);
+        F[m] = Fv[a];
+    }
+    return s;
 }
 
 // The two linear face values of six cells: the fifth-order upwind value right of c2 from c0 .. c4, 0.1 p0 + 0.6 p1 + 0.3 p2
@@ -168,6 +173,33 @@ __device__ __forceinline__ void lin5_pair(float c0, float c1, float c2, float c3
     s = f2_fma(f2(27.0f, 27.0f), f2(c3, c2), s);
     s = f2_fma(f2(-3.0f, -3.0f), f2(c4, c1), s);
     f2_get(f2_mul(s, f2(1.0f / 60.0f, 1.0f / 60.0f)), wl, wr);
+}
+
+// The primitive state of a cell (cons_to_prim in FP64) for the mixed form, each operation rounded explicitly (the same bits
+// in every kernel that rounds it to FP32); inv receives 1 / rho of the floored density: the hardware's approximate
+// reciprocal and two Newton steps, within a unit in the last place of FP64.
+template <int NV> __device__ __forceinline__ St<double, NV> prim_d(const Eos<double>& e, const St<double, NV>& U, double& inv) {
+    St<double, NV> W;
+    const double rho = vmax(U[0], Num<double>::eos_eps);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(rho));
+    y = __fma_rn(__fma_rn(-rho, y, 1.0), y, y);
+    y = __fma_rn(__fma_rn(-rho, y, 1.0), y, y);
+    inv = y;
+    const double u = __dmul_rn(U[1], inv), v = __dmul_rn(U[2], inv);
+    double k = __fma_rn(v, v, __dmul_rn(u, u));
+    if constexpr (NV == 5) {
+        const double w = __dmul_rn(U[4], inv);
+        k = __fma_rn(w, w, k);
+        W[4] = w;
+    }
+    const double ei = __fma_rn(__dmul_rn(-0.5, rho), k, U[3]);
+    const double gp = e.type == kIdeal ? 0.0 : __dmul_rn(e.gamma, e.p_inf);
+    W[0] = rho;
+    W[1] = u;
+    W[2] = v;
+    W[3] = vmax(__fma_rn(__dsub_rn(e.gamma, 1.0), ei, -gp), Num<double>::eos_eps);
+    return W;
 }
 
 template <int DIM, int RECON, int TX, int TY, int TZ> struct MixedShape {
@@ -190,14 +222,10 @@ template <int DIM, int RECON, int TX, int TY, int TZ> struct MixedShape {
 // GATED (WENO5-Z with the learned sensor): the tile's flag for this axis (one byte per tile and axis, from the sensor's
 // last refresh) makes the reconstructions of the sweep linear (0) or WENO5-Z (1), a branch uniform over the CTA; the seam
 // faces of a linear tile whose tile across stays WENO5-Z take WENO5-Z in a short pass of their own.
-// TMA (mixed_stage_kernel_tma): a tile whose box lies inside the mesh is staged by one bulk tensor copy into the face-value
-// arrays (free during the load) and converted from there; the others take the index-mapping loader. `phase` counts the
-// barrier's completed copies (its parity is the one to wait for).
-template <int AXIS, int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool GATED = false, bool FULL = true, bool TMA = false>
+template <int AXIS, int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool GATED = false, bool FULL = true>
 __device__ __forceinline__ void mixed_axis(const StageArgs& a, const GasF& ef, float sb, float weps, float* __restrict__ P,
                                            float* __restrict__ WL, float* __restrict__ WR, float* __restrict__ acc, unsigned char* __restrict__ Sf,
-                                           const int o3[3], float& smax, const CUtensorMap* maps = nullptr, unsigned long long* bar = nullptr,
-                                           unsigned* phase = nullptr) {
+                                           const int o3[3], float& smax) {
     using S = MixedShape<DIM, RECON, TX, TY, TZ>;
     constexpr int NV = S::NV, H = S::H, NC = S::NC;
     constexpr int axis = AXIS;
@@ -209,43 +237,13 @@ __device__ __forceinline__ void mixed_axis(const StageArgs& a, const GasF& ef, f
         constexpr int Fd[3] = {TX + (AXIS == 0), TY + (AXIS == 1), TZ + (AXIS == 2)};
         constexpr int nE = E[0] * E[1] * E[2], nF = Fd[0] * Fd[1] * Fd[2];
         // ---- 1. load: the primitive state recovered in FP64, stored as FP32
-        bool via_tma = false;
-        if constexpr (TMA) {
-            constexpr int BX = AXIS == 0 ? 16 : TX, BY = TY + (AXIS == 1 ? 2 * H : 0), BZ = TZ + (AXIS == 2 ? 2 * H : 0);
-            const int x0 = AXIS == 0 ? o3[0] - 4 : o3[0], y0 = AXIS == 1 ? o3[1] - H : o3[1], z0 = AXIS == 2 ? o3[2] - H : o3[2];
-            via_tma = x0 >= 0 && x0 + BX <= n3[0] && y0 >= 0 && y0 + BY <= n3[1] && z0 >= 0 && z0 + BZ <= n3[2] && (tma::su32(WL) & 127u) == 0;
-            if (via_tma) {
-                const double* stg = reinterpret_cast<const double*>(WL);
-                if (tid == 0) {
-                    tma::fence_proxy_async();
-                    tma::mbar_expect_tx(bar, (unsigned)(BX * BY * BZ * NV * 8));
-                    tma::load_4d(WL, &maps[AXIS], x0, y0, z0, 0, bar);
-                }
-                // every thread waits for this copy's phase of the barrier, at most 2^22 polls; a copy that never
-                // completes stops the run (status 5) instead of hanging the GPU
-                bool done = false;
-                for (int it = 0; it < (1 << 22) && !done; ++it) done = tma::mbar_try_wait(bar, *phase & 1u);
-                ++*phase;
-                if (!done && tid == 0) atomicExch(const_cast<int*>(&a.ctl->status), 5);
-                for (int e = tid; e < nE; e += NT) {
-                    const int l3[3] = {e % E[0], (e / E[0]) % E[1], e / (E[0] * E[1])};
-                    const int si = (l3[2] * BY + l3[1]) * BX + (AXIS == 0 ? l3[0] + 1 : l3[0]);
-                    St<double, NV> u;
-#pragma unroll
-                    for (int q = 0; q < NV; ++q) u[q] = done ? stg[q * (BX * BY * BZ) + si] : 1.0;
-                    const St<double, NV> w = c2p(a.eos, u);
-#pragma unroll
-                    for (int q = 0; q < NV; ++q) P[q * S::EXT + e] = (float)w[q];
-                }
-            }
-        }
-        if (!via_tma)
         for (int e = tid; e < nE; e += NT) {
             int l3[3] = {e % E[0], (e / E[0]) % E[1], e / (E[0] * E[1])};
             l3[axis] -= H;
-            const St<double, NV> w = c2p(a.eos, stencil_cons<DIM, NV, FULL>(m, a.bc, a.eos, a.U, o3[0] + l3[0], o3[1] + l3[1], o3[2] + l3[2]));
+            double inv;
+            const St<double, NV> w = prim_d(a.eos, stencil_cons<DIM, NV, FULL>(m, a.bc, a.eos, a.U, o3[0] + l3[0], o3[1] + l3[1], o3[2] + l3[2]), inv);
             if constexpr (RECON == kWeno5)
-                if (!TMA && a.bc.solid) Sf[e] = stencil_solid<DIM>(m, a.bc, o3[0] + l3[0], o3[1] + l3[1], o3[2] + l3[2]);
+                if (a.bc.solid) Sf[e] = stencil_solid<DIM>(m, a.bc, o3[0] + l3[0], o3[1] + l3[1], o3[2] + l3[2]);
 #pragma unroll
             for (int q = 0; q < NV; ++q) P[q * S::EXT + e] = (float)w[q];
         }
@@ -291,7 +289,7 @@ __device__ __forceinline__ void mixed_axis(const StageArgs& a, const GasF& ef, f
                 const float c0 = c[0], c1 = c[sstride], c2 = c[2 * sstride], c3 = c[3 * sstride], c4 = c[4 * sstride], c5 = c[5 * sstride];
                 const int base = (f3[2] * E[1] + f3[1]) * E[0] + f3[0];
                 bool four = false;
-                if (!TMA && a.bc.solid)   // (the TMA kernel never runs with an immersed body)
+                if (a.bc.solid)
 #pragma unroll
                     for (int s6 = 0; s6 < 6; ++s6) four = four || Sf[base + s6 * sstride] != 0;
                 if (four) {
@@ -328,7 +326,7 @@ __device__ __forceinline__ void mixed_axis(const StageArgs& a, const GasF& ef, f
                     const float* c = P + q * S::EXT + base;
                     const float c0 = c[0], c1 = c[sstride], c2 = c[2 * sstride], c3 = c[3 * sstride], c4 = c[4 * sstride], c5 = c[5 * sstride];
                     bool four = false;
-                    if (!TMA && a.bc.solid)   // (the TMA kernel never runs with an immersed body)
+                    if (a.bc.solid)
 #pragma unroll
                         for (int s6 = 0; s6 < 6; ++s6) four = four || Sf[base + s6 * sstride] != 0;
                     float wl, wr;
@@ -537,7 +535,7 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
         else
             u = cell_at(a, g[0], g[1], g[2]);
         double inv;
-        const St<double, 5> w = c2p(a.eos, u, inv);
+        const St<double, 5> w = prim_d(a.eos, u, inv);
         R[e] = (float)u[0];
         V[e] = make_float4((float)w[1], (float)w[2], (float)w[4], (float)(w[3] * inv));
     }
@@ -701,352 +699,6 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
         if (s > smax) smax = s;
     }
     const double bm = block_max<NT>(smax, red);
-    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
-}
-
-// The per-axis sweep's shared memory with TMA boxes (mixed_axis with TMA): red [32 doubles] | the barrier | P | acc | Sf |
-// (128-byte aligned) WL, WR, sized for the largest box (16 x 8 x 8 x 5 doubles, 40 KB), which the copy fills while the
-// face-value arrays are idle.
-template <int TX, int TY, int TZ> struct MixedTmaShape {
-    using S = MixedShape<3, kWeno5, TX, TY, TZ>;
-    static constexpr int P_OFF = 272, ACC_OFF = P_OFF + 4 * S::NV * S::EXT, SF_OFF = ACC_OFF + 4 * S::NV * S::NC;
-    static constexpr int STG_OFF = (SF_OFF + S::FLAG_BYTES + 127) / 128 * 128;
-    static constexpr int BOX_BYTES = 16 * TY * TZ * S::NV * 8;   // the x sweep's box, the largest
-    static constexpr int STG_BYTES = BOX_BYTES > 8 * S::NV * S::NF ? BOX_BYTES : 8 * S::NV * S::NF;
-    static constexpr size_t SMEM_BYTES = STG_OFF + STG_BYTES;
-};
-
-// The mixed WENO5-Z stage kernel of a 3-D mesh without part interfaces, non-reflecting sides or an immersed body, whose
-// boxes come in by TMA (tma.cuh; no copy multicasts), in two forms chosen per tile (a branch uniform over the CTA):
-// - the per-axis sweep of mixed_stage_kernel (mixed_axis with TMA: a 16 x 8 x 8, 8 x 14 x 8 or 8 x 8 x 14 box per axis),
-//   for every tile of the ungated kernel and for the gated tiles that keep WENO5-Z along some axis or beside a seam;
-// - the cross (gated tiles linear along all three axes and at all six seams): one image of the tile and its three halos
-//   (the 8x8x8 tile and 3 cells beyond each of its six faces, 1664 cells) converted once, from a 16 x 8 x 8 box (the tile
-//   and its x halos) and four 3-deep halo boxes; then every face of the three axes in one pass, one thread per face and
-//   all five variables (the linear face values straight into the Riemann solver, no face-value arrays); then the
-//   balance ((0 - x) - y) - z of each cell from the three flux arrays in the epilogue.
-// Both forms give the bits of mixed_stage_kernel (the explicitly rounded lin5 / weno5z, balance and update), so a face
-// between tiles of the two forms gets one flux. A tile whose boxes would leave the mesh (wrapped or ghost cells) takes the
-// index-mapping loader for those parts. Measured at 256^3 (Taylor-Green, every tile-axis linear, with the viscous sums
-// and U0): 1.60 ms per launch for the cross against 2.11 ms for the per-axis sweep; with WENO5-Z along every axis the
-// per-axis sweep is the faster (2.74 against 3.01 ms for a cross that solved WENO5-Z faces too: the per-axis sweep's
-// (face, variable) items spread the WENO5-Z work finer).
-// Shared memory: the larger of the two layouts (74.1 KB), three CTAs of 384 threads per SM (at most 56 registers).
-struct CrossShape {
-    // slots of the cross: the tile's 512 cells in rows of 9 (576 slots: x + 9 y + 72 z, so that a warp reading one x
-    // column of 32 rows touches 32 banks), then the six 3-deep halos of 192 cells
-    static constexpr int NV = 5, NCORE = 576, NHALO = 192, NPC = NCORE + 6 * NHALO;
-    static constexpr int NFA = 576, NFACE = 3 * NFA, NINNER = 448;                    // faces per axis; t = 1 .. 7
-    static constexpr int BAR_OFF = 256, P_OFF = 272;
-    static constexpr int STG_OFF = (P_OFF + 4 * NV * NPC + 127) / 128 * 128;
-    static constexpr int XBOX = 16 * 8 * 8, HBOX = 8 * 3 * 8;   // cells of the x box and of one halo box
-    static constexpr int STG_BYTES = XBOX * NV * 8;
-    static constexpr size_t CROSS_BYTES = STG_OFF + STG_BYTES;
-    static constexpr size_t SMEM_BYTES = CROSS_BYTES > MixedTmaShape<8, 8, 8>::SMEM_BYTES ? CROSS_BYTES : MixedTmaShape<8, 8, 8>::SMEM_BYTES;
-    static_assert(4 * HBOX * NV * 8 <= STG_BYTES && 3 * NV * NFA * 4 <= STG_BYTES, "the staging area holds the halo boxes and the fluxes");
-};
-
-// the cross's slot of the cell at s along axis A (s in [-3, 11)) and (u, v) along the other two axes in increasing
-// order: the tile's cells (x + 9 y + 72 z), then the six halos (axis-major, low side first), each 3 deep x 64 cells
-template <int A> __device__ __forceinline__ int cross_slot(int s, int u, int v) {
-    if (s < 0) return 576 + (2 * A) * 192 + (s + 3) + 3 * (u + 8 * v);
-    if (s >= 8) return 576 + (2 * A + 1) * 192 + (s - 8) + 3 * (u + 8 * v);
-    return A == 0 ? s + 9 * u + 72 * v : (A == 1 ? u + 9 * s + 72 * v : u + 9 * v + 72 * s);
-}
-// cell e of the cross (the tile's 512 cells, x fastest, then the six halos of cross_slot's order): its tile-local
-// coordinates and its slot
-__device__ __forceinline__ int cross_cell(int e, int l3[3]) {
-    if (e < 512) {
-        l3[0] = e & 7;
-        l3[1] = (e >> 3) & 7;
-        l3[2] = e >> 6;
-        return l3[0] + 9 * l3[1] + 72 * l3[2];
-    }
-    const int k = (e - 512) / 192, r = (e - 512) % 192, A = k >> 1;
-    const int l = r % 3, uv = r / 3, u = uv & 7, v = uv >> 3;
-    const int s = (k & 1) ? 8 + l : l - 3;
-    l3[0] = A == 0 ? s : u;
-    l3[1] = A == 0 ? u : (A == 1 ? s : v);
-    l3[2] = A == 2 ? s : v;
-    return e + 64;
-}
-
-// One face of axis A in the cross (linear face values): item r of the axis (the 448 faces inside the tile, t = 1 .. 7,
-// then the two seam layers t = 0 and 8); its flux goes to Fs at the face's index in mixed_axis's numbering.
-template <int A, int RIEMANN>
-__device__ __forceinline__ void cross_face(const StageArgs& a, const GasF& ef, float sb, const float* __restrict__ P, float* __restrict__ Fs,
-                                           int r, const int o3[3], float& smax) {
-    constexpr int NV = 5, NPC = CrossShape::NPC;
-    int t, u, v;
-    if (r < CrossShape::NINNER) {   // (the lanes of a warp run along the cross's rows: no two on one bank)
-        if (A == 0) {
-            t = 1 + r % 7;
-            u = (r / 7) & 7;
-            v = r / 56;
-        } else if (A == 1) {
-            u = r & 7;
-            t = 1 + (r >> 3) % 7;
-            v = (r >> 3) / 7;
-        } else {
-            u = r & 7;
-            v = (r >> 3) & 7;
-            t = 1 + (r >> 6);
-        }
-    } else {
-        const int q = r - CrossShape::NINNER;
-        u = q & 7;
-        v = (q >> 3) & 7;
-        t = (q >> 6) * 8;
-    }
-    const int f = A == 0 ? t + 9 * (u + 8 * v) : (A == 1 ? u + 8 * (t + 9 * v) : u + 8 * (v + 8 * t));
-    int sl[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) sl[k] = cross_slot<A>(t - 3 + k, u, v);
-    St<float, NV> wl, wr;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        const float* c = P + q * NPC;
-        const float c0 = c[sl[0]], c1 = c[sl[1]], c2 = c[sl[2]], c3 = c[sl[3]], c4 = c[sl[4]], c5 = c[sl[5]];
-        lin5_pair(c0, c1, c2, c3, c4, c5, wl[q], wr[q]);
-    }
-    const Mesh& m = a.m;
-    const int n3[3] = {m.nx, m.ny, m.nz};
-    const int g3[3] = {o3[0] + (A == 0 ? t : u), o3[1] + (A == 0 ? u : (A == 1 ? t : v)), o3[2] + (A == 2 ? t : v)};
-    bool inside = true;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) inside = inside && (d == A ? g3[d] <= n3[d] : g3[d] < n3[d]);
-    St<float, NV> F;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) F[q] = 0.0f;
-    // (no face of a tile in the cross form lies on a side without a halo: the gate keeps every tile whose extension along
-    // an axis leaves the mesh across a side that is not periodic WENO5-Z along that axis, so such a tile never takes the
-    // cross form; mixed_axis's first-order side states are not needed here)
-    if (inside) {
-        const float sp = face_flux_prim<RIEMANN>(ef, sb, wl, wr, A, F);
-        if (sp > smax) smax = sp;
-    }
-#pragma unroll
-    for (int q = 0; q < NV; ++q) Fs[(A * NV + q) * CrossShape::NFA + f] = F[q];
-}
-
-// The epilogue's operands that no box brings in (the 8x8x8 tile's rows of U0 and of the FP32 viscous sums) head for L2
-// at the start of the tile, so that the epilogue's loads find them there (measured at 256^3 in the cross form: 1.79 ->
-// 1.72 ms per launch)
-template <int NT> __device__ __forceinline__ void prefetch_epilogue(const StageArgs& a, const int o3[3]) {
-    if (a.mode != kCombine && !a.Rvf) return;
-    const Mesh& m = a.m;
-    for (int k = threadIdx.x; k < 9 * 64; k += NT) {
-        const int q = k >> 6, y = o3[1] + (k & 7), z = o3[2] + ((k >> 3) & 7);
-        if (y >= m.ny || z >= m.nz) continue;
-        const long long row = ((long long)z * m.ny + y) * m.nx + o3[0];
-        if (q < 5 && a.mode == kCombine) prefetch_l2(a.U0 + q * m.plane + row);
-        if (q >= 5 && a.Rvf) prefetch_l2(a.Rvf + (q - 5) * m.plane + row);
-    }
-}
-
-// The cross form of a tile (see mixed_stage_kernel_tma): maps m[0] (the 16 x 8 x 8 box), m[3] and m[4] (the y and z halo
-// boxes); `phase` counts the barrier's completed copies.
-template <int RIEMANN, int NT>
-__device__ __forceinline__ void cross_tile(const StageArgs& a, const TmaMaps& maps, unsigned char* smem_b, const int o3[3], unsigned& phase, float& smax) {
-    using L = CrossShape;
-    constexpr int NV = 5, NPC = L::NPC;
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem_b + L::BAR_OFF);
-    float* P = reinterpret_cast<float*>(smem_b + L::P_OFF);
-    double* stg = reinterpret_cast<double*>(smem_b + L::STG_OFF);
-    float* Fs = reinterpret_cast<float*>(smem_b + L::STG_OFF);
-    const Mesh& m = a.m;
-    const int n3[3] = {m.nx, m.ny, m.nz};
-    const GasF ef = gas_f(a.eos);
-    const float sb = (float)a.shock_blend;
-    const int tid = threadIdx.x;
-    const bool aligned = (tma::su32(stg) & 127u) == 0;
-    // every thread waits for the barrier's current phase, at most 2^22 polls; a copy that never completes stops the run
-    // (status 5) instead of hanging the GPU
-    auto wait = [&]() -> bool {
-        bool done = false;
-        for (int it = 0; it < (1 << 22) && !done; ++it) done = tma::mbar_try_wait(bar, phase & 1u);
-        ++phase;
-        if (!done && tid == 0) atomicExch(const_cast<int*>(&a.ctl->status), 5);
-        return done;
-    };
-    // cells e0 .. e1 of the cross by index mapping (wrapped and ghost cells), the primitive state recovered in FP64
-    auto load_slots = [&](int e0, int e1) {
-        for (int e = e0 + tid; e < e1; e += NT) {
-            int l3[3];
-            const int p = cross_cell(e, l3);
-            const St<double, NV> w = c2p(a.eos, stencil_cons<3, NV, false>(m, a.bc, a.eos, a.U, o3[0] + l3[0], o3[1] + l3[1], o3[2] + l3[2]));
-#pragma unroll
-            for (int q = 0; q < NV; ++q) P[q * NPC + p] = (float)w[q];
-        }
-    };
-    prefetch_epilogue<NT>(a, o3);
-    // ---- 1. the tile and its x halos (cells 0 .. 895): one 16 x 8 x 8 box from x = o - 4
-    if (aligned && o3[0] >= 4 && o3[0] + 12 <= n3[0] && o3[1] + 8 <= n3[1] && o3[2] + 8 <= n3[2]) {
-        if (tid == 0) {
-            tma::fence_proxy_async();
-            tma::mbar_expect_tx(bar, (unsigned)(L::XBOX * NV * 8));
-            tma::load_4d(stg, &maps.m[0], o3[0] - 4, o3[1], o3[2], 0, bar);
-        }
-        const bool done = wait();
-        for (int e = tid; e < 14 * 64; e += NT) {
-            const int xl = e % 14 - 3, y = (e / 14) & 7, z = e / 112;
-            const int si = (z * 8 + y) * 16 + xl + 4;
-            St<double, NV> uc;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) uc[q] = done ? stg[q * L::XBOX + si] : 1.0;
-            const St<double, NV> w = c2p(a.eos, uc);
-            const int p = cross_slot<0>(xl, y, z);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) P[q * NPC + p] = (float)w[q];
-        }
-    } else {
-        load_slots(0, 896);
-    }
-    __syncthreads();
-    // ---- 2. the y and z halos (cells 896 .. 1663): four 3-deep boxes on one barrier phase
-    if (aligned && o3[1] >= 3 && o3[1] + 11 <= n3[1] && o3[2] >= 3 && o3[2] + 11 <= n3[2] && o3[0] + 8 <= n3[0]) {
-        if (tid == 0) {
-            tma::fence_proxy_async();
-            tma::mbar_expect_tx(bar, (unsigned)(4 * L::HBOX * NV * 8));
-            tma::load_4d(stg, &maps.m[3], o3[0], o3[1] - 3, o3[2], 0, bar);
-            tma::load_4d(stg + 1 * L::HBOX * NV, &maps.m[3], o3[0], o3[1] + 8, o3[2], 0, bar);
-            tma::load_4d(stg + 2 * L::HBOX * NV, &maps.m[4], o3[0], o3[1], o3[2] - 3, 0, bar);
-            tma::load_4d(stg + 3 * L::HBOX * NV, &maps.m[4], o3[0], o3[1], o3[2] + 8, 0, bar);
-        }
-        const bool done = wait();
-        for (int e = tid; e < 4 * L::HBOX; e += NT) {
-            const int k = e / L::HBOX, r = e % L::HBOX;
-            const double* box = stg + k * L::HBOX * NV;
-            int si, p;
-            if (k < 2) {   // 8 x 3 x 8 boxes below and above the tile along y
-                const int x = r & 7, yb = (r >> 3) % 3, z = r / 24;
-                si = (z * 3 + yb) * 8 + x;
-                p = cross_slot<1>(k == 0 ? yb - 3 : 8 + yb, x, z);
-            } else {       // 8 x 8 x 3 boxes along z
-                const int x = r & 7, y = (r >> 3) & 7, zb = r >> 6;
-                si = (zb * 8 + y) * 8 + x;
-                p = cross_slot<2>(k == 2 ? zb - 3 : 8 + zb, x, y);
-            }
-            St<double, NV> uc;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) uc[q] = done ? box[q * L::HBOX + si] : 1.0;
-            const St<double, NV> w = c2p(a.eos, uc);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) P[q * NPC + p] = (float)w[q];
-        }
-    } else {
-        load_slots(896, 1664);
-    }
-    __syncthreads();
-    // ---- 3. every face of the three axes (the faces inside the tile first, 448 per axis, then the seam layers)
-    for (int it = tid; it < L::NFACE; it += NT) {
-        int A, r;
-        if (it < 3 * L::NINNER) {
-            A = it / L::NINNER;
-            r = it - A * L::NINNER;
-        } else {
-            const int q = it - 3 * L::NINNER;
-            A = q >> 7;
-            r = L::NINNER + (q & 127);
-        }
-        if (A == 0)
-            cross_face<0, RIEMANN>(a, ef, sb, P, Fs, r, o3, smax);
-        else if (A == 1)
-            cross_face<1, RIEMANN>(a, ef, sb, P, Fs, r, o3, smax);
-        else
-            cross_face<2, RIEMANN>(a, ef, sb, P, Fs, r, o3, smax);
-    }
-    __syncthreads();
-    // ---- 4. the balance ((0 - x) - y) - z, the residual widened to FP64 and the FP64 stage update
-    const float Ax = (float)m.area[0], Ay = (float)m.area[1], Az = (float)m.area[2];
-    const double dt = a.ctl->dt;
-    for (int c = tid; c < 512; c += NT) {
-        const int c3[3] = {c & 7, (c >> 3) & 7, c >> 6};
-        const int g3[3] = {o3[0] + c3[0], o3[1] + c3[1], o3[2] + c3[2]};
-        if (g3[0] >= m.nx || g3[1] >= m.ny || g3[2] >= m.nz) continue;
-        const long long cell = ((long long)g3[2] * m.ny + g3[1]) * m.nx + g3[0];
-        const int fx = (c3[2] * 8 + c3[1]) * 9 + c3[0], fy = (c3[2] * 9 + c3[1]) * 8 + c3[0], fz = c;
-        CellIn<NV> in;
-        cell_load(a, cell, in);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            const float* X = Fs + (0 * NV + q) * L::NFA;
-            const float* Y = Fs + (1 * NV + q) * L::NFA;
-            const float* Z = Fs + (2 * NV + q) * L::NFA;
-            float acc = -__fmul_rn(X[fx + 1] - X[fx], Ax);
-            acc = __fmaf_rn(-(Y[fy + 8] - Y[fy]), Ay, acc);
-            acc = __fmaf_rn(-(Z[fz + 64] - Z[fz]), Az, acc);
-            a.out[q * m.plane + cell] = cell_out(a, in, q, acc, dt);
-        }
-    }
-}
-
-// whether a gated tile is linear along all three axes and at all six seams (the seam rule of mixed_axis)
-__device__ __forceinline__ bool tile_all_linear(const StageArgs& a, int b, const int o3[3]) {
-    const long long nt3 = (long long)a.tiles[0] * a.tiles[1] * a.tiles[2];
-    bool lin = true;
-#pragma unroll
-    for (int A = 0; A < 3; ++A) {
-        const unsigned char* fl = a.sens_flags + A * nt3;
-        const int nt = a.tiles[A];
-        const int st = A == 0 ? 1 : (A == 1 ? a.tiles[0] : a.tiles[0] * a.tiles[1]);
-        const int ta = A == 0 ? b % a.tiles[0] : (A == 1 ? (b / a.tiles[0]) % a.tiles[1] : b / (a.tiles[0] * a.tiles[1]));
-        const bool wrap_lo = a.bc.halo[2 * A] == kHaloWrap, wrap_hi = a.bc.halo[2 * A + 1] == kHaloWrap;
-        lin = lin && fl[b] == 0;
-        lin = lin && (ta > 0 ? fl[b - st] == 0 : (wrap_lo ? fl[b + (nt - 1) * st] == 0 : true));
-        lin = lin && (ta < nt - 1 ? fl[b + st] == 0 : (wrap_hi ? fl[b - (nt - 1) * st] == 0 : true));
-    }
-    return lin;
-}
-
-template <int RIEMANN, int NT, bool GATED>
-__global__ void __launch_bounds__(NT, 3) mixed_stage_kernel_tma(const StageArgs a, const __grid_constant__ TmaMaps maps) {
-    using S = MixedShape<3, kWeno5, 8, 8, 8>;
-    using LO = MixedTmaShape<8, 8, 8>;
-    constexpr int NV = S::NV, NC = S::NC;
-    extern __shared__ __align__(128) unsigned char smem_b[];
-    double* red = reinterpret_cast<double*>(smem_b);
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem_b + CrossShape::BAR_OFF);
-    if (!*a.gate) return;
-    if (threadIdx.x == 0) {
-        tma::mbar_init(bar, 1);
-        tma::fence_mbar_init();
-    }
-    __syncthreads();
-    const Mesh& m = a.m;
-    const int tid = threadIdx.x, b = blockIdx.x + a.b0;
-    const int o3[3] = {(b % a.tiles[0]) * 8, ((b / a.tiles[0]) % a.tiles[1]) * 8, (b / (a.tiles[0] * a.tiles[1])) * 8};
-    float smax = 0.0f;
-    unsigned phase = 0;
-    bool cross = false;
-    if constexpr (GATED) cross = tile_all_linear(a, b, o3);
-    if (cross) {
-        cross_tile<RIEMANN, NT>(a, maps, smem_b, o3, phase, smax);
-    } else {
-        prefetch_epilogue<NT>(a, o3);
-        float* P = reinterpret_cast<float*>(smem_b + LO::P_OFF);
-        float* acc = reinterpret_cast<float*>(smem_b + LO::ACC_OFF);
-        unsigned char* Sf = smem_b + LO::SF_OFF;
-        float* WL = reinterpret_cast<float*>(smem_b + LO::STG_OFF);
-        float* WR = WL + NV * S::NF;
-        const GasF ef = gas_f(a.eos);
-        const float sb = (float)a.shock_blend, weps = (float)a.weno_eps;
-        mixed_axis<0, 3, kWeno5, RIEMANN, 8, 8, 8, NT, GATED, false, true>(a, ef, sb, weps, P, WL, WR, acc, Sf, o3, smax, maps.m, bar, &phase);
-        mixed_axis<1, 3, kWeno5, RIEMANN, 8, 8, 8, NT, GATED, false, true>(a, ef, sb, weps, P, WL, WR, acc, Sf, o3, smax, maps.m, bar, &phase);
-        mixed_axis<2, 3, kWeno5, RIEMANN, 8, 8, 8, NT, GATED, false, true>(a, ef, sb, weps, P, WL, WR, acc, Sf, o3, smax, maps.m, bar, &phase);
-        const double dt = a.ctl->dt;
-        for (int c = tid; c < NC; c += NT) {
-            const int c3[3] = {c % 8, (c / 8) % 8, c / 64};
-            const int g3[3] = {o3[0] + c3[0], o3[1] + c3[1], o3[2] + c3[2]};
-            if (g3[0] >= m.nx || g3[1] >= m.ny || g3[2] >= m.nz) continue;
-            const long long cell = ((long long)g3[2] * m.ny + g3[1]) * m.nx + g3[0];
-            CellIn<NV> in;
-            cell_load(a, cell, in);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) a.out[q * m.plane + cell] = cell_out(a, in, q, acc[q * NC + c], dt);
-        }
-    }
-    const double bm = block_max<NT>((double)smax, red);
     if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
 }
 
