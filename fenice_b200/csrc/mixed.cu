@@ -82,24 +82,21 @@ MixedStage mixed_stage_gated(int dim, int riemann, bool full) {
     return full ? pick_gated<2, true>(riemann) : pick_gated<2, false>(riemann);
 }
 
-// the FP32 viscous sweep: 384 threads per 8x8x8 tile (1.15 ms per launch at 256^3 against 1.28 with 192 threads); the
-// instantiation without the ghost rules and wall tests when every side of the launch is periodic or a part interface
+// the FP32 viscous sweep: the marching kernel where every side of the launch wraps or is a part interface and no body is
+// immersed, else 8x8x8 tiles of 384 threads
 constexpr int kMixedViscNT = 384;
 cudaError_t mixed_viscous_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(mixed_viscous_kernel<8, 8, 8, kMixedViscNT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(mixed_viscous_kernel<8, 8, 8, kMixedViscNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)MixedViscShape<8, 8, 8>::SMEM_BYTES);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mixed_viscous_kernel<8, 8, 8, kMixedViscNT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)MixedViscShape<8, 8, 8>::SMEM_BYTES);
+        e = cudaFuncSetAttribute(mixed_viscous_march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscMarchShape::SMEM_BYTES);
     return e;
 }
 cudaError_t mixed_viscous_launch(const ViscArgs& a, int nblocks, cudaStream_t s) {
-    bool walls = false;
-    for (int side = 0; side < 6; ++side) walls = walls || !a.through[side];
-    if (walls)
-        mixed_viscous_kernel<8, 8, 8, kMixedViscNT, true><<<nblocks, kMixedViscNT, MixedViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
-    else
-        mixed_viscous_kernel<8, 8, 8, kMixedViscNT, false><<<nblocks, kMixedViscNT, MixedViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
+    bool march = !a.bc.slot;
+    for (int side = 0; side < 6; ++side) march = march && a.through[side];
+    if (march) return visc_march_launch(a, nblocks, s);
+    mixed_viscous_kernel<8, 8, 8, kMixedViscNT><<<nblocks, kMixedViscNT, MixedViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
     return cudaGetLastError();
 }
 

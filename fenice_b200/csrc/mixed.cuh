@@ -490,11 +490,9 @@ __device__ __forceinline__ float f4c(float4 v, int a) { return a == 0 ? v.x : (a
 // periodic sides and part interfaces around it) reads its box without the ghost rules and solves its faces without the
 // wall tests; a tile wholly inside the mesh skips the test for faces beyond it. The four values a position, a face or a
 // cell carries sit together in one float4 (one shared-memory access each); each axis's balance shares a phase with the
-// next axis's gradients (six barriers per tile); WALLS = false drops the ghost rules and wall tests from launches whose
-// every side is periodic or a part interface. Measured at 256^3 (Taylor-Green): 0.77 ms per launch against 1.14 ms for
-// the first form (rho u_a in the box, 1 / rho, the general path for every tile), the same distance from the FP64 viscous
-// residual (1.24e-3 of its largest value, both).
-template <int TX, int TY, int TZ, int NT, bool WALLS = true>
+// next axis's gradients (six barriers per tile). Launches without walls, inlets, outlets or an immersed body march instead
+// (march.cuh).
+template <int TX, int TY, int TZ, int NT>
 __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) {
     using S = MixedViscShape<TX, TY, TZ>;
     constexpr int NC = S::NC, BX = S::BX, BY = S::BY, NB = S::NB;
@@ -517,7 +515,7 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
     auto bidx = [&](int i, int j, int k) { return ((k + 1) * BY + (j + 1)) * BX + (i + 1); };
     // whether a side of the tile lies on a side of the mesh that is neither periodic nor a part interface
     bool walls = false;
-    if constexpr (WALLS) {
+    {
 #pragma unroll
         for (int x = 0; x < 3; ++x) walls = walls || (o3[x] == 0 && !a.through[2 * x]) || (o3[x] + (x == 0 ? TX : (x == 1 ? TY : TZ)) >= n3[x] && !a.through[2 * x + 1]);
     }
@@ -529,11 +527,7 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
             if (a.periodic[x] && (g[x] < 0 || g[x] >= n3[x])) g[x] = ((g[x] % n3[x]) + n3[x]) % n3[x];
 #pragma unroll
         for (int x = 0; x < 3; ++x) g[x] = box_clamp(a, x, g[x], n3[x]);
-        St<double, 5> u;
-        if constexpr (WALLS)
-            u = walls ? padded_cons(a, g[0], g[1], g[2]) : cell_at(a, g[0], g[1], g[2]);
-        else
-            u = cell_at(a, g[0], g[1], g[2]);
+        const St<double, 5> u = walls ? padded_cons(a, g[0], g[1], g[2]) : cell_at(a, g[0], g[1], g[2]);
         double inv;
         const St<double, 5> w = prim_d(a.eos, u, inv);
         R[e] = (float)u[0];
@@ -585,7 +579,7 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
             bool inside = true;
             int xL = eL, xR = eR;
             bool phys = false, lo = false;
-            if (WALLS && walls) {
+            if (walls) {
                 const int g3[3] = {o3[0] + f3[0], o3[1] + f3[1], o3[2] + f3[2]};
 #pragma unroll
                 for (int x = 0; x < 3; ++x) inside = inside && (x == d ? g3[x] <= n3[x] : g3[x] < n3[x]);
@@ -603,7 +597,7 @@ __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) 
             }
             if (inside) {
                 float Gc[4];
-                if (WALLS && phys) {
+                if (phys) {
 #pragma unroll
                     for (int s = 0; s < 4; ++s) {
                         const int ga = GA[d][s], gb = GB[d][s];

@@ -250,8 +250,8 @@ template <int NV, int TX, int TY, int TZ, int NT> __device__ __forceinline__ voi
     }
 }
 
-template <int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool FULL = true>
-__global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
+template <int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool FULL = true, int MB = 1>
+__global__ void __launch_bounds__(NT, MB) stage_kernel(const StageArgs a) {
     using S = StageShape<DIM, RECON, TX, TY, TZ>;
     constexpr int NV = S::NV, NC = S::NC;
     extern __shared__ double smem[];
