@@ -318,11 +318,217 @@ __global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const St
     }
 }
 
+// The 2-D form: a CTA owns W columns of cells and marches along y. A thread keeps the six rows of its column around its y
+// face in registers; the row being solved lies in shared memory with the halo along x; per row a thread solves its low x
+// face and its high y face in one loop with one copy of the face code. The last column's cell belongs to the next CTA (its
+// low face is this CTA's last high face), so every thread has the same work. Tiles of the gate: 16 x 15 cells. 2048^2 quadrants
+// with the sensor: 342 us per launch in 16 x 15 tiles, 206 here.
+template <int W_> struct March2Shape {
+    static constexpr int W = W_, NT = W_, NHALO = 5, RP = W_ + 8, RAW = W_ + 8;
+    // doubles: red [32], raw row [4][RAW] (the column, three rows ahead, then the halo of the next row), u [4][W], u0 [4][W],
+    // viscous residual [4][W]; floats: P [4][RP], FX [4][W]
+    static constexpr size_t SMEM_BYTES = 8 * (32 + 4 * RAW + 12 * W) + 4 * (4 * RP + 4 * W);
+};
+template <int RIEMANN, bool GATED, int W, int MB>
+__global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, const int z0, const int z1, const int lz, const int nslots) {
+    using S = March2Shape<W>;
+    constexpr int NV = 4, RP = S::RP, RAW = S::RAW;
+    extern __shared__ double smem_d[];
+    double* red = smem_d;
+    double* Rc = smem_d + 32;
+    double* Ru = Rc + 4 * RAW;
+    double* R0 = Ru + 4 * W;
+    double* Rv = R0 + 4 * W;
+    float* P = reinterpret_cast<float*>(Rv + 4 * W);
+    float* FX = P + 4 * RP;
+    if (!*a.gate) return;
+    const Mesh& m = a.m;
+    const GasF gas = gas_f(a.eos);
+    const float sb = (float)a.shock_blend, weps = (float)a.weno_eps;
+    const int tid = threadIdx.x, cta = blockIdx.x;
+    const int cx = (m.nx + W - 2) / (W - 1);
+    const int x0 = (cta % cx) * (W - 1), za = z0 + (cta / cx) * lz;
+    const int zb = za + lz < z1 ? za + lz : z1;
+    const int gx = x0 + tid;
+    const bool cell_in = tid < W - 1 && gx < m.nx, face_in = gx <= m.nx;
+    int cside, hside = -1, coff, hoff = 0;
+    coff = march_cell(a.bc, 0, gx, m.nx, cside);
+    const bool halo = tid < S::NHALO;
+    const int hx = tid < 3 ? tid - 3 : W + tid - 3;
+    if (halo) hoff = march_cell(a.bc, 0, x0 + hx, m.nx, hside);
+    auto prim = [&](const double* raw, long long stride, int side) {
+        St<double, NV> u;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) u[q] = raw[q * stride];
+        if (side >= 0) u = ghost_state(a.eos, a.bc, side, u);
+        double inv;
+        return prim_d(a.eos, u, inv);
+    };
+    auto fetch_core = [&](int g) {
+        int sy;
+        const double* src = a.U + (long long)march_cell(a.bc, 1, g, m.ny, sy) * m.nx + coff;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * RAW + tid, src + q * m.plane);
+    };
+    auto fetch_halo = [&](int g) {
+        const double* src = a.U + (long long)g * m.nx + hoff;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * RAW + W + tid, src + q * m.plane);
+    };
+    auto fetch_cell = [&](int g) {
+        const long long cell = (long long)g * m.nx + coff;
+        if (a.mode != kStoreR)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(Ru + q * W + tid, a.U + q * m.plane + cell);
+        if (a.mode == kCombine)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(R0 + q * W + tid, a.U0 + q * m.plane + cell);
+        if (a.Rv)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(Rv + q * W + tid, a.Rv + q * m.plane + cell);
+    };
+    auto tile_linear = [&](int axis, int x, int y) -> bool {   // (as the 3-D kernel's)
+        int p[2] = {x, y};
+        const int n2[2] = {m.nx, m.ny};
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            if (p[d] >= 0 && p[d] < n2[d]) continue;
+            if (a.bc.halo[2 * d + (p[d] < 0 ? 0 : 1)] != kHaloWrap) return true;
+            p[d] = ((p[d] % n2[d]) + n2[d]) % n2[d];
+        }
+        const long long t = (long long)(p[1] / 15) * a.tiles[0] + (p[0] >> 4);
+        return a.sens_flags[(long long)axis * a.tiles[0] * a.tiles[1] + t] == 0;
+    };
+    fetch_core(za + 3);
+    if (halo) fetch_halo(za);
+    if (cell_in) fetch_cell(za);
+    float r[NV][6];
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        int sy;
+        const double* src = a.U + (long long)march_cell(a.bc, 1, za - 3 + p, m.ny, sy) * m.nx + coff;
+        const St<double, NV> w = prim(src, m.plane, sy >= 0 ? sy : cside);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) r[q][p] = (float)w[q];
+    }
+    const float Ax = (float)m.area[0], Ay = (float)m.area[1];
+    const double dt = a.ctl->dt;
+    float smax = 0.0f, Fl[NV] = {0.0f, 0.0f, 0.0f, 0.0f}, Fh[NV] = {0.0f, 0.0f, 0.0f, 0.0f};   // the y faces below and above the row
+    int lin = 0, tile_end = za - 1;   // bit 0, 1: the thread's x and y faces are linear; the row after which to look again
+#pragma unroll 1
+    for (int k = za - 1; k < zb; ++k) {
+        const bool first = k < za;
+        if (!first) {
+            cp_async_wait();
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+#pragma unroll
+                for (int p = 0; p < 5; ++p) r[q][p] = r[q][p + 1];
+            int sy;
+            march_cell(a.bc, 1, k + 3, m.ny, sy);
+            const St<double, NV> w = prim(Rc + tid, RAW, sy >= 0 ? sy : cside);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                r[q][5] = (float)w[q];
+                P[q * RP + tid + 3] = r[q][2];
+            }
+            if (halo) {
+                const St<double, NV> h = prim(Rc + W + tid, RAW, hside);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) P[q * RP + hx + 3] = (float)h[q];
+            }
+            if (k + 1 < zb) {
+                fetch_core(k + 4);
+                if (halo) fetch_halo(k + 1);
+            }
+        }
+        if constexpr (GATED) {
+            if (k >= tile_end) {   // (the y face above a tile's last row looks at the next tile)
+                lin = (tile_linear(0, gx - 1, k) && tile_linear(0, gx, k) ? 1 : 0) | (tile_linear(1, gx, k) && tile_linear(1, gx, k + 1) ? 2 : 0);
+                const int last = k < 0 ? -1 : k / 15 * 15 + 14;
+                tile_end = k < last ? last : last + 1;
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int it = first ? 1 : 0; it < 2; ++it) {
+            float c[NV][6];   // rho, p, the normal velocity, the other one
+            if (it == 1) {
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    c[0][p] = r[0][p];
+                    c[1][p] = r[3][p];
+                    c[2][p] = r[2][p];
+                    c[3][p] = r[1][p];
+                }
+            } else {
+                const float* b = P + tid;
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    c[0][p] = b[p];
+                    c[1][p] = b[3 * RP + p];
+                    c[2][p] = b[RP + p];
+                    c[3][p] = b[2 * RP + p];
+                }
+            }
+            float L[NV], R[NV];
+            if (GATED && (lin >> it & 1)) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) lin5_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], L[q], R[q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) weno5z_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], weps, L[q], R[q]);
+            }
+            float vL[2] = {L[2], L[3]}, vR[2] = {R[2], R[3]}, Fm, Fe, Fv[2];
+            const float s = riemann_f<RIEMANN>(gas, sb, L[0], L[1], vL, R[0], R[1], vR, Fm, Fe, Fv);
+            if ((it == 1 ? cell_in : face_in) && s > smax) smax = s;
+            if (it == 0) {
+                FX[tid] = Fm;
+                FX[W + tid] = Fv[0];
+                FX[2 * W + tid] = Fv[1];
+                FX[3 * W + tid] = Fe;
+            } else {
+                Fh[0] = Fm;
+                Fh[1] = Fv[1];
+                Fh[2] = Fv[0];
+                Fh[3] = Fe;
+            }
+        }
+        __syncthreads();
+        if (!first && cell_in) {
+            const long long cell = (long long)k * m.nx + coff;
+            CellIn<NV> in;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                in.u[q] = a.mode != kStoreR ? Ru[q * W + tid] : 0.0;
+                in.u0[q] = a.mode == kCombine ? R0[q * W + tid] : 0.0;
+                in.rv[q] = a.Rv ? Rv[q * W + tid] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                float acc = -__fmul_rn(FX[q * W + tid + 1] - FX[q * W + tid], Ax);
+                acc = __fmaf_rn(-(Fh[q] - Fl[q]), Ay, acc);
+                a.out[q * m.plane + cell] = cell_out(a, in, q, acc, dt);
+            }
+            if (k + 1 < zb) fetch_cell(k + 1);
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q) Fl[q] = Fh[q];
+    }
+    const double bm = block_max<W>((double)smax, red);
+    if (tid == 0) {
+        if (a.fin.kind == kFinNone)
+            for (int i = cta; i < nslots; i += gridDim.x) a.blockmax[a.b0 + i] = i == cta ? bm : 0.0;
+        else
+            stage_finish(a.fin, nullptr, 0, bm);
+    }
+}
+
 // Whether a launch can march: a lean WENO5-Z run without an immersed body whose every side wraps or has a ghost slab (no
 // first-order boundary faces).
-inline bool can_march(const StageArgs& a) {
+inline bool can_march(const StageArgs& a, int dim) {
     bool ok = !a.bc.solid && !a.bc.slot;
-    for (int s = 0; s < 6; ++s) ok = ok && (a.bc.halo[s] == kHaloWrap || a.bc.halo[s] == kHaloSlab);
+    for (int s = 0; s < 2 * dim; ++s) ok = ok && (a.bc.halo[s] == kHaloWrap || a.bc.halo[s] == kHaloSlab);
     return ok;
 }
 // The planes a CTA marches over, for `cols` column blocks and nz planes: the count that gives the fewest rounds of the
@@ -354,6 +560,24 @@ template <int RIEMANN, bool GATED> struct MarchK {
         const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
         a.fin.ctas = ctas;
         mixed_march_kernel<RIEMANN, GATED><<<ctas, MarchShape::NT, MarchShape::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
+        return cudaGetLastError();
+    }
+};
+
+// `nblocks` 16x15 tiles from a.b0, whole rows of tiles
+constexpr int kMarch2W = 128, kMarch2CTAs = 5;
+template <int RIEMANN, bool GATED> struct March2K {
+    using S = March2Shape<kMarch2W>;
+    static constexpr auto kern = mixed_march2_kernel<RIEMANN, GATED, kMarch2W, kMarch2CTAs>;
+    static cudaError_t prepare() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES); }
+    static cudaError_t launch(const StageArgs& a0, int nblocks, cudaStream_t s) {
+        StageArgs a = a0;
+        const int z0 = a.b0 / a.tiles[0] * 15, z_end = (a.b0 + nblocks) / a.tiles[0] * 15, z1 = z_end < a.m.ny ? z_end : a.m.ny;
+        const int cols = (a.m.nx + S::W - 2) / (S::W - 1);
+        const int lz = march_planes(cols, z1 - z0, a.fin.kind == kFinNone ? 15 : 4, kMarch2CTAs);
+        const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
+        a.fin.ctas = ctas;
+        kern<<<ctas, S::NT, S::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
         return cudaGetLastError();
     }
 };

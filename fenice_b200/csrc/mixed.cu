@@ -13,8 +13,9 @@ template <int DIM> struct MTile;
 template <> struct MTile<3> { static constexpr int X = 8, Y = 8, Z = 8, NT = 384; };
 template <> struct MTile<2> { static constexpr int X = 16, Y = 15, Z = 1, NT = 256; };
 
-// the marching kernel (march.cuh): the 3-D WENO5-Z lean kernels, where can_march
-template <int DIM, int RECON, bool FULL> constexpr bool kHasMarch = DIM == 3 && RECON == kWeno5 && !FULL;
+// the marching kernels (march.cuh): the WENO5-Z lean kernels, where can_march
+template <int DIM, int RECON, bool FULL> constexpr bool kHasMarch = RECON == kWeno5 && !FULL;
+template <int DIM, int RIEMANN, bool GATED> using MarchOf = std::conditional_t<DIM == 3, MarchK<RIEMANN, GATED>, March2K<RIEMANN, GATED>>;
 
 template <int DIM, int RECON, int RIEMANN, bool FULL> struct MixedK {
     using T = MTile<DIM>;
@@ -23,12 +24,12 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct MixedK {
         cudaError_t e = cudaFuncSetAttribute(mixed_stage_kernel<DIM, RECON, RIEMANN, T::X, T::Y, T::Z, T::NT, false, FULL>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
         if constexpr (kHasMarch<DIM, RECON, FULL>)
-            if (e == cudaSuccess) e = MarchK<RIEMANN, false>::prepare();
+            if (e == cudaSuccess) e = MarchOf<DIM, RIEMANN, false>::prepare();
         return e;
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
         if constexpr (kHasMarch<DIM, RECON, FULL>)
-            if (can_march(a)) return MarchK<RIEMANN, false>::launch(a, nblocks, s);
+            if (can_march(a, DIM)) return MarchOf<DIM, RIEMANN, false>::launch(a, nblocks, s);
         mixed_stage_kernel<DIM, RECON, RIEMANN, T::X, T::Y, T::Z, T::NT, false, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
@@ -42,12 +43,12 @@ template <int DIM, int RIEMANN, bool FULL> struct GatedK {
         cudaError_t e = cudaFuncSetAttribute(mixed_stage_kernel<DIM, kWeno5, RIEMANN, T::X, T::Y, T::Z, T::NT, true, FULL>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
         if constexpr (kHasMarch<DIM, kWeno5, FULL>)
-            if (e == cudaSuccess) e = MarchK<RIEMANN, true>::prepare();
+            if (e == cudaSuccess) e = MarchOf<DIM, RIEMANN, true>::prepare();
         return e;
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
         if constexpr (kHasMarch<DIM, kWeno5, FULL>)
-            if (can_march(a)) return MarchK<RIEMANN, true>::launch(a, nblocks, s);
+            if (can_march(a, DIM)) return MarchOf<DIM, RIEMANN, true>::launch(a, nblocks, s);
         mixed_stage_kernel<DIM, kWeno5, RIEMANN, T::X, T::Y, T::Z, T::NT, true, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }

@@ -250,7 +250,7 @@ template <int NV, int TX, int TY, int TZ, int NT> __device__ __forceinline__ voi
     }
 }
 
-template <int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool FULL = true, int MB = 1>
+template <int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool FULL = true, int MB = DIM == 3 ? 2 : 1>
 __global__ void __launch_bounds__(NT, MB) stage_kernel(const StageArgs a) {
     using S = StageShape<DIM, RECON, TX, TY, TZ>;
     constexpr int NV = S::NV, NC = S::NC;
