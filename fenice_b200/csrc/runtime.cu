@@ -517,7 +517,24 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct StageK {
                                     (int)S::SMEM_BYTES);
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
+        if constexpr (DIM == 2 && RECON != kFirstOrder && !FULL)
+            if (!a.bc.solid) return launch2d(a, nblocks, s);
         stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL><<<nblocks, Tl::NT, S::SMEM_BYTES, s>>>(a);
+        return cudaGetLastError();
+    }
+    // the one-pass kernel, over the rows of the launch's tiles. A launch whose tiles do not fill half the SMs' places takes
+    // tiles a third as high (where its CTAs need not be its tiles: the speeds folded into the control block).
+    static cudaError_t launch2d(const StageArgs& a, int nblocks, cudaStream_t s) {
+        const int row0 = a.b0 / a.tiles[0] * Tl::Y, row_end = (a.b0 + nblocks) / a.tiles[0] * Tl::Y, row1 = row_end < a.m.ny ? row_end : a.m.ny;
+        if (a.fin.kind != kFinNone && nblocks < 148 * 2) {
+            constexpr int TY = 5, NT = 192;
+            StageArgs b = a;
+            b.fin.ctas = a.tiles[0] * ((row1 - row0 + TY - 1) / TY);
+            stage2d_kernel<RECON, RIEMANN, Tl::X, TY, NT, 3><<<b.fin.ctas, NT, Stage2Shape<RECON, Tl::X, TY>::SMEM_BYTES, s>>>(b, row0, row1, a.tiles[0]);
+        } else {
+            stage2d_kernel<RECON, RIEMANN, Tl::X, Tl::Y, Tl::NT, 2><<<nblocks, Tl::NT, Stage2Shape<RECON, Tl::X, Tl::Y>::SMEM_BYTES, s>>>(a, row0, row1,
+                                                                                                                                  a.tiles[0]);
+        }
         return cudaGetLastError();
     }
 };
