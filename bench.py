@@ -436,7 +436,7 @@ def batch_arm(args, world, rank, local):
         bt, _, _ = batch_timed(params, states, prec, (shape, cps), local, timing=True)
         tm = bt.timing()
         bt.close()
-        sched = {"tile": [[64, 1], [128, 1], [256, 1], [16, 15]][shape], "ctas_per_sm": cps, "autotune_stage_ms": stage_ms}
+        sched = {"tile": [[63, 1], [127, 1], [255, 1], [16, 15]][shape], "ctas_per_sm": cps, "autotune_stage_ms": stage_ms}
         mixed_schedule = (shape, cps)
         stage_avg = tm["stage_ms"] / max(tm["stage_launches"], 1)
         # algorithmic bytes of one stage launch, averaged over the run: the cells of the running problems per launch

@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(1024) k_batch_end(const BatchProb* prob, Batch
     __shared__ int sum[1024];
     __shared__ int nact[1024];
     const int tid = threadIdx.x;
+    int dropped = 0;
     if (nstages > 0)
         for (int p = tid; p < n; p += 1024) {
             BatchCtl& c = ctl[p];
@@ -61,10 +62,12 @@ __global__ void __launch_bounds__(1024) k_batch_end(const BatchProb* prob, Batch
                     c.steps += 1;
                     c.active = (c.t < c.t_end) && (c.max_steps <= 0 || c.steps < c.max_steps) && c.status == 0;
                 }
+                dropped |= !c.active;
             }
             c.s_bits[0] = c.s_bits[1] = c.s_bits[2] = 0ull;
         }
-    __syncthreads();
+    // a step that ended no problem leaves the list as it is (512 tubes: 15 -> 5 us)
+    if (!__syncthreads_or(dropped) && nstages > 0) return;
     // thread t lists the problems [t per, (t + 1) per)
     const int per = (n + 1023) / 1024, p0 = tid * per, p1 = min(n, p0 + per);
     int cnt = 0, act = 0;
@@ -115,13 +118,18 @@ __global__ void k_batch_dt_axpy(const BatchProb* prob, BatchCtl* ctl, const Batc
         const long long off = prob[it.prob].off;
         const int tx = (m.nx + TX - 1) / TX;
         const int i0 = (it.tile % tx) * TX, j0 = (it.tile / tx) * TY;
-        const int nc = TX * TY;
-        for (int k = threadIdx.x; k < 4 * nc; k += blockDim.x) {
-            const int q = k / nc, cc = k % nc;
-            const int i = i0 + cc % TX, j = j0 + cc / TX;
+        for (int k = threadIdx.x; k < TX * TY; k += blockDim.x) {   // a cell per thread, its four variables' loads in flight together
+            const int i = i0 + k % TX, j = j0 + k / TX;
             if (i >= m.nx || j >= m.ny) continue;
-            const long long e = off + q * m.plane + (long long)j * m.nx + i;
-            out[e] = a[e] + dt * r[e];
+            const long long e = off + (long long)j * m.nx + i;
+            double av[4], rv[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                av[q] = a[e + q * m.plane];
+                rv[q] = r[e + q * m.plane];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) out[e + q * m.plane] = av[q] + dt * rv[q];
         }
     }
 }
@@ -225,7 +233,7 @@ struct fvg_batch {
     bool kern_ok[kBatchShapes] = {};
     int shape = -1, ctas_per_sm = 0, grid = 0, sms = 148;
     cudaGraphExec_t graph = nullptr;
-    int graph_steps = 8;
+    int graph_steps = 4;
     bool timing = false;
     std::vector<cudaEvent_t> ev;
     size_t ev_used = 0;
@@ -336,13 +344,13 @@ cudaError_t enqueue_end(fvg_batch* b, int nstages) {
 cudaError_t enqueue_step(fvg_batch* b) {
     cudaError_t e;
     const BatchShape sh = kBatchShape[b->shape];
-    const int ag = b->grid;
+    const int ag = 148 * 16, an = sh.nt;   // (its CTAs keep nothing from item to item: as many as fill the SMs)
     if ((e = launch_stage(b, stage_args(b, b->U, nullptr, b->R, kStoreR, 0, 0, 0)))) return e;
     if (b->scheme == FVG_TS_EULER) {
-        k_batch_dt_axpy<<<ag, 256, 0, b->stream>>>(b->d_prob, b->d_ctl, b->d_work, b->d_nwork, sh.tx, sh.ty, b->U, b->U, b->R);
+        k_batch_dt_axpy<<<ag, an, 0, b->stream>>>(b->d_prob, b->d_ctl, b->d_work, b->d_nwork, sh.tx, sh.ty, b->U, b->U, b->R);
         return enqueue_end(b, 1);
     }
-    k_batch_dt_axpy<<<ag, 256, 0, b->stream>>>(b->d_prob, b->d_ctl, b->d_work, b->d_nwork, sh.tx, sh.ty, b->Ut, b->U, b->R);
+    k_batch_dt_axpy<<<ag, an, 0, b->stream>>>(b->d_prob, b->d_ctl, b->d_work, b->d_nwork, sh.tx, sh.ty, b->Ut, b->U, b->R);
     if (b->scheme == FVG_TS_SSPRK2) {
         if ((e = launch_stage(b, stage_args(b, b->Ut, b->U, b->U, kCombine, 0.5, 0.5, 1)))) return e;
         return enqueue_end(b, 2);
@@ -653,6 +661,7 @@ int fvg_batch_run(fvg_batch* b, double t_end, int max_steps, long long* cell_sta
             ev_flush(b);
         }
         if (k > 0 && b->h_remaining[(k - 1) & 1] == 0) break;
+        if (max_steps > 0 && (k + 1) * b->graph_steps >= max_steps) break;   // every problem has taken its steps
     }
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);

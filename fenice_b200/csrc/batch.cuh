@@ -79,12 +79,21 @@ __device__ __forceinline__ void batch_stage_max(BatchCtl* c, int stage, double s
     if (s > 0.0) atomicMax(&c->s_bits[stage], (unsigned long long)__double_as_longlong(s));
 }
 
-// Tile shapes of the batched stage kernels (the autotuner's choices): cells along x and y, threads per CTA.
+// The work items of this CTA: a run of consecutive ones, so that most follow another of the same problem and share its
+// arguments and its speed reduction (items dealt out in turn rebuilt both for every tile).
+__device__ __forceinline__ void batch_share(int nw, int& w0, int& w1) {
+    w0 = (int)((long long)nw * blockIdx.x / gridDim.x);
+    w1 = (int)((long long)nw * (blockIdx.x + 1) / gridDim.x);
+}
+
+// Tile shapes of the batched stage kernels (the autotuner's choices): cells along x and y, threads per CTA. A row tile has
+// one face per thread, one more than it has cells, so that its faces are one round of the CTA (with a cell per thread, the
+// last face took a round of its own).
 struct BatchShape {
     int tx, ty, nt;
 };
 constexpr int kBatchShapes = 4;
-constexpr BatchShape kBatchShape[kBatchShapes] = {{64, 1, 64}, {128, 1, 128}, {256, 1, 256}, {16, 15, 256}};
+constexpr BatchShape kBatchShape[kBatchShapes] = {{63, 1, 64}, {127, 1, 128}, {255, 1, 256}, {16, 15, 256}};
 
 // Whether the y sweep of a work item takes the thin path: a one-cell-high mesh (a shock tube) whose bottom and top sides
 // have no halo. Both y faces of every column are then first-order boundary faces, whose states the general sweep takes
@@ -108,6 +117,18 @@ __device__ __forceinline__ void thin_y_fp64(const StageArgs& a, double* __restri
         if constexpr (RECON != kFirstOrder) {
             UL = round_trip(a.eos, UL);
             UR = round_trip(a.eos, UR);
+        }
+        if (same) {
+            // both faces lie between the cell's state and itself: their fluxes cancel, their speed remains (face_flux's for
+            // equal states; the low-Mach scaling of no jump leaves it)
+            double inv;
+            const St<double, 4> W = c2p(a.eos, UL, inv);
+            const double cs = sound_speed_inv(a.eos, W[3], inv);
+            const double s = vmax(fabs(W[2] - cs), fabs(W[2] + cs));
+            if (isfinite(s)) {
+                if (s > smax) smax = s;
+                continue;
+            }
         }
         const double sb = face_flux<RIEMANN>(a.eos, a.shock_blend, UL, UR, 1, Fb);
         double st = sb;
@@ -146,15 +167,24 @@ __global__ void __launch_bounds__(NT) batch_stage_kernel(const BatchArgs b) {
     unsigned char* Sf = reinterpret_cast<unsigned char*>(red + 32);
     __shared__ StageArgs sa;
     const int tid = threadIdx.x;
-    const int nw = *b.nwork;
-    for (int w = blockIdx.x; w < nw; w += gridDim.x) {
+    int w0, w1, cur = -1;
+    batch_share(*b.nwork, w0, w1);
+    double smax = 0.0;
+    for (int w = w0; w < w1; ++w) {
         const BatchWork it = b.work[w];
-        if (tid == 0) batch_item_args(b, b.prob[it.prob], sa);
+        if (it.prob != cur) {
+            if (cur >= 0) {
+                const double bm = block_max<NT>(smax, red);
+                if (tid == 0) batch_stage_max(&b.ctl[cur], b.stage, bm);
+            }
+            if (tid == 0) batch_item_args(b, b.prob[it.prob], sa);
+            cur = it.prob;
+            smax = 0.0;
+        }
         __syncthreads();
         const Mesh& m = sa.m;
         const int tx = (m.nx + TX - 1) / TX;
         const int o3[3] = {(it.tile % tx) * TX, (it.tile / tx) * TY, 0};
-        double smax = 0.0;
         stage_axis<0, 2, RECON, RIEMANN, TX, TY, 1, NT, false>(sa, P, WL, WR, acc, Sf, o3, smax);
         bool thin = false;
         if constexpr (TY == 1) thin = thin_y(m, sa.bc);
@@ -181,9 +211,10 @@ __global__ void __launch_bounds__(NT) batch_stage_kernel(const BatchArgs b) {
                 sa.out[e] = o;
             }
         }
+    }
+    if (cur >= 0) {
         const double bm = block_max<NT>(smax, red);
-        if (tid == 0) batch_stage_max(&b.ctl[it.prob], b.stage, bm);
-        __syncthreads();
+        if (tid == 0) batch_stage_max(&b.ctl[cur], b.stage, bm);
     }
 }
 

@@ -363,7 +363,8 @@ __device__ __forceinline__ void mixed_axis(const StageArgs& a, const GasF& ef, f
                     if (hi_face) c3[axis] = na - 1;
                     St<double, NV> UL, UR;
                     side_states<NV, FULL>(m, a.bc, a.eos, a.U, lo_face ? lo_side : hi_side, c3[0], c3[1], c3[2], UL, UR);
-                    const St<double, NV> dl = c2p(a.eos, UL), dr = c2p(a.eos, UR);
+                    double inv;
+                    const St<double, NV> dl = prim_d(a.eos, UL, inv), dr = prim_d(a.eos, UR, inv);
 #pragma unroll
                     for (int q = 0; q < NV; ++q) {
                         wl[q] = (float)dl[q];

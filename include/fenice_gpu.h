@@ -338,7 +338,7 @@ int fvg_batch_download(fvg_batch* b, double* U, size_t ncells);
 int fvg_batch_run(fvg_batch* b, double t_end, int max_steps, long long* cell_stages);
 /* problem i after a run: its time, steps taken and status (0 ok, 1 diverged) */
 int fvg_batch_problem(const fvg_batch* b, int i, double* t, int* steps, int* status);
-/* Autotuner: times one stage of every problem for each tile shape the library has (64x1, 128x1, 256x1, 16x15 cells)
+/* Autotuner: times one stage of every problem for each tile shape the library has (63x1, 127x1, 255x1, 16x15 cells)
  * and each persistent grid (1 .. the CTAs an SM holds, per SM) and keeps the fastest; returns the choice and its
  * stage time in ms. fvg_batch_set_schedule sets one by hand (ctas_per_sm 0: as many as an SM holds). */
 int fvg_batch_autotune(fvg_batch* b, int* shape, int* ctas_per_sm, double* stage_ms);
