@@ -270,20 +270,48 @@ __device__ __forceinline__ void weno5z_pair(float c0, float c1, float c2, float 
 // ------------------------------------------------------------------ HLLC (Toro) with Einfeldt bounds (Schemes.cpp:116-200)
 template <typename T> __device__ __forceinline__ T safe_denom(T x) { return copysign(vmax(fabs(x), Num<T>::denom_eps), x); }
 
+// The velocity along `axis` of a primitive state (a choice, not an index: the axis may be a run-time value).
+template <typename T, int NV> __device__ __forceinline__ T normal_velocity(const St<T, NV>& W, int axis) {
+    return axis == 0 ? W[1] : (NV == 4 || axis == 1 ? W[2] : W[NV - 1]);
+}
 // One side's Euler flux along `axis`.
 template <typename T, int NV>
 __device__ __forceinline__ void hllc_side_flux(const St<T, NV>& W, T E, int axis, St<T, NV>& F) {
     constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
-    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
-    const T rho = W[0], p = W[3], Vn = W[mn];
+    const T rho = W[0], p = W[3], Vn = normal_velocity(W, axis);
     F[0] = rho * Vn;
 #pragma unroll
     for (int a = 0; a < NA; ++a) {
         const int m = a == 0 ? 1 : (a == 1 ? 2 : 4);
-        F[m] = rho * W[m] * Vn;
+        const T f = rho * W[m] * Vn;
+        F[m] = a == axis ? f + p : f;
     }
-    F[mn] = F[mn] + p;
     F[3] = Vn * (rho * E + p);
+}
+
+// Whether the pressure jump |p_R - p_L| / min(p_L, p_R) may exceed the blend's threshold: false only where it is below it by
+// more than its rounding (most faces, which are spared the division).
+template <typename T> __device__ __forceinline__ bool may_blend(T p_L, T p_R, T shock_blend) {
+    return !(fabs(p_R - p_L) < T(0.999) * shock_blend * vmin(p_L, p_R));
+}
+// F with the share phi of the upwind or HLL flux blended in.
+template <typename T, int NV>
+__device__ __forceinline__ void hll_blend(T S_L, T S_R, T phi, const St<T, NV>& FL, const St<T, NV>& FR, const St<T, NV>& UL, const St<T, NV>& UR,
+                                          St<T, NV>& F) {
+    if (S_L >= T(0)) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) F[q] = (T(1) - phi) * F[q] + phi * FL[q];
+    } else if (S_R <= T(0)) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) F[q] = (T(1) - phi) * F[q] + phi * FR[q];
+    } else {
+        const T inv = T(1) / (S_R - S_L);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            const T fh = (S_R * FL[q] - S_L * FR[q] + S_L * S_R * (UR[q] - UL[q])) * inv;
+            F[q] = (T(1) - phi) * F[q] + phi * fh;
+        }
+    }
 }
 
 // The flux along `axis` (0, 1, 2) from the primitive (floored) and conservative states of both sides; returns max(|S_L|, |S_R|).
@@ -294,10 +322,9 @@ template <typename T, int NV>
 __device__ __forceinline__ T hllc_core(const St<T, NV>& WL, const St<T, NV>& WR, const St<T, NV>& UL, const St<T, NV>& UR, T inv_L,
                                        T inv_R, T c_L, T c_R, int axis, T shock_blend, St<T, NV>& F) {
     constexpr int NA = NV == 5 ? 3 : 2;   // velocity components
-    const int mn = axis == 0 ? 1 : (axis == 1 ? 2 : 4);
     const T rho_L = WL[0], p_L = WL[3];
     const T rho_R = WR[0], p_R = WR[3];
-    const T Vn_L = WL[mn], Vn_R = WR[mn];
+    const T Vn_L = normal_velocity(WL, axis), Vn_R = normal_velocity(WR, axis);
     const T S_L = vmin(Vn_L - c_L, Vn_R - c_R);
     const T S_R = vmax(Vn_L + c_L, Vn_R + c_R);
     const T num = rho_R * Vn_R * (S_R - Vn_R) - rho_L * Vn_L * (S_L - Vn_L) + p_L - p_R;
@@ -318,7 +345,7 @@ __device__ __forceinline__ T hllc_core(const St<T, NV>& WL, const St<T, NV>& WR,
     hllc_side_flux(W, E, axis, F);
     if (star) {
         const T S = right ? S_R : S_L;
-        const T rho = W[0], p = W[3], Vn = W[mn];
+        const T rho = W[0], p = W[3], Vn = right ? Vn_R : Vn_L;
         const T den_star = safe_denom(S - S_M);
         const T den_p = safe_denom(S - Vn);
         const T f = rho * (S - Vn) / den_star;
@@ -336,27 +363,14 @@ __device__ __forceinline__ T hllc_core(const St<T, NV>& WL, const St<T, NV>& WR,
     if (none)
 #pragma unroll
         for (int q = 0; q < NV; ++q) F[q] = T(0);
-    if (shock_blend > T(0)) {
+    if (shock_blend > T(0) && may_blend(p_L, p_R, shock_blend)) {
         const T s = fabs(p_R - p_L) / vmin(p_L, p_R);
         if (s > shock_blend) {
             const T phi = vmin((s - shock_blend) / shock_blend, T(1));
             St<T, NV> FL, FR;
             hllc_side_flux(WL, UL[3] * inv_L, axis, FL);
             hllc_side_flux(WR, UR[3] * inv_R, axis, FR);
-            if (S_L >= T(0)) {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) F[q] = (T(1) - phi) * F[q] + phi * FL[q];
-            } else if (S_R <= T(0)) {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) F[q] = (T(1) - phi) * F[q] + phi * FR[q];
-            } else {
-                const T inv = T(1) / (S_R - S_L);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) {
-                    const T fh = (S_R * FL[q] - S_L * FR[q] + S_L * S_R * (UR[q] - UL[q])) * inv;
-                    F[q] = (T(1) - phi) * F[q] + phi * fh;
-                }
-            }
+            hll_blend(S_L, S_R, phi, FL, FR, UL, UR, F);
         }
     }
     return vmax(fabs(S_L), fabs(S_R));

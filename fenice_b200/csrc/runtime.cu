@@ -512,14 +512,23 @@ template <> struct Tile<2> { static constexpr int X = 16, Y = 15, Z = 1, NT = 25
 template <int DIM, int RECON, int RIEMANN, bool FULL> struct StageK {
     using Tl = Tile<DIM>;
     using S = StageShape<DIM, RECON, Tl::X, Tl::Y, Tl::Z>;
+    // 3-D WENO3-Z / WENO5-Z without the code of FULL: the loop over the axes (stage3_kernel)
+    static constexpr bool kLoop = DIM == 3 && (RECON == kWeno3 || RECON == kWeno5) && !FULL;
     static cudaError_t prepare() {
-        return cudaFuncSetAttribute(stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)S::SMEM_BYTES);
+        if constexpr (kLoop)
+            return cudaFuncSetAttribute(stage3_kernel<RECON, RIEMANN, 512, FULL, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)Stage3Shape<RECON>::SMEM_BYTES);
+        else
+            return cudaFuncSetAttribute(stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)S::SMEM_BYTES);
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
         if constexpr (DIM == 2 && RECON != kFirstOrder && !FULL)
             if (!a.bc.solid) return launch2d(a, nblocks, s);
-        stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL><<<nblocks, Tl::NT, S::SMEM_BYTES, s>>>(a);
+        if constexpr (kLoop)
+            stage3_kernel<RECON, RIEMANN, 512, FULL, 2><<<nblocks, 512, Stage3Shape<RECON>::SMEM_BYTES, s>>>(a);
+        else
+            stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL><<<nblocks, Tl::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
     // the one-pass kernel, over the rows of the launch's tiles. A launch whose tiles do not fill half the SMs' places takes

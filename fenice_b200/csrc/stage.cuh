@@ -436,4 +436,207 @@ __global__ void __launch_bounds__(NT, MB) stage2d_kernel(const StageArgs a, cons
     if (tid == 0) stage_finish(a.fin, a.blockmax, a.b0 + cta, bm);
 }
 
+// The FP64 stage kernel of a 3-D mesh: the phases of stage_kernel on an 8x8x8 tile, in a loop over the axes whose body is
+// the only copy of the reconstruction and the Riemann solver (an unrolled copy per axis stalled on instruction fetch, 11 %
+// of the issue slots). A position of the extended tile or of the face grid is (s, u, v): s along the axis, u and v the other
+// two axes in increasing order; one slot is s * 65 + v * 8 + u (rows of 65 so that a row along s touches every bank).
+//
+// Bound by the latency of FP64 chains (a division is a chain of a dozen dependent operations): 512 threads, two CTAs per SM
+// (32 warps; 64 registers, some spilled) beat fewer warps with more registers. ms per launch at 128^3, WENO5-Z, low-Mach HLLC /
+// HLLC: the sweep with 256 threads 1.51 / 1.44, with 320 1.31 / 1.24; this loop with 256 1.52, 320 1.29 / 1.25, 384 1.30 / 1.21, 512
+// 1.24 / 1.16 (kept); a pair of lanes per face, one for each side, 1.37 / 1.32. MUSCL, whose faces have no WENO divisions, is no
+// faster in it (0.56 against 0.55): it keeps the sweep.
+template <int RECON> struct Stage3Shape {
+    static constexpr int NV = 5, H = RECON == kWeno5 ? 3 : (RECON == kFirstOrder ? 1 : 2);
+    static constexpr int ROW = 65, NS = 8 + 2 * H, EXT = NS * ROW, NF = 9 * 64, NC = 512;
+    static constexpr int FLAG_BYTES = (EXT + 7) / 8 * 8;
+    static constexpr size_t SMEM_BYTES = sizeof(double) * (NV * EXT + 2 * NV * NF + NV * NC + 32) + FLAG_BYTES;
+};
+template <int RECON, int RIEMANN, int NT, bool FULL, int MB>
+__global__ void __launch_bounds__(NT, MB) stage3_kernel(const StageArgs a) {
+    using S = Stage3Shape<RECON>;
+    constexpr int NV = 5, H = S::H, NC = S::NC, NF = S::NF, EXT = S::EXT, ROW = S::ROW;
+    extern __shared__ double smem[];
+    double* P = smem;                       // [NV][EXT]
+    double* WL = P + NV * EXT;              // [NV][NF]
+    double* WR = WL + NV * NF;              // [NV][NF]
+    double* acc = WR + NV * NF;             // [NV][NC]
+    double* red = acc + NV * NC;            // [32]
+    unsigned char* Sf = reinterpret_cast<unsigned char*>(red + 32);   // [EXT]
+    if (!*a.gate) return;
+    const Mesh& m = a.m;
+    const int tid = threadIdx.x;
+    const int b = blockIdx.x + a.b0;
+    const int o3[3] = {b % a.tiles[0] * 8, (b / a.tiles[0]) % a.tiles[1] * 8, b / (a.tiles[0] * a.tiles[1]) * 8};
+    double smax = 0.0;
+    prefetch_tile_rows<NV, 8, 8, 8, NT>(a, o3);
+#pragma unroll 1
+    for (int axis = 0; axis < 3; ++axis) {
+        const auto place = [&](int s, int u, int v, int& i, int& j, int& k) {   // mesh position of (s, u, v)
+            i = o3[0] + (axis == 0 ? s : u);
+            j = o3[1] + (axis == 1 ? s : (axis == 0 ? u : v));
+            k = o3[2] + (axis == 2 ? s : v);
+        };
+        // ---- 1. load (primitive; first order keeps the conservative state), x fastest
+        for (int e = tid; e < S::NS * 64; e += NT) {
+            int s, u, v, i, j, k;
+            if (axis == 0) {
+                s = e % S::NS;
+                u = (e / S::NS) & 7;
+                v = e / (S::NS * 8);
+            } else {
+                u = e & 7;
+                s = axis == 1 ? (e >> 3) % S::NS : e >> 6;
+                v = axis == 1 ? (e >> 3) / S::NS : (e >> 3) & 7;
+            }
+            const int slot = s * ROW + v * 8 + u;
+            place(s - H, u, v, i, j, k);
+            const St<double, NV> c = stencil_cons<3, NV, FULL>(m, a.bc, a.eos, a.U, i, j, k);
+            if constexpr (RECON == kWeno5)
+                if (a.bc.solid) Sf[slot] = stencil_solid<3>(m, a.bc, i, j, k);
+            if constexpr (RECON == kFirstOrder) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) P[q * EXT + slot] = c[q];
+            } else {
+                const St<double, NV> w = c2p(a.eos, c);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) P[q * EXT + slot] = w[q];
+            }
+        }
+        __syncthreads();
+        // ---- 2. face values: face t = f / 64 has its stencil at the rows t .. t + 2H - 1
+        if constexpr (RECON != kFirstOrder) {
+            for (int it = tid; it < NF * NV; it += NT) {
+                const int q = it / NF, f = it - q * NF, slot = (f >> 6) * ROW + (f & 63);
+                const double* c = P + q * EXT + slot;
+                double wl, wr;
+                if constexpr (RECON == kMuscl) {
+                    const double c0 = c[0], c1 = c[ROW], c2 = c[2 * ROW], c3 = c[3 * ROW];
+                    const double bb = c2 - c1;
+                    wl = c1 + 0.5 * limiter(a.limiter, c1 - c0, bb);
+                    wr = c2 - 0.5 * limiter(a.limiter, c3 - c2, bb);
+                } else if constexpr (RECON == kWeno3) {
+                    wl = weno3z(c[0], c[ROW], c[2 * ROW], a.weno_eps);
+                    wr = weno3z(c[3 * ROW], c[2 * ROW], c[ROW], a.weno_eps);
+                } else {
+                    const double c0 = c[0], c1 = c[ROW], c2 = c[2 * ROW], c3 = c[3 * ROW], c4 = c[4 * ROW], c5 = c[5 * ROW];
+                    bool four = false;   // a solid cell among the six: the four-cell WENO3-Z stencil (weno_line_states, Schemes.cpp:815-831)
+                    if (a.bc.solid)
+#pragma unroll
+                        for (int s6 = 0; s6 < 6; ++s6) four = four || Sf[slot + s6 * ROW] != 0;
+                    if (four) {
+                        wl = weno3z(c1, c2, c3, a.weno_eps);
+                        wr = weno3z(c4, c3, c2, a.weno_eps);
+                    } else {
+                        wl = weno5z(c0, c1, c2, c3, c4, a.weno_eps);
+                        wr = weno5z(c5, c4, c3, c2, c1, a.weno_eps);
+                    }
+                }
+                WL[q * NF + f] = wl;
+                WR[q * NF + f] = wr;
+            }
+            __syncthreads();
+        }
+        // ---- 3. fluxes, written over the face values: slot f of WL is read and written by the thread of face f only
+        const int na = axis == 0 ? m.nx : (axis == 1 ? m.ny : m.nz);
+        const int lo_side = 2 * axis, hi_side = 2 * axis + 1;
+        for (int f = tid; f < NF; f += NT) {
+            int i, j, k;
+            place(f >> 6, f & 7, (f >> 3) & 7, i, j, k);
+            const bool inside = i < m.nx + (axis == 0) && j < m.ny + (axis == 1) && k < m.nz + (axis == 2);
+            St<double, NV> F;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) F[q] = 0.0;
+            if (inside) {
+                const int t = axis == 0 ? i : (axis == 1 ? j : k);
+                const bool lo_face = t == 0 && a.bc.halo[lo_side] == kHaloNone;
+                const bool hi_face = t == na && a.bc.halo[hi_side] == kHaloNone;
+                St<double, NV> UL, UR;
+                if (lo_face || hi_face) {
+                    const int d = hi_face ? 1 : 0;
+                    side_states<NV, FULL>(m, a.bc, a.eos, a.U, lo_face ? lo_side : hi_side, i - (axis == 0 ? d : 0), j - (axis == 1 ? d : 0),
+                                          k - (axis == 2 ? d : 0), UL, UR);
+                    if constexpr (RECON != kFirstOrder) {
+                        UL = round_trip(a.eos, UL);
+                        UR = round_trip(a.eos, UR);
+                    }
+                } else if constexpr (RECON == kFirstOrder) {
+                    const int slot = (f >> 6) * ROW + (f & 63);   // the cell before the face, and the next row's after it
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) {
+                        UL[q] = P[q * EXT + slot];
+                        UR[q] = P[q * EXT + slot + ROW];
+                    }
+                } else {
+                    const int li = i - (axis == 0), lj = j - (axis == 1), lk = k - (axis == 2);
+                    if (FULL && a.fb && (fb_flagged<3>(m, a.bc, a.fb, li, lj, lk) || fb_flagged<3>(m, a.bc, a.fb, i, j, k))) {
+                        // next to a flagged cell: the two cells' states (the ghost of a side's halo beyond it)
+                        UL = stencil_cons<3, NV>(m, a.bc, a.eos, a.U, li, lj, lk);
+                        UR = stencil_cons<3, NV>(m, a.bc, a.eos, a.U, i, j, k);
+                    } else {
+                        St<double, NV> wl, wr;
+#pragma unroll
+                        for (int q = 0; q < NV; ++q) {
+                            wl[q] = WL[q * NF + f];
+                            wr[q] = WR[q * NF + f];
+                        }
+                        UL = p2c(a.eos, wl);
+                        UR = p2c(a.eos, wr);
+                    }
+                }
+                const double s = face_flux<RIEMANN>(a.eos, a.shock_blend, UL, UR, axis, F);
+                if (s > smax) smax = s;
+            }
+#pragma unroll
+            for (int q = 0; q < NV; ++q) WL[q * NF + f] = F[q];
+        }
+        __syncthreads();
+        // ---- 4. balance of this axis
+        const double A = axis == 0 ? m.area[0] : (axis == 1 ? m.area[1] : m.area[2]);
+        for (int c = tid; c < NC; c += NT) {
+            const int x = c & 7, y = (c >> 3) & 7, z = c >> 6;
+            const int fl = axis == 0 ? x * 64 + z * 8 + y : (axis == 1 ? y * 64 + z * 8 + x : c);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                const double d = WL[q * NF + fl + 64] * A - WL[q * NF + fl] * A;
+                acc[q * NC + c] = axis == 0 ? 0.0 - d : acc[q * NC + c] - d;
+            }
+        }
+        __syncthreads();
+    }
+    // ---- epilogue: the residual and the stage update
+    const double dt = a.ctl->dt;
+    for (int c = tid; c < NC; c += NT) {
+        const int g0 = o3[0] + (c & 7), g1 = o3[1] + ((c >> 3) & 7), g2 = o3[2] + (c >> 6);
+        if (g0 >= m.nx || g1 >= m.ny || g2 >= m.nz) continue;
+        const long long cell = ((long long)g2 * m.ny + g1) * m.nx + g0;
+        St<double, NV> r;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            r[q] = acc[q * NC + c] * m.inv_cell;
+            if (a.Rv) r[q] = r[q] + a.Rv[q * m.plane + cell];
+        }
+        // the body force, then the case's source terms, join after the viscous term (Simulation::assemble,
+        // cpp/src/Simulation.cpp:1038-1049; RhsSourceTerms in the order Simulation::setup adds them, :372-412)
+        if constexpr (FULL) {
+            if (a.bc.grav_on) add_body_force<NV>(a.bc, read_state<NV>(a.bc, a.U, m.plane, cell), r);
+            if (a.bc.src) add_source<NV>(a.bc, m.plane, cell, r);
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            const long long e = q * m.plane + cell;
+            double o;
+            if (a.mode == kStoreR)
+                o = r[q];
+            else if (a.mode == kAxpy)
+                o = a.U[e] + dt * r[q];
+            else
+                o = a.ca * a.U0[e] + a.cb * (a.U[e] + dt * r[q]);
+            a.out[e] = o;
+        }
+    }
+    const double bm = block_max<NT>(smax, red);
+    if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
+}
+
 }   // namespace fvg
