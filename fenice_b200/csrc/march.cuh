@@ -7,17 +7,18 @@
 // - a thread keeps the six planes of its column around its z face in registers; the plane being solved lies in shared
 //   memory with three cells around the columns, for the x and y faces (rows of 40 floats: a warp reads 32 neighbours of
 //   one row, no two on a bank);
-// - per plane a thread solves its low x, its low y and its high z face in one loop whose body is the only copy of the
-//   reconstruction and the Riemann solver (a copy per axis would not fit the instruction cache); a ninth warp solves the
-//   40 faces on the high sides of the columns;
+// - per plane a thread solves its low x, its low y and its high z face; the 40 faces on the high sides of the columns fall
+//   to two of the warps in turn;
+// - four of the five variables lie in one float4, so a stencil cell is two loads and its pairs (rho, p) and (u, v) are
+//   operands of packed operations as they stand;
 // - fluxes meet in shared memory, and the balance ((0 - x) - y) - z and the FP64 update finish the plane.
 // All global operands of a plane (the raw state three planes ahead, the raw halo of the next plane, U, U0 and the viscous
 // sums of the cell) are on their way to shared memory (cp.async, each thread its own values, so no barrier) while the plane
-// before is solved. Two CTAs per SM (288 threads, at most 112 registers, 87 KB of shared memory).
+// before is solved. Two CTAs per SM (256 threads, at most 128 registers, 77 KB of shared memory).
 //
-// What bounds it: instruction issue at 16 to 18 warps per SM (ncu at 192^3: 58 warp instructions per cell, issue 59 %, DRAM 18 %;
-// the tiled form with boxes by TMA took 80). Against that form, mixed + sensor at 256^3: 7.29 -> 7.17 ms per step; mixed at 64^3:
-// 225 -> 209 us per step.
+// What bounds it: instruction issue at 16 warps per SM (DRAM 18 %). Mixed + sensor at 256^3: 7.29 ms per step in 8x8x8 tiles with
+// boxes by TMA, 7.17 marching with scalar loads, a loop over the axes and a ninth warp (58 warp instructions per cell, issue
+// 59 % at 192^3, where the tiles took 80), 6.28 with the viscous sweep below, 5.58 in this form. Mixed at 64^3: 225, 209, 198, 183 us.
 #pragma once
 
 #include "mixed.cuh"
@@ -25,14 +26,53 @@
 namespace fvg {
 
 struct MarchShape {
-    static constexpr int W = 32, H = 8, NT = 288, NCOL = W * H;
-    static constexpr int PITCH = 40, PL = 14 * PITCH;             // a plane of P: rows y = -3 .. 10, x = -3 .. 34
+    static constexpr int W = 32, H = 8, NT = 256, NCOL = W * H;
+    static constexpr int PITCH = 40, PL = 14 * PITCH;             // a plane: rows y = -3 .. 10, x = -3 .. 34
     static constexpr int NHALO = 6 * W + 6 * H;                    // cells around the columns
-    static constexpr int FXP = 36, NFX = H * FXP, NFY = (H + 1) * W;
-    // doubles: red [32], the raw values on their way: core [5][256], halo [5][256], u [5][256], u0 [5][256]; then floats:
-    // the viscous sums [4][256], P [5][PL], FX [5][NFX], FY [5][NFY], FZ [2][5][256]
-    static constexpr size_t SMEM_BYTES = 8 * (32 + 20 * NCOL) + 4 * (4 * NCOL + 5 * PL + 5 * NFX + 5 * NFY + 10 * NCOL);
+    static constexpr int FXP = 33, NFX = H * FXP, NFY = (H + 1) * W;
+    // doubles: red [32], the raw values on their way: core [5][256], halo [5][256], u [5][256], u0 [5][256]; float4 (rho, p, u,
+    // v or the fluxes of rho, rho E, rho u, rho v): P [PL], FX [NFX], FY [NFY], FZ [2][256]; floats (w, or the flux of rho w):
+    // the same four, and the viscous sums [4][256]
+    static constexpr size_t SMEM_BYTES = 8 * (32 + 20 * NCOL) + 20 * (PL + NFX + NFY + 2 * NCOL) + 4 * 4 * NCOL;
 };
+// a cell's primitive state, or a face's fluxes, in the order of MarchShape
+struct March5 {
+    float4 a;
+    float w;
+};
+// the face along axis A from its six cells
+template <int A, int RIEMANN>
+__device__ __forceinline__ float march_face(const GasF& gas, float sb, float weps, bool linear, const March5 (&c)[6], March5& F) {
+    const auto lo = [&](int p) { return f2(c[p].a.x, c[p].a.y); };
+    const auto hi = [&](int p) { return f2(c[p].a.z, c[p].a.w); };
+    F2 l0, l1, r0, r1;
+    float lw, rw;
+    if (linear) {
+        l0 = lin5_f2(lo(0), lo(1), lo(2), lo(3), lo(4));
+        r0 = lin5_f2(lo(5), lo(4), lo(3), lo(2), lo(1));
+        l1 = lin5_f2(hi(0), hi(1), hi(2), hi(3), hi(4));
+        r1 = lin5_f2(hi(5), hi(4), hi(3), hi(2), hi(1));
+        lin5_pair(c[0].w, c[1].w, c[2].w, c[3].w, c[4].w, c[5].w, lw, rw);
+    } else {
+        l0 = weno5z_f2(lo(0), lo(1), lo(2), lo(3), lo(4), weps);
+        r0 = weno5z_f2(lo(5), lo(4), lo(3), lo(2), lo(1), weps);
+        l1 = weno5z_f2(hi(0), hi(1), hi(2), hi(3), hi(4), weps);
+        r1 = weno5z_f2(hi(5), hi(4), hi(3), hi(2), hi(1), weps);
+        weno5z_pair(c[0].w, c[1].w, c[2].w, c[3].w, c[4].w, c[5].w, weps, lw, rw);
+    }
+    float rL, pL, rR, pR, uL, vv, uR, vR_;
+    f2_get(l0, rL, pL);
+    f2_get(r0, rR, pR);
+    f2_get(l1, uL, vv);
+    f2_get(r1, uR, vR_);
+    const float L[3] = {uL, vv, lw}, R[3] = {uR, vR_, rw};
+    float vL[3] = {L[A], L[(A + 1) % 3], L[(A + 2) % 3]}, vR[3] = {R[A], R[(A + 1) % 3], R[(A + 2) % 3]}, Fv[3];
+    const float s = riemann_f<RIEMANN>(gas, sb, rL, pL, vL, rR, pR, vR, F.a.x, F.a.y, Fv);
+    F.a.z = Fv[(3 - A) % 3];
+    F.a.w = Fv[(4 - A) % 3];
+    F.w = Fv[(5 - A) % 3];
+    return s;
+}
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -61,8 +101,8 @@ __device__ __forceinline__ int march_cell(const Bc& bc, int axis, int g, int n, 
 // z0 .. z1: the planes of the launch; lz: planes per CTA (a multiple of 8 where the CTAs write blockmax). GATED: a face is
 // linear when the tiles of both its cells are linear along its axis (inside a tile: when the tile is), which is the seam
 // rule of mixed_axis face by face.
-template <int RIEMANN, bool GATED>
-__global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const StageArgs a, const int z0, const int z1, const int lz, const int nslots) {
+template <int RIEMANN, bool GATED, int MB = 2>
+__global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const StageArgs a, const int z0, const int z1, const int lz, const int nslots) {
     using S = MarchShape;
     constexpr int NV = 5, PL = S::PL, NCOL = S::NCOL;
     extern __shared__ double smem_d[];
@@ -71,11 +111,15 @@ __global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const St
     double* Rh = Rc + 5 * NCOL;      // raw halo of the next plane
     double* Ru = Rh + 5 * NCOL;      // U of the cell
     double* R0 = Ru + 5 * NCOL;      // U0 of the cell
-    float* Rv = reinterpret_cast<float*>(R0 + 5 * NCOL);
-    float* P = Rv + 4 * NCOL;        // [rho, u, v, p, w][PL]
-    float* FX = P + 5 * PL;          // [5][NFX]
-    float* FY = FX + 5 * S::NFX;     // [5][NFY]
-    float* FZ = FY + 5 * S::NFY;     // [2][5][256]: the z faces below and above the plane, by turns
+    float4* P4 = reinterpret_cast<float4*>(R0 + 5 * NCOL);   // [PL] the plane being solved
+    float4* FX4 = P4 + PL;                                    // [NFX]
+    float4* FY4 = FX4 + S::NFX;                               // [NFY]
+    float4* FZ4 = FY4 + S::NFY;                               // [2][256]: the z faces below and above the plane, by turns
+    float* Pw = reinterpret_cast<float*>(FZ4 + 2 * NCOL);
+    float* FXw = Pw + PL;
+    float* FYw = FXw + S::NFX;
+    float* FZw = FYw + S::NFY;
+    float* Rv = FZw + 2 * NCOL;                               // [4][256] the viscous sums
     if (!*a.gate) return;
     const Mesh& m = a.m;
     const GasF gas = gas_f(a.eos);
@@ -85,10 +129,9 @@ __global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const St
     const int cta = blockIdx.x;
     const int x0 = (cta % cx) * S::W, y0 = ((cta / cx) % cy) * S::H, za = z0 + (cta / (cx * cy)) * lz;
     const int zb = za + lz < z1 ? za + lz : z1;
-    const bool col = tid < NCOL;
-    const int tx = tid & 31, ty = tid >> 5;             // (the ninth warp: ty = 8)
+    const int tx = tid & 31, ty = tid >> 5;
     const int gx = x0 + tx, gy = y0 + ty;
-    const bool cell_in = col && gx < m.nx && gy < m.ny;
+    const bool cell_in = gx < m.nx && gy < m.ny;
     const long long zs = (long long)m.nx * m.ny;
 
     // the thread's column and its halo cell: what they read, and the side whose ghost rule they follow
@@ -167,125 +210,96 @@ __global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const St
         const long long t = ((long long)(p[2] >> 3) * a.tiles[1] + (p[1] >> 3)) * a.tiles[0] + (p[0] >> 3);
         return a.sens_flags[(long long)axis * a.tiles[0] * a.tiles[1] * a.tiles[2] + t] == 0;
     };
-    const int fx = col ? tx : S::W, fy = col ? ty : (tx < S::H ? tx : 0);   // the thread's x face: its low one, or the ninth warp's
-
-    if (col) fetch_core(za + 3);
+    fetch_core(za + 3);
     if (hslot >= 0) fetch_halo(za);
     if (cell_in) fetch_cell(za);
-    // the column's planes k - 2 .. k + 3 in registers ([variable][plane]), from k = za - 1
-    float r[NV][6];
-    if (col) {
+    // the column's planes k - 2 .. k + 3 in registers, from k = za - 1
+    const auto rounded = [](const St<double, NV>& w) {
+        return March5{make_float4((float)w[0], (float)w[3], (float)w[1], (float)w[2]), (float)w[4]};
+    };
+    March5 r[6];
 #pragma unroll
-        for (int p = 0; p < 6; ++p) {
-            int sz;
-            const double* src = a.U + march_cell(a.bc, 2, za - 3 + p, m.nz, sz) * zs + coff;
-            const St<double, NV> w = prim(src, m.plane, sz >= 0 ? sz : cside);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) r[q][p] = (float)w[q];
-        }
+    for (int p = 0; p < 6; ++p) {
+        int sz;
+        const double* src = a.U + march_cell(a.bc, 2, za - 3 + p, m.nz, sz) * zs + coff;
+        r[p] = rounded(prim(src, m.plane, sz >= 0 ? sz : cside));
     }
     const float Ax = (float)m.area[0], Ay = (float)m.area[1], Az = (float)m.area[2];
     const double dt = a.ctl->dt;
     float smax = 0.0f;
-    int lin = 0;   // bit 0, 1, 2: the thread's x, y and z faces are linear
+    int lin = 0;   // bits: the thread's low x, low y and high z faces are linear; its faces on the high sides along x and y
+    const auto speed = [&](bool inside, float s) {
+        if (inside && s > smax) smax = s;
+    };
     // k = za - 1: only the z faces below the first plane
 #pragma unroll 1
     for (int k = za - 1; k < zb; ++k) {
         const bool first = k < za;
         if (!first) {
             cp_async_wait();
-            if (col) {
 #pragma unroll
-                for (int q = 0; q < NV; ++q)
-#pragma unroll
-                    for (int p = 0; p < 5; ++p) r[q][p] = r[q][p + 1];
-                const St<double, NV> w = prim(Rc + tid, NCOL, core_side(k + 3));
-#pragma unroll
-                for (int q = 0; q < NV; ++q) {
-                    r[q][5] = (float)w[q];
-                    P[q * PL + pslot] = r[q][2];
-                }
-            }
+            for (int p = 0; p < 5; ++p) r[p] = r[p + 1];
+            r[5] = rounded(prim(Rc + tid, NCOL, core_side(k + 3)));
+            P4[pslot] = r[2].a;
+            Pw[pslot] = r[2].w;
             if (hslot >= 0) {
-                const St<double, NV> w = prim(Rh + tid, NCOL, hside);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) P[q * PL + hslot] = (float)w[q];
+                const March5 h = rounded(prim(Rh + tid, NCOL, hside));
+                P4[hslot] = h.a;
+                Pw[hslot] = h.w;
             }
             if (k + 1 < zb) {
-                if (col) fetch_core(k + 4);
+                fetch_core(k + 4);
                 if (hslot >= 0) fetch_halo(k + 1);
             }
         }
         if constexpr (GATED) {
             if (k <= za || (k & 7) == 0 || (k & 7) == 7) {
-                const int xf = x0 + fx, yf = y0 + fy;
-                lin = (tile_linear(0, xf - 1, yf, k) && tile_linear(0, xf, yf, k) ? 1 : 0) |
+                lin = (tile_linear(0, gx - 1, gy, k) && tile_linear(0, gx, gy, k) ? 1 : 0) |
                       (tile_linear(1, gx, gy - 1, k) && tile_linear(1, gx, gy, k) ? 2 : 0) |
-                      (tile_linear(2, gx, gy, k) && tile_linear(2, gx, gy, k + 1) ? 4 : 0);
+                      (tile_linear(2, gx, gy, k) && tile_linear(2, gx, gy, k + 1) ? 4 : 0) |
+                      (tx < S::H && tile_linear(0, x0 + S::W - 1, y0 + tx, k) && tile_linear(0, x0 + S::W, y0 + tx, k) ? 8 : 0) |
+                      (tile_linear(1, gx, y0 + S::H - 1, k) && tile_linear(1, gx, y0 + S::H, k) ? 16 : 0);
             }
         }
         __syncthreads();
-        // ---- the faces: x (the low side of the cell), y (low), z (high)
+        March5 c[6], F;
+        if (gy < m.ny) {   // ---- the high z face
+            speed(cell_in, march_face<2, RIEMANN>(gas, sb, weps, GATED && (lin & 4), r, F));
+            FZ4[(k & 1) * NCOL + tid] = F.a;
+            FZw[(k & 1) * NCOL + tid] = F.w;
+        }
+        if (!first) {
+            // ---- the low x face, and by one warp in turn the high ones of the eight rows
 #pragma unroll 1
-        for (int it = first ? 2 : 0; it < 3; ++it) {
-            float c[NV][6];   // rho, p, the normal velocity, the other two in cyclic order
-            bool on, inside;
-            if (it == 2) {
-                on = col && gy < m.ny;
-                inside = cell_in;
+            for (int fx = tx, fy = ty;;) {
+                const bool high = fx >= S::W;
+                if (y0 + fy < m.ny) {
+                    const float4* b4 = P4 + (fy + 3) * S::PITCH + fx;
+                    const float* bw = Pw + (fy + 3) * S::PITCH + fx;
 #pragma unroll
-                for (int p = 0; p < 6; ++p) {
-                    c[0][p] = r[0][p];
-                    c[1][p] = r[3][p];
-                    c[2][p] = r[4][p];
-                    c[3][p] = r[1][p];
-                    c[4][p] = r[2][p];
+                    for (int p = 0; p < 6; ++p) c[p] = March5{b4[p], bw[p]};
+                    speed(x0 + fx <= m.nx, march_face<0, RIEMANN>(gas, sb, weps, GATED && (lin & (high ? 8 : 1)), c, F));
+                    FX4[fy * S::FXP + fx] = F.a;
+                    FXw[fy * S::FXP + fx] = F.w;
                 }
-            } else if (it == 1) {
-                on = gy <= m.ny;
-                inside = gx < m.nx && gy <= m.ny;
-                const float* b = P + ty * S::PITCH + tx + 3;
-#pragma unroll
-                for (int p = 0; p < 6; ++p) {
-                    c[0][p] = b[p * S::PITCH];
-                    c[1][p] = b[3 * PL + p * S::PITCH];
-                    c[2][p] = b[2 * PL + p * S::PITCH];
-                    c[3][p] = b[4 * PL + p * S::PITCH];
-                    c[4][p] = b[1 * PL + p * S::PITCH];
-                }
-            } else {
-                on = (col || tx < S::H) && y0 + fy < m.ny;
-                inside = x0 + fx <= m.nx && y0 + fy < m.ny;
-                const float* b = P + (fy + 3) * S::PITCH + fx;
-#pragma unroll
-                for (int p = 0; p < 6; ++p) {
-                    c[0][p] = b[p];
-                    c[1][p] = b[3 * PL + p];
-                    c[2][p] = b[1 * PL + p];
-                    c[3][p] = b[2 * PL + p];
-                    c[4][p] = b[4 * PL + p];
-                }
+                if (high || ty != (k & 7) || tx >= S::H) break;
+                fx = S::W;
+                fy = tx;
             }
-            if (!on) continue;
-            float L[NV], R[NV];
-            if (GATED && (lin >> it & 1)) {
+            // ---- the low y face, and by another warp in turn the high ones
+#pragma unroll 1
+            for (int fy = ty;; fy = S::H) {
+                if (y0 + fy <= m.ny) {
+                    const float4* b4 = P4 + fy * S::PITCH + tx + 3;
+                    const float* bw = Pw + fy * S::PITCH + tx + 3;
 #pragma unroll
-                for (int q = 0; q < NV; ++q) lin5_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], L[q], R[q]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) weno5z_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], weps, L[q], R[q]);
+                    for (int p = 0; p < 6; ++p) c[p] = March5{b4[p * S::PITCH], bw[p * S::PITCH]};
+                    speed(gx < m.nx, march_face<1, RIEMANN>(gas, sb, weps, GATED && (lin & (fy == S::H ? 16 : 2)), c, F));
+                    FY4[fy * S::W + tx] = F.a;
+                    FYw[fy * S::W + tx] = F.w;
+                }
+                if (fy == S::H || ty != ((k + 4) & 7)) break;
             }
-            float vL[3] = {L[2], L[3], L[4]}, vR[3] = {R[2], R[3], R[4]}, Fm, Fe, Fv[3];
-            const float s = riemann_f<RIEMANN>(gas, sb, L[0], L[1], vL, R[0], R[1], vR, Fm, Fe, Fv);
-            if (inside && s > smax) smax = s;
-            float* dst = it == 0 ? FX + fy * S::FXP + fx : (it == 1 ? FY + tid : FZ + (k & 1) * 5 * NCOL + tid);
-            const int st = it == 0 ? S::NFX : (it == 1 ? S::NFY : NCOL);
-            const int n = it == 0 ? 1 : (it == 1 ? 2 : 4), t1 = it == 0 ? 2 : (it == 1 ? 4 : 1), t2 = it == 0 ? 4 : (it == 1 ? 1 : 2);
-            dst[0] = Fm;
-            dst[3 * st] = Fe;
-            dst[n * st] = Fv[0];
-            dst[t1 * st] = Fv[1];
-            dst[t2 * st] = Fv[2];
         }
         __syncthreads();
         // ---- the balance, the residual widened to FP64 and the FP64 update of plane k
@@ -298,14 +312,18 @@ __global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const St
                 in.u0[q] = a.mode == kCombine ? R0[q * NCOL + tid] : 0.0;
                 in.rv[q] = a.Rvf && q > 0 ? (double)Rv[(q - 1) * NCOL + tid] : 0.0;
             }
-            const float *X = FX + ty * S::FXP + tx, *Y = FY + tid, *Zh = FZ + (k & 1) * 5 * NCOL + tid, *Zl = FZ + ((k + 1) & 1) * 5 * NCOL + tid;
+            const int ix = ty * S::FXP + tx, zh = (k & 1) * NCOL + tid, zl = ((k + 1) & 1) * NCOL + tid;
+            const float4 xl = FX4[ix], xr = FX4[ix + 1], yl = FY4[tid], yr = FY4[tid + S::W], zd = FZ4[zl], zu = FZ4[zh];
+            const auto balance = [&](float x0_, float x1, float y0_, float y1, float z0_, float z1_) {
+                float acc = -__fmul_rn(x1 - x0_, Ax);
+                acc = __fmaf_rn(-(y1 - y0_), Ay, acc);
+                return __fmaf_rn(-(z1_ - z0_), Az, acc);
+            };
+            const float sum[NV] = {balance(xl.x, xr.x, yl.x, yr.x, zd.x, zu.x), balance(xl.z, xr.z, yl.z, yr.z, zd.z, zu.z),
+                                   balance(xl.w, xr.w, yl.w, yr.w, zd.w, zu.w), balance(xl.y, xr.y, yl.y, yr.y, zd.y, zu.y),
+                                   balance(FXw[ix], FXw[ix + 1], FYw[tid], FYw[tid + S::W], FZw[zl], FZw[zh])};
 #pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                float acc = -__fmul_rn(X[q * S::NFX + 1] - X[q * S::NFX], Ax);
-                acc = __fmaf_rn(-(Y[q * S::NFY + S::W] - Y[q * S::NFY]), Ay, acc);
-                acc = __fmaf_rn(-(Zh[q * NCOL] - Zl[q * NCOL]), Az, acc);
-                a.out[q * m.plane + cell] = cell_out(a, in, q, acc, dt);
-            }
+            for (int q = 0; q < NV; ++q) a.out[q * m.plane + cell] = cell_out(a, in, q, sum[q], dt);
             if (k + 1 < zb) fetch_cell(k + 1);
         }
     }
@@ -320,27 +338,54 @@ __global__ void __launch_bounds__(MarchShape::NT, 2) mixed_march_kernel(const St
 
 // The 2-D form: a CTA owns W columns of cells and marches along y. A thread keeps the six rows of its column around its y
 // face in registers; the row being solved lies in shared memory with the halo along x; per row a thread solves its low x
-// face and its high y face in one loop with one copy of the face code. The last column's cell belongs to the next CTA (its
+// face and its high y face. A cell is one float4 (rho, p, u, v), its pairs operands of packed operations. The last column's cell belongs to the next CTA (its
 // low face is this CTA's last high face), so every thread has the same work. Tiles of the gate: 16 x 15 cells. 2048^2 quadrants
-// with the sensor: 342 us per launch in 16 x 15 tiles, 206 here.
+// with the sensor: 342 us per launch in 16 x 15 tiles, 206 marching with scalar loads and one loop over both faces, 182 here.
 template <int W_> struct March2Shape {
     static constexpr int W = W_, NT = W_, NHALO = 5, RP = W_ + 8, RAW = W_ + 8;
     // doubles: red [32], raw row [4][RAW] (the column, three rows ahead, then the halo of the next row), u [4][W], u0 [4][W],
-    // viscous residual [4][W]; floats: P [4][RP], FX [4][W]
-    static constexpr size_t SMEM_BYTES = 8 * (32 + 4 * RAW + 12 * W) + 4 * (4 * RP + 4 * W);
+    // viscous residual [4][W]; float4: P [RP], FX [W] (the fluxes of rho, rho E, rho u, rho v)
+    static constexpr size_t SMEM_BYTES = 8 * (32 + 4 * RAW + 12 * W) + 16 * (RP + W);
 };
+// the face along axis A from its six cells (rho, p, u, v)
+template <int A, int RIEMANN>
+__device__ __forceinline__ float march2_face(const GasF& gas, float sb, float weps, bool linear, const float4 (&c)[6], float4& F) {
+    const auto lo = [&](int p) { return f2(c[p].x, c[p].y); };
+    const auto hi = [&](int p) { return f2(c[p].z, c[p].w); };
+    F2 l0, l1, r0, r1;
+    if (linear) {
+        l0 = lin5_f2(lo(0), lo(1), lo(2), lo(3), lo(4));
+        r0 = lin5_f2(lo(5), lo(4), lo(3), lo(2), lo(1));
+        l1 = lin5_f2(hi(0), hi(1), hi(2), hi(3), hi(4));
+        r1 = lin5_f2(hi(5), hi(4), hi(3), hi(2), hi(1));
+    } else {
+        l0 = weno5z_f2(lo(0), lo(1), lo(2), lo(3), lo(4), weps);
+        r0 = weno5z_f2(lo(5), lo(4), lo(3), lo(2), lo(1), weps);
+        l1 = weno5z_f2(hi(0), hi(1), hi(2), hi(3), hi(4), weps);
+        r1 = weno5z_f2(hi(5), hi(4), hi(3), hi(2), hi(1), weps);
+    }
+    float rL, pL, rR, pR, vL[2], vR[2], Fv[2];
+    f2_get(l0, rL, pL);
+    f2_get(r0, rR, pR);
+    f2_get(l1, vL[A], vL[1 - A]);
+    f2_get(r1, vR[A], vR[1 - A]);
+    const float s = riemann_f<RIEMANN>(gas, sb, rL, pL, vL, rR, pR, vR, F.x, F.y, Fv);
+    F.z = Fv[A];
+    F.w = Fv[1 - A];
+    return s;
+}
 template <int RIEMANN, bool GATED, int W, int MB>
 __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, const int z0, const int z1, const int lz, const int nslots) {
     using S = March2Shape<W>;
-    constexpr int NV = 4, RP = S::RP, RAW = S::RAW;
+    constexpr int NV = 4, RAW = S::RAW;
     extern __shared__ double smem_d[];
     double* red = smem_d;
     double* Rc = smem_d + 32;
     double* Ru = Rc + 4 * RAW;
     double* R0 = Ru + 4 * W;
     double* Rv = R0 + 4 * W;
-    float* P = reinterpret_cast<float*>(Rv + 4 * W);
-    float* FX = P + 4 * RP;
+    float4* P4 = reinterpret_cast<float4*>(Rv + 4 * W);
+    float4* FX4 = P4 + S::RP;
     if (!*a.gate) return;
     const Mesh& m = a.m;
     const GasF gas = gas_f(a.eos);
@@ -402,18 +447,18 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
     fetch_core(za + 3);
     if (halo) fetch_halo(za);
     if (cell_in) fetch_cell(za);
-    float r[NV][6];
+    const auto rounded = [](const St<double, NV>& w) { return make_float4((float)w[0], (float)w[3], (float)w[1], (float)w[2]); };
+    float4 r[6];
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
         int sy;
         const double* src = a.U + (long long)march_cell(a.bc, 1, za - 3 + p, m.ny, sy) * m.nx + coff;
-        const St<double, NV> w = prim(src, m.plane, sy >= 0 ? sy : cside);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) r[q][p] = (float)w[q];
+        r[p] = rounded(prim(src, m.plane, sy >= 0 ? sy : cside));
     }
     const float Ax = (float)m.area[0], Ay = (float)m.area[1];
     const double dt = a.ctl->dt;
-    float smax = 0.0f, Fl[NV] = {0.0f, 0.0f, 0.0f, 0.0f}, Fh[NV] = {0.0f, 0.0f, 0.0f, 0.0f};   // the y faces below and above the row
+    float smax = 0.0f;
+    float4 Fl = make_float4(0.0f, 0.0f, 0.0f, 0.0f), Fh;   // the y faces below and above the row
     int lin = 0, tile_end = za - 1;   // bit 0, 1: the thread's x and y faces are linear; the row after which to look again
 #pragma unroll 1
     for (int k = za - 1; k < zb; ++k) {
@@ -421,22 +466,12 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
         if (!first) {
             cp_async_wait();
 #pragma unroll
-            for (int q = 0; q < NV; ++q)
-#pragma unroll
-                for (int p = 0; p < 5; ++p) r[q][p] = r[q][p + 1];
+            for (int p = 0; p < 5; ++p) r[p] = r[p + 1];
             int sy;
             march_cell(a.bc, 1, k + 3, m.ny, sy);
-            const St<double, NV> w = prim(Rc + tid, RAW, sy >= 0 ? sy : cside);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                r[q][5] = (float)w[q];
-                P[q * RP + tid + 3] = r[q][2];
-            }
-            if (halo) {
-                const St<double, NV> h = prim(Rc + W + tid, RAW, hside);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) P[q * RP + hx + 3] = (float)h[q];
-            }
+            r[5] = rounded(prim(Rc + tid, RAW, sy >= 0 ? sy : cside));
+            P4[tid + 3] = r[2];
+            if (halo) P4[hx + 3] = rounded(prim(Rc + W + tid, RAW, hside));
             if (k + 1 < zb) {
                 fetch_core(k + 4);
                 if (halo) fetch_halo(k + 1);
@@ -450,49 +485,15 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
             }
         }
         __syncthreads();
-#pragma unroll 1
-        for (int it = first ? 1 : 0; it < 2; ++it) {
-            float c[NV][6];   // rho, p, the normal velocity, the other one
-            if (it == 1) {
+        float s = march2_face<1, RIEMANN>(gas, sb, weps, GATED && (lin & 2), r, Fh);
+        if (cell_in && s > smax) smax = s;
+        if (!first) {
+            float4 c[6], F;
 #pragma unroll
-                for (int p = 0; p < 6; ++p) {
-                    c[0][p] = r[0][p];
-                    c[1][p] = r[3][p];
-                    c[2][p] = r[2][p];
-                    c[3][p] = r[1][p];
-                }
-            } else {
-                const float* b = P + tid;
-#pragma unroll
-                for (int p = 0; p < 6; ++p) {
-                    c[0][p] = b[p];
-                    c[1][p] = b[3 * RP + p];
-                    c[2][p] = b[RP + p];
-                    c[3][p] = b[2 * RP + p];
-                }
-            }
-            float L[NV], R[NV];
-            if (GATED && (lin >> it & 1)) {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) lin5_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], L[q], R[q]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) weno5z_pair(c[q][0], c[q][1], c[q][2], c[q][3], c[q][4], c[q][5], weps, L[q], R[q]);
-            }
-            float vL[2] = {L[2], L[3]}, vR[2] = {R[2], R[3]}, Fm, Fe, Fv[2];
-            const float s = riemann_f<RIEMANN>(gas, sb, L[0], L[1], vL, R[0], R[1], vR, Fm, Fe, Fv);
-            if ((it == 1 ? cell_in : face_in) && s > smax) smax = s;
-            if (it == 0) {
-                FX[tid] = Fm;
-                FX[W + tid] = Fv[0];
-                FX[2 * W + tid] = Fv[1];
-                FX[3 * W + tid] = Fe;
-            } else {
-                Fh[0] = Fm;
-                Fh[1] = Fv[1];
-                Fh[2] = Fv[0];
-                Fh[3] = Fe;
-            }
+            for (int p = 0; p < 6; ++p) c[p] = P4[tid + p];
+            s = march2_face<0, RIEMANN>(gas, sb, weps, GATED && (lin & 1), c, F);
+            if (face_in && s > smax) smax = s;
+            FX4[tid] = F;
         }
         __syncthreads();
         if (!first && cell_in) {
@@ -504,16 +505,15 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
                 in.u0[q] = a.mode == kCombine ? R0[q * W + tid] : 0.0;
                 in.rv[q] = a.Rv ? Rv[q * W + tid] : 0.0;
             }
+            const float4 xl = FX4[tid], xr = FX4[tid + 1];
+            const auto balance = [&](float x0_, float x1, float y0_, float y1) { return __fmaf_rn(-(y1 - y0_), Ay, -__fmul_rn(x1 - x0_, Ax)); };
+            const float sum[NV] = {balance(xl.x, xr.x, Fl.x, Fh.x), balance(xl.z, xr.z, Fl.z, Fh.z), balance(xl.w, xr.w, Fl.w, Fh.w),
+                                   balance(xl.y, xr.y, Fl.y, Fh.y)};
 #pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                float acc = -__fmul_rn(FX[q * W + tid + 1] - FX[q * W + tid], Ax);
-                acc = __fmaf_rn(-(Fh[q] - Fl[q]), Ay, acc);
-                a.out[q * m.plane + cell] = cell_out(a, in, q, acc, dt);
-            }
+            for (int q = 0; q < NV; ++q) a.out[q * m.plane + cell] = cell_out(a, in, q, sum[q], dt);
             if (k + 1 < zb) fetch_cell(k + 1);
         }
-#pragma unroll
-        for (int q = 0; q < NV; ++q) Fl[q] = Fh[q];
+        Fl = Fh;
     }
     const double bm = block_max<W>((double)smax, red);
     if (tid == 0) {
@@ -590,11 +590,11 @@ template <int RIEMANN, bool GATED> struct March2K {
 // the neighbours along x and y through shared memory and along z through its own registers; then the low x, y and z faces
 // of the cell; the ninth warp takes the cells and faces on the high sides. Fluxes and gradients as in mixed_viscous_kernel,
 // which meshes with walls, inlets or outlets and immersed bodies keep. Bound by shared-memory
-// bandwidth and issue (ncu at 192^3: L1 77 %, issue 60 %, 20 warp instructions per cell). 256^3: 0.78 -> 0.48 ms per launch; the
-// mixed + sensor step 7.17 -> 6.28 ms.
+// bandwidth and issue (ncu at 192^3 before a thread kept its own column in registers: L1 77 %, issue 60 %, 20 warp instructions per
+// cell; 221 -> 209 us with it). 256^3: 0.78 -> 0.48 ms per launch; the mixed + sensor step 7.17 -> 6.28 ms.
 struct ViscMarchShape {
     static constexpr int W = 32, H = 8, NT = 288, BX = W + 2, BY = H + 2, NB = BX * BY, PITCH = 36, PL = BY * PITCH;
-    static constexpr int NGX = H * BX, NGY = BY * W, FXP = W + 1, NFX = H * FXP, NFY = (H + 1) * W;
+    static constexpr int NCOL = W * H, NGX = H * BX, NGY = BY * W, FXP = W + 1, NFX = H * FXP, NFY = (H + 1) * W;
     // doubles: red [32], raw [5][NB]; float4: V [3][PL], GX, GY, FX, FY; floats: R [3][PL]
     static constexpr size_t SMEM_BYTES = 8 * (32 + 5 * NB) + 16 * (3 * PL + NGX + NGY + NFX + NFY) + 4 * 3 * PL;
 };
@@ -692,9 +692,10 @@ __global__ void __launch_bounds__(ViscMarchShape::NT, 3) mixed_viscous_march_ker
     }
     fetch(za + 1);
     const int own = (ty + 1) * S::PITCH + tx + 1;                                  // the column in a plane
-    const int fx = col ? tx : S::W, fy = col ? ty : (tx < S::H ? tx : 0);          // the thread's x face
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float4 gz_prev = zero, fz_prev = zero, sum_prev = zero;
+    float4 cm = zero, c = zero, zp = zero;   // the column at k - 1, k, k + 1
+    float rm = 0.0f, rc = 0.0f, rzp = 0.0f;
     float smax = 0.0f;
     int s0 = 0;   // the slot of plane k
 #pragma unroll 1
@@ -717,21 +718,36 @@ __global__ void __launch_bounds__(ViscMarchShape::NT, 3) mixed_viscous_march_ker
         const float4 *Vk = V + s0 * PL, *Vp = V + sp * PL, *Vm = V + sm * PL;
         const float *Rk = R + s0 * PL, *Rp = R + sp * PL, *Rm = R + sm * PL;
         // one gradient entry from the cells after and before along an axis
-        auto entry = [](float rp, float up, float rm, float um, float uc, float s) { return (rp * (up - uc) - rm * (um - uc)) * s; };
-        float4 gz = zero, fz = zero;
+        auto entry = [](float rp, float up, float rmm, float um, float uc, float s) { return (rp * (up - uc) - rmm * (um - uc)) * s; };
+        float4 gz = zero, fz = zero, gx = zero, gy = zero, xm = zero, ym = zero;
         if (col) {
-            const float4 c = Vk[own], xp = Vk[own + 1], xm = Vk[own - 1], yp = Vk[own + S::PITCH], ym = Vk[own - S::PITCH];
+            if (k < za) {
+                c = Vk[own];
+                rc = Rk[own];
+            } else {
+                cm = c;
+                rm = rc;
+                c = zp;
+                rc = rzp;
+            }
+            if (k < zb) {
+                zp = Vp[own];
+                rzp = Rp[own];
+            }
+            const float4 xp = Vk[own + 1], yp = Vk[own + S::PITCH];
+            xm = Vk[own - 1];
+            ym = Vk[own - S::PITCH];
             const float rxp = Rk[own + 1], rxm = Rk[own - 1], ryp = Rk[own + S::PITCH], rym = Rk[own - S::PITCH];
-            const float rho = vmax(Rk[own], Num<float>::eos_eps), inv = 1.0f / rho;
+            const float rho = vmax(rc, Num<float>::eos_eps), inv = 1.0f / rho;
             const float sx = ix2 * inv, sy = iy2 * inv, sz = iz2 * inv;
             const float ux = entry(rxp, xp.x, rxm, xm.x, c.x, sx), vy = entry(ryp, yp.y, rym, ym.y, c.y, sy);
             gz = make_float4(ux, vy, entry(rxp, xp.z, rxm, xm.z, c.z, sx), entry(ryp, yp.z, rym, ym.z, c.z, sy));
             if (inner) {
-                const float4 zp = Vp[own], zm = Vm[own];
-                const float rzp = Rp[own], rzm = Rm[own];
-                const float wz = entry(rzp, zp.z, rzm, zm.z, c.z, sz);
-                GX[ty * S::BX + tx + 1] = make_float4(entry(ryp, yp.x, rym, ym.x, c.x, sy), vy, wz, entry(rzp, zp.x, rzm, zm.x, c.x, sz));
-                GY[(ty + 1) * S::W + tx] = make_float4(ux, entry(rxp, xp.y, rxm, xm.y, c.y, sx), wz, entry(rzp, zp.y, rzm, zm.y, c.y, sz));
+                const float wz = entry(rzp, zp.z, rm, cm.z, c.z, sz);
+                gx = make_float4(entry(ryp, yp.x, rym, ym.x, c.x, sy), vy, wz, entry(rzp, zp.x, rm, cm.x, c.x, sz));
+                gy = make_float4(ux, entry(rxp, xp.y, rxm, xm.y, c.y, sx), wz, entry(rzp, zp.y, rm, cm.y, c.y, sz));
+                GX[ty * S::BX + tx + 1] = gx;
+                GY[(ty + 1) * S::W + tx] = gy;
                 if (cell_in) {   // the speed bound of the cell
                     const float nu_eff = vmax((4.0f / 3.0f) * (mu / rho), (kc * gm1) / rho) + 1e-12f;
                     const float vm = vmax(vmax(fabsf(c.x), fabsf(c.y)), fabsf(c.z));
@@ -740,27 +756,24 @@ __global__ void __launch_bounds__(ViscMarchShape::NT, 3) mixed_viscous_march_ker
                     if (s > smax) smax = s;
                 }
             }
-            if (k >= za) {
-                const float4 vb = Vm[own];
-                fz = visc_face<2>(vb, c, gz_prev, gz, ihz, mu, kc, Az);
-            }
+            if (k >= za) fz = visc_face<2>(cm, c, gz_prev, gz, ihz, mu, kc, Az);
         } else if (inner) {   // the ninth warp: the cells beside the columns
 #pragma unroll
             for (int side = 0; side < 2; ++side) {   // below and above along y: [du/dx, dv/dx, dw/dz, dv/dz]
                 const int by = side ? S::BY - 1 : 0, p = by * S::PITCH + tx + 1;
-                const float4 c = Vk[p], xp = Vk[p + 1], xm = Vk[p - 1], zp = Vp[p], zm = Vm[p];
-                const float rxp = Rk[p + 1], rxm = Rk[p - 1], rzp = Rp[p], rzm = Rm[p];
+                const float4 q = Vk[p], xp = Vk[p + 1], xq = Vk[p - 1], zq = Vp[p], zm = Vm[p];
+                const float rxp = Rk[p + 1], rxm = Rk[p - 1], rzq = Rp[p], rzm = Rm[p];
                 const float inv = 1.0f / vmax(Rk[p], Num<float>::eos_eps), sx = ix2 * inv, sz = iz2 * inv;
-                GY[by * S::W + tx] = make_float4(entry(rxp, xp.x, rxm, xm.x, c.x, sx), entry(rxp, xp.y, rxm, xm.y, c.y, sx),
-                                                 entry(rzp, zp.z, rzm, zm.z, c.z, sz), entry(rzp, zp.y, rzm, zm.y, c.y, sz));
+                GY[by * S::W + tx] = make_float4(entry(rxp, xp.x, rxm, xq.x, q.x, sx), entry(rxp, xp.y, rxm, xq.y, q.y, sx),
+                                                 entry(rzq, zq.z, rzm, zm.z, q.z, sz), entry(rzq, zq.y, rzm, zm.y, q.y, sz));
             }
             if (tx < 2 * S::H) {   // before and after along x: [du/dy, dv/dy, dw/dz, du/dz]
                 const int row = tx & (S::H - 1), bx = tx < S::H ? 0 : S::BX - 1, p = (row + 1) * S::PITCH + bx;
-                const float4 c = Vk[p], yp = Vk[p + S::PITCH], ym = Vk[p - S::PITCH], zp = Vp[p], zm = Vm[p];
-                const float ryp = Rk[p + S::PITCH], rym = Rk[p - S::PITCH], rzp = Rp[p], rzm = Rm[p];
+                const float4 q = Vk[p], yp = Vk[p + S::PITCH], yq = Vk[p - S::PITCH], zq = Vp[p], zm = Vm[p];
+                const float ryp = Rk[p + S::PITCH], rym = Rk[p - S::PITCH], rzq = Rp[p], rzm = Rm[p];
                 const float inv = 1.0f / vmax(Rk[p], Num<float>::eos_eps), sy = iy2 * inv, sz = iz2 * inv;
-                GX[row * S::BX + bx] = make_float4(entry(ryp, yp.x, rym, ym.x, c.x, sy), entry(ryp, yp.y, rym, ym.y, c.y, sy),
-                                                   entry(rzp, zp.z, rzm, zm.z, c.z, sz), entry(rzp, zp.x, rzm, zm.x, c.x, sz));
+                GX[row * S::BX + bx] = make_float4(entry(ryp, yp.x, rym, yq.x, q.x, sy), entry(ryp, yp.y, rym, yq.y, q.y, sy),
+                                                   entry(rzq, zq.z, rzm, zm.z, q.z, sz), entry(rzq, zq.x, rzm, zm.x, q.x, sz));
             }
         }
         if (cell_in && k > za) {   // the plane below is complete: its x and y sums and its two z faces
@@ -774,17 +787,25 @@ __global__ void __launch_bounds__(ViscMarchShape::NT, 3) mixed_viscous_march_ker
         fz_prev = fz;
         if (k == zb) break;
         __syncthreads();
+        float4 xl = zero, yl = zero;
         if (inner) {
-            if (col || tx < S::H) {
-                const int p = (fy + 1) * S::PITCH + fx, g = fy * S::BX + fx;
-                FX[fy * S::FXP + fx] = visc_face<0>(Vk[p], Vk[p + 1], GX[g], GX[g + 1], ihx, mu, kc, Ax);
+            if (col) {   // the low faces of the cell: its own side's state and gradients are in registers
+                xl = visc_face<0>(xm, c, GX[ty * S::BX + tx], gx, ihx, mu, kc, Ax);
+                yl = visc_face<1>(ym, c, GY[tid], gy, ihy, mu, kc, Ay);
+                FX[ty * S::FXP + tx] = xl;
+                FY[tid] = yl;
+            } else {     // the faces on the high sides of the columns
+                const int p = S::H * S::PITCH + tx + 1;
+                FY[S::NCOL + tx] = visc_face<1>(Vk[p], Vk[p + S::PITCH], GY[S::NCOL + tx], GY[S::NCOL + S::W + tx], ihy, mu, kc, Ay);
+                if (tx < S::H) {
+                    const int px = (tx + 1) * S::PITCH + S::W, g = tx * S::BX + S::W;
+                    FX[tx * S::FXP + S::W] = visc_face<0>(Vk[px], Vk[px + 1], GX[g], GX[g + 1], ihx, mu, kc, Ax);
+                }
             }
-            const int p = ty * S::PITCH + tx + 1;
-            FY[tid] = visc_face<1>(Vk[p], Vk[p + S::PITCH], GY[tid], GY[tid + S::W], ihy, mu, kc, Ay);
         }
         __syncthreads();
         if (inner && col) {
-            const float4 xl = FX[ty * S::FXP + tx], xr = FX[ty * S::FXP + tx + 1], yl = FY[tid], yr = FY[tid + S::W];
+            const float4 xr = FX[ty * S::FXP + tx + 1], yr = FY[tid + S::W];
             sum_prev = make_float4((xr.x - xl.x) + (yr.x - yl.x), (xr.y - xl.y) + (yr.y - yl.y), (xr.z - xl.z) + (yr.z - yl.z),
                                    (xr.w - xl.w) + (yr.w - yl.w));
         }

@@ -163,18 +163,6 @@ __device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend
     return s;
 }
 
-// The two linear face values of six cells: the fifth-order upwind value right of c2 from c0 .. c4, 0.1 p0 + 0.6 p1 + 0.3 p2
-// of the three candidate stencils, and its mirror image left of c3 from c5 .. c1, in the two lanes of packed operations
-// (half the issue slots of two scalar evaluations; explicitly rounded, as weno5z_pair: the same bits in every kernel).
-__device__ __forceinline__ void lin5_pair(float c0, float c1, float c2, float c3, float c4, float c5, float& wl, float& wr) {
-    F2 s = f2_mul(f2(2.0f, 2.0f), f2(c0, c5));
-    s = f2_fma(f2(-13.0f, -13.0f), f2(c1, c4), s);
-    s = f2_fma(f2(47.0f, 47.0f), f2(c2, c3), s);
-    s = f2_fma(f2(27.0f, 27.0f), f2(c3, c2), s);
-    s = f2_fma(f2(-3.0f, -3.0f), f2(c4, c1), s);
-    f2_get(f2_mul(s, f2(1.0f / 60.0f, 1.0f / 60.0f)), wl, wr);
-}
-
 // The primitive state of a cell (cons_to_prim in FP64) for the mixed form, each operation rounded explicitly (the same bits
 // in every kernel that rounds it to FP32); inv receives 1 / rho of the floored density: the hardware's approximate
 // reciprocal and two Newton steps, within a unit in the last place of FP64.

@@ -233,13 +233,12 @@ __device__ __forceinline__ F2 f2_rcp(F2 v) {
     return f2(rcp_f(a), rcp_f(b));
 }
 
-// The single-precision WENO5-Z of the mixed form, both values of a face at once: wl right of c2 from c0 .. c4 in the low
-// lane, wr left of c3 from c5 .. c1 in the high lane. The same weights, with every product and sum rounded by an explicit
-// packed operation (FMAs placed by hand) and the candidates' common 1/6 folded into the last division, so that no compiler
-// pass contracts it one way in one kernel and another way in the next: every kernel that solves a face gets the same bits.
-__device__ __forceinline__ void weno5z_pair(float c0, float c1, float c2, float c3, float c4, float c5, float eps_rel, float& wl, float& wr) {
+// The single-precision WENO5-Z of the mixed form on packed operands (two variables, or the two values of a face): the value
+// right of c from (a, b, c, d, e). Every product and sum is rounded by an explicit packed operation (FMAs placed by hand)
+// and the candidates' common 1/6 folded into the last division, so that no compiler pass contracts it one way in one kernel
+// and another way in the next: every kernel that solves a face gets the same bits.
+__device__ __forceinline__ F2 weno5z_f2(F2 a, F2 b, F2 c, F2 d, F2 e, float eps_rel) {
     const auto k = [](float v) { return f2(v, v); };
-    const F2 a = f2(c0, c5), b = f2(c1, c4), c = f2(c2, c3), d = f2(c3, c2), e = f2(c4, c1);
     F2 ss = f2_mul(a, a);
     ss = f2_fma(b, b, ss);
     ss = f2_fma(c, c, ss);
@@ -264,7 +263,24 @@ __device__ __forceinline__ void weno5z_pair(float c0, float c1, float c2, float 
     const F2 a2 = f2_mul(k(0.3f), f2_fma(tau, f2_rcp(f2_add(b2, eps)), k(1.0f)));
     const F2 num = f2_fma(a2, p2, f2_fma(a1, p1, f2_mul(a0, p0)));
     const F2 den = f2_mul(k(6.0f), f2_add(f2_add(a0, a1), a2));
-    f2_get(f2_mul(num, f2_rcp(den)), wl, wr);
+    return f2_mul(num, f2_rcp(den));
+}
+// the linear fifth-order upwind value (0.1, 0.6, 0.3 of the candidates), likewise
+__device__ __forceinline__ F2 lin5_f2(F2 a, F2 b, F2 c, F2 d, F2 e) {
+    const auto k = [](float v) { return f2(v, v); };
+    F2 s = f2_mul(k(2.0f), a);
+    s = f2_fma(k(-13.0f), b, s);
+    s = f2_fma(k(47.0f), c, s);
+    s = f2_fma(k(27.0f), d, s);
+    s = f2_fma(k(-3.0f), e, s);
+    return f2_mul(s, k(1.0f / 60.0f));
+}
+// both values of a face of six cells: wl right of c2 from c0 .. c4, and its mirror image wr left of c3 from c5 .. c1
+__device__ __forceinline__ void weno5z_pair(float c0, float c1, float c2, float c3, float c4, float c5, float eps_rel, float& wl, float& wr) {
+    f2_get(weno5z_f2(f2(c0, c5), f2(c1, c4), f2(c2, c3), f2(c3, c2), f2(c4, c1), eps_rel), wl, wr);
+}
+__device__ __forceinline__ void lin5_pair(float c0, float c1, float c2, float c3, float c4, float c5, float& wl, float& wr) {
+    f2_get(lin5_f2(f2(c0, c5), f2(c1, c4), f2(c2, c3), f2(c3, c2), f2(c4, c1)), wl, wr);
 }
 
 // ------------------------------------------------------------------ HLLC (Toro) with Einfeldt bounds (Schemes.cpp:116-200)
