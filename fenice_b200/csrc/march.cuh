@@ -18,7 +18,8 @@
 //
 // What bounds it: instruction issue at 16 warps per SM (DRAM 18 %). Mixed + sensor at 256^3: 7.29 ms per step in 8x8x8 tiles with
 // boxes by TMA, 7.17 marching with scalar loads, a loop over the axes and a ninth warp (58 warp instructions per cell, issue
-// 59 % at 192^3, where the tiles took 80), 6.28 with the viscous sweep below, 5.58 in this form. Mixed at 64^3: 225, 209, 198, 183 us.
+// 59 % at 192^3, where the tiles took 80), 6.28 with the viscous sweep below, 5.58 with cells as float4, 5.31 with the
+// update's operands waited for where they are used. Mixed at 64^3: 225, 209, 198, 183, 182 us.
 #pragma once
 
 #include "mixed.cuh"
@@ -81,6 +82,9 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// the copies since the last commit as one group; all groups but the latest one arrived
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // The cell a stencil position g along an axis reads, and the side whose ghost-slab rule applies to it (-1: none); the rules
 // of stencil_cons for one axis.
@@ -212,7 +216,9 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
     };
     fetch_core(za + 3);
     if (hslot >= 0) fetch_halo(za);
+    cp_async_commit();
     if (cell_in) fetch_cell(za);
+    cp_async_commit();
     // the column's planes k - 2 .. k + 3 in registers, from k = za - 1
     const auto rounded = [](const St<double, NV>& w) {
         return March5{make_float4((float)w[0], (float)w[3], (float)w[1], (float)w[2]), (float)w[4]};
@@ -236,7 +242,7 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
     for (int k = za - 1; k < zb; ++k) {
         const bool first = k < za;
         if (!first) {
-            cp_async_wait();
+            cp_async_wait_but_one();   // (the update's operands, issued last, are waited for where they are used)
 #pragma unroll
             for (int p = 0; p < 5; ++p) r[p] = r[p + 1];
             r[5] = rounded(prim(Rc + tid, NCOL, core_side(k + 3)));
@@ -251,6 +257,7 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
                 fetch_core(k + 4);
                 if (hslot >= 0) fetch_halo(k + 1);
             }
+            cp_async_commit();
         }
         if constexpr (GATED) {
             if (k <= za || (k & 7) == 0 || (k & 7) == 7) {
@@ -303,6 +310,7 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
         }
         __syncthreads();
         // ---- the balance, the residual widened to FP64 and the FP64 update of plane k
+        if (!first) cp_async_wait_but_one();
         if (!first && cell_in) {
             const long long cell = k * zs + coff;
             CellIn<NV> in;
@@ -326,6 +334,7 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
             for (int q = 0; q < NV; ++q) a.out[q * m.plane + cell] = cell_out(a, in, q, sum[q], dt);
             if (k + 1 < zb) fetch_cell(k + 1);
         }
+        if (!first) cp_async_commit();
     }
     const double bm = block_max<S::NT>((double)smax, red);
     if (tid == 0) {
@@ -340,7 +349,8 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
 // face in registers; the row being solved lies in shared memory with the halo along x; per row a thread solves its low x
 // face and its high y face. A cell is one float4 (rho, p, u, v), its pairs operands of packed operations. The last column's cell belongs to the next CTA (its
 // low face is this CTA's last high face), so every thread has the same work. Tiles of the gate: 16 x 15 cells. 2048^2 quadrants
-// with the sensor: 342 us per launch in 16 x 15 tiles, 206 marching with scalar loads and one loop over both faces, 182 here.
+// with the sensor: 342 us per launch in 16 x 15 tiles, 206 marching with scalar loads and one loop over both faces, 182 with cells
+// as float4, 167 with the update's operands waited for where they are used.
 template <int W_> struct March2Shape {
     static constexpr int W = W_, NT = W_, NHALO = 5, RP = W_ + 8, RAW = W_ + 8;
     // doubles: red [32], raw row [4][RAW] (the column, three rows ahead, then the halo of the next row), u [4][W], u0 [4][W],
@@ -446,7 +456,9 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
     };
     fetch_core(za + 3);
     if (halo) fetch_halo(za);
+    cp_async_commit();
     if (cell_in) fetch_cell(za);
+    cp_async_commit();
     const auto rounded = [](const St<double, NV>& w) { return make_float4((float)w[0], (float)w[3], (float)w[1], (float)w[2]); };
     float4 r[6];
 #pragma unroll
@@ -464,7 +476,7 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
     for (int k = za - 1; k < zb; ++k) {
         const bool first = k < za;
         if (!first) {
-            cp_async_wait();
+            cp_async_wait_but_one();   // (the update's operands, issued last, are waited for where they are used)
 #pragma unroll
             for (int p = 0; p < 5; ++p) r[p] = r[p + 1];
             int sy;
@@ -476,6 +488,7 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
                 fetch_core(k + 4);
                 if (halo) fetch_halo(k + 1);
             }
+            cp_async_commit();
         }
         if constexpr (GATED) {
             if (k >= tile_end) {   // (the y face above a tile's last row looks at the next tile)
@@ -496,6 +509,7 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
             FX4[tid] = F;
         }
         __syncthreads();
+        if (!first) cp_async_wait_but_one();
         if (!first && cell_in) {
             const long long cell = (long long)k * m.nx + coff;
             CellIn<NV> in;
@@ -513,6 +527,7 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
             for (int q = 0; q < NV; ++q) a.out[q * m.plane + cell] = cell_out(a, in, q, sum[q], dt);
             if (k + 1 < zb) fetch_cell(k + 1);
         }
+        if (!first) cp_async_commit();
         Fl = Fh;
     }
     const double bm = block_max<W>((double)smax, red);
