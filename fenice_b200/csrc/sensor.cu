@@ -483,9 +483,9 @@ __global__ void __launch_bounds__(256) k_sensor_infer(const SensorW* __restrict_
 __device__ __forceinline__ bool refresh_due(const Ctl* ctl, int every) { return !ctl || (ctl->active && ctl->steps % every == 0); }
 
 // The network's flags of every (cell, axis), tiled: a CTA takes a BX x BY (x BZ) block of cells, recovers the
-// primitive state of the block and a 2-cell halo once per cell into shared memory (float), then its warps take 16
-// (cell, axis) rows at a time: features of the row's 5-cell stencil into the warp's bf16 tile (one lane per row and
-// quantity), logits on the tensor cores.
+// primitive state of the block and a 2-cell halo once per cell into shared memory (float), then its warpgroups take 128
+// (cell, axis) rows at a time: features of the row's 5-cell stencil into the group's bf16 tile (a thread per row), logits on
+// the tensor cores.
 template <int DIM, int NV, int BX, int BY, int BZ>
 __global__ void __launch_bounds__(256) k_sensor_flags_t(Mesh m, Bc bc, Eos<double> eos, const double* __restrict__ U, const SensorW* __restrict__ wg,
                                                         float theta, unsigned char* __restrict__ flags, const Ctl* ctl, int every, int nb0, int nb1,
@@ -501,48 +501,57 @@ __global__ void __launch_bounds__(256) k_sensor_flags_t(Mesh m, Bc bc, Eos<doubl
     sens_tc_setup(st, wg);
     const int b = blockIdx.x;
     const int o0 = (b % nb0) * BX, o1 = ((b / nb0) % nb1) * BY, o2 = DIM == 3 ? (b / (nb0 * nb1)) * BZ : 0;
+    // a box inside the mesh needs no boundary rule (uniform over the CTA)
+    const bool inner = o0 >= 2 && o0 + BX + 2 <= m.nx && o1 >= 2 && o1 + BY + 2 <= m.ny && (DIM == 2 || (o2 >= 2 && o2 + BZ + 2 <= m.nz));
     for (int e = threadIdx.x; e < BOX; e += blockDim.x) {
         const int i = o0 + e % EX - 2, j = o1 + (e / EX) % EY - 2, k = DIM == 3 ? o2 + e / (EX * EY) - 2 : 0;
-        const St<double, NV> wv = c2p(eos, stencil_cons<DIM, NV>(m, bc, eos, U, i, j, k));
+        const St<double, NV> u = inner ? read_state<NV>(bc, U, m.plane, ((long long)k * m.ny + j) * m.nx + i) : stencil_cons<DIM, NV>(m, bc, eos, U, i, j, k);
+        const St<double, NV> wv = c2p(eos, u);
 #pragma unroll
         for (int q = 0; q < NV; ++q) P[q * PS + e] = (float)wv[q];
     }
     __syncthreads();
-    const int g = threadIdx.x >> 7, q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+    const int g = threadIdx.x >> 7;
     const float gam = (float)eos.gamma, pinf = eos.type == kIdeal ? 0.0f : (float)eos.p_inf;
     unsigned phase = 0;
-    // warpgroup g takes the 128-row tiles 2 k + g of the block's ROWS (cell, axis) rows
+    // warpgroup g takes the 128-row tiles 2 k + g of the block's ROWS rows, axis-major (a tile's rows share their axis); a thread
+    // forms its row's 25 features and stores them as four 16-byte core-matrix rows (a lane per row and quantity with 2-byte
+    // stores took 32 store instructions a row: 1.28 -> 0.83 ms per refresh at 192^3)
+    static_assert(NC % 128 == 0, "the rows of a tile share their axis");
+    const int row = threadIdx.x & 127;
     for (int t0 = 128 * g; t0 < ROWS; t0 += 256) {
-        // features of the tile's rows: warp q of the group rows 32 q .. 32 q + 31, one lane per (row, quantity)
-        for (int it = lane; it < 32 * kSensQ; it += 32) {
-            const int row = 32 * q + it / kSensQ, sq = it % kSensQ, r = t0 + row;
-            float f[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            if (r < ROWS) {
-                const int c = r / DIM, axis = r % DIM;
+        const int axis = t0 / NC, c = t0 % NC + row;
+        {
+            const int e = ((DIM == 3 ? c / (BX * BY) + 2 : 0) * EY + (c / BX) % BY + 2) * EX + c % BX + 2;
+            const int st_ = axis == 0 ? 1 : (axis == 1 ? EX : EX * EY);
+            float f[2 * 13];
+            f[25] = 0.0f;
+            const float rho = P[e], pr = P[3 * PS + e];
+            const float sc[3] = {sensor_scale<float>(0, rho, pr, gam, pinf), sensor_scale<float>(1, rho, pr, gam, pinf),
+                                 sensor_scale<float>(4, rho, pr, gam, pinf)};
+#pragma unroll
+            for (int sq = 0; sq < kSensQ; ++sq) {
                 const int var = sensor_var<NV>(sq, axis);
+                float v[5], fq[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
                 if (var >= 0) {
-                    const int e = ((DIM == 3 ? c / (BX * BY) + 2 : 0) * EY + (c / BX) % BY + 2) * EX + c % BX + 2;
-                    const int st_ = axis == 0 ? 1 : (axis == 1 ? EX : EX * EY);
-                    float v[5];
 #pragma unroll
                     for (int k = 0; k < 5; ++k) v[k] = P[var * PS + e + (k - 2) * st_];
-                    sensor_quantity_features(v, sensor_scale<float>(sq, P[e], P[3 * PS + e], gam, pinf), f);
+                    sensor_quantity_features(v, sc[sq == 0 ? 0 : (sq == 4 ? 2 : 1)], fq);
                 }
-            }
 #pragma unroll
-            for (int k = 0; k < 5; ++k) st.X[g][tc::cl_index(row, 5 * sq + k)] = __float2bfloat16_rn(f[k]);
+                for (int k = 0; k < 5; ++k) f[5 * sq + k] = fq[k];
+            }
+            uint32_t pk[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) pk[k] = k < 13 ? pack_bf16(f[2 * k], f[2 * k + 1]) : 0u;   // (the padding inputs zero)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(&st.X[g][tc::cl_index(row, 8 * k)]) = make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
         }
-        // the padding inputs (the previous tile's hidden values sit there)
-        for (int k = kSensF; k < kSensK; ++k) st.X[g][tc::cl_index(threadIdx.x & 127, k)] = __float2bfloat16_rn(0.0f);
         tma::fence_proxy_async();
         const float z = sens_tc_tile(st, g, phase);
-        const int r = t0 + 32 * q + lane;
-        if (r < ROWS) {
-            const int c = r / DIM, axis = r % DIM;
-            const int i = o0 + c % BX, j = o1 + (c / BX) % BY, k = DIM == 3 ? o2 + c / (BX * BY) : 0;
-            // a tensor-core step that did not complete leaves the row WENO5-Z
-            if (i < m.nx && j < m.ny && k < m.nz) flags[axis * m.plane + ((long long)k * m.ny + j) * m.nx + i] = (!st.fail && z < theta) ? 0 : 1;
-        }
+        const int i = o0 + c % BX, j = o1 + (c / BX) % BY, k = DIM == 3 ? o2 + c / (BX * BY) : 0;
+        // a tensor-core step that did not complete leaves the row WENO5-Z
+        if (i < m.nx && j < m.ny && k < m.nz) flags[axis * m.plane + ((long long)k * m.ny + j) * m.nx + i] = (!st.fail && z < theta) ? 0 : 1;
     }
     if (st.fail && threadIdx.x == 0 && err) atomicExch(err, 6);
     sens_tc_release(st);
