@@ -108,14 +108,25 @@ __global__ void __launch_bounds__(NT, 3) hancock_kernel(const HancockArgs a) {
     const double half_dt = a.ctl->half_dt;
     const double hx = half_dt / m.dx, hy = half_dt / m.dy;
 
-    // ---- 1. primitive box: cells ox-2 .. ox+TX+1, oy-2 .. oy+TY+1
+    // ---- 1. primitive box: cells ox-2 .. ox+TX+1, oy-2 .. oy+TY+1. A box inside the mesh needs no boundary rule, and one
+    // without a solid cell no rule of the immersed body (both uniform over the CTA).
+    const bool inner = ox >= 2 && ox + TX + 2 <= nx && oy >= 2 && oy + TY + 2 <= ny;
+    int solid_here = 0;
     for (int p = tid; p < NP; p += NT) {
         const int i = ox + p % PX - 2, j = oy + p / PX - 2;
-        const St<double, 4> w = c2p(e, stencil_cons<2, 4, FULL>(m, a.bc, e, a.U, i, j, 0));
+        St<double, 4> u;
+        if (inner) {
+            const long long c = (long long)j * nx + i;
+            u = read_state<4>(a.bc, a.U, m.plane, c);
+            if (a.bc.solid) solid_here |= a.bc.solid[c];
+        } else {
+            u = stencil_cons<2, 4, FULL>(m, a.bc, e, a.U, i, j, 0);
+        }
+        const St<double, 4> w = c2p(e, u);
 #pragma unroll
         for (int q = 0; q < 4; ++q) P[q * NP + p] = w[q];
     }
-    __syncthreads();
+    const unsigned char* const sol = __syncthreads_or(!inner || solid_here) ? a.bc.solid : nullptr;
     // ---- 2. the four states of the cells ox-1 .. ox+TX, oy-1 .. oy+TY (not the four corners)
     const bool wrap_x = a.bc.halo[0] == kHaloWrap, wrap_y = a.bc.halo[2] == kHaloWrap;
     for (int p = tid; p < NB; p += NT) {
@@ -141,10 +152,11 @@ __global__ void __launch_bounds__(NT, 3) hancock_kernel(const HancockArgs a) {
             st[2 * ax] = p2c(e, wr);
         }
         // a real cell: of the mesh, of a periodic wrap, or of the neighbouring part beyond a part interface
-        const bool real = gi >= -1 && gi <= nx && gj >= -1 && gj <= ny && (wrap_x || held<FULL>(a.bc, 0, gi, nx)) && (wrap_y || held<FULL>(a.bc, 1, gj, ny));
+        const bool real = inner || (gi >= -1 && gi <= nx && gj >= -1 && gj <= ny && (wrap_x || held<FULL>(a.bc, 0, gi, nx)) &&
+                                    (wrap_y || held<FULL>(a.bc, 1, gj, ny)));
         if (real) {
             // the mesh cell (wrapped): sides without a halo give it the round trip of its own state there
-            const int ci = wrap_x ? (gi + nx) % nx : gi, cj = wrap_y ? (gj + ny) % ny : gj;
+            const int ci = inner || !wrap_x ? gi : (gi + nx) % nx, cj = inner || !wrap_y ? gj : (gj + ny) % ny;
             const bool b0 = ci == 0 && a.bc.halo[0] == kHaloNone, b1 = ci == nx - 1 && a.bc.halo[1] == kHaloNone;
             const bool b2 = cj == 0 && a.bc.halo[2] == kHaloNone, b3 = cj == ny - 1 && a.bc.halo[3] == kHaloNone;
             if (b0 || b1 || b2 || b3) {
@@ -156,7 +168,6 @@ __global__ void __launch_bounds__(NT, 3) hancock_kernel(const HancockArgs a) {
             }
             // an immersed body: its cells are not predicted, nor the sides of a cell that face one (the states of those
             // sides keep the time level of the ghost cells; solid_side_mask, Schemes.cpp:2890-2905, no wrap-around)
-            const unsigned char* sol = a.bc.solid;
             const bool is_solid = sol && sol[(long long)cj * nx + ci];
             int sd = 0;
             if (sol && !is_solid) {

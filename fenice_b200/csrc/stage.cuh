@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(NT, MB) stage2d_kernel(const StageArgs a, cons
     const Eos<double>& e = a.eos;
     const int tid = threadIdx.x, cta = blockIdx.x;
     const int ox = (cta % tiles_x) * TX, oy = row0 + (cta / tiles_x) * TY;
+    const bool inner = ox >= H && ox + TX + H <= m.nx && oy >= H && oy + TY + H <= m.ny;   // no boundary rule (uniform over the CTA)
     for (int c = tid; c < S::NCROSS; c += NT) {
         int i, j;
         if (c < S::NROW) {
@@ -347,7 +348,9 @@ __global__ void __launch_bounds__(NT, MB) stage2d_kernel(const StageArgs a, cons
             i = (c - S::NROW) % TX;
             j = r < H ? r - H : TY + r - H;
         }
-        const St<double, NV> w = c2p(e, stencil_cons<2, NV, false>(m, a.bc, e, a.U, ox + i, oy + j, 0));
+        const St<double, NV> u = inner ? read_cell<NV>(a.U, m.plane, (long long)(oy + j) * m.nx + ox + i)
+                                       : stencil_cons<2, NV, false>(m, a.bc, e, a.U, ox + i, oy + j, 0);
+        const St<double, NV> w = c2p(e, u);
 #pragma unroll
         for (int q = 0; q < NV; ++q) P[q * NP + (j + H) * PX + i + H] = w[q];
     }
