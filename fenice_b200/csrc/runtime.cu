@@ -577,10 +577,18 @@ template <int DIM> StageLauncher stage_launcher(int recon, int riemann, bool ful
 // 256^3 against 4.76 with 192 threads, the same bits)
 constexpr int kViscNT = 384;
 cudaError_t prepare_viscous() {
-    return cudaFuncSetAttribute(viscous_kernel<8, 8, 8, kViscNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscShape<8, 8, 8>::SMEM_BYTES);
+    const cudaError_t e = cudaFuncSetAttribute(viscous_kernel<8, 8, 8, kViscNT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)ViscShape<8, 8, 8>::SMEM_BYTES);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(viscous_kernel<8, 8, 8, kViscNT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)ViscShape<8, 8, 8>::SMEM_BYTES);
 }
 cudaError_t launch_viscous(const ViscArgs& a, int nblocks, cudaStream_t s) {
-    viscous_kernel<8, 8, 8, kViscNT><<<nblocks, kViscNT, ViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
+    bool walls = false;
+    for (int side = 0; side < 6; ++side) walls = walls || !a.through[side];
+    if (walls)
+        viscous_kernel<8, 8, 8, kViscNT, true><<<nblocks, kViscNT, ViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
+    else
+        viscous_kernel<8, 8, 8, kViscNT, false><<<nblocks, kViscNT, ViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
     return cudaGetLastError();
 }
 // the 2-D sweep: 16 x 16 tiles, 256 threads (the mixed form uses it too: the FP32 viscous kernel is 3-D only)

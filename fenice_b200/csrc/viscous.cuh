@@ -142,51 +142,49 @@ template <int TX, int TY, int TZ> struct ViscShape {
     static constexpr int cmax(int x, int y) { return x > y ? x : y; }
     static constexpr int NE = cmax(cmax((TX + 2) * TY * TZ, TX * (TY + 2) * TZ), TX * TY * (TZ + 2));
     static constexpr int NF = cmax(cmax((TX + 1) * TY * TZ, TX * (TY + 1) * TZ), TX * TY * (TZ + 1));
-    // B [5][NB] padded conservative box, G [4][NE] gradient entries, F [4][NF] face fluxes (components 1..4), acc [5][NC], red [32]
-    static constexpr int SMEM_DOUBLES = 5 * NB + 4 * NE + 4 * NF + 5 * NC + 32;
+    // B [6][NB] padded box (rho, rho u, rho v, rho w, T, 1 / rho), G [4][NE] gradient entries, F [4][NF] face fluxes (components
+    // 1..4), acc [4][NC], red [32]
+    static constexpr int SMEM_DOUBLES = 6 * NB + 4 * NE + 4 * NF + 4 * NC + 32;
     static constexpr size_t SMEM_BYTES = sizeof(double) * SMEM_DOUBLES;
 };
 
-template <int TX, int TY, int TZ, int NT>
+// A box position's T, 1 / rho and (a cell's) speed bound are formed once, as it is loaded; the sweeps take velocities as
+// (rho u) (1 / rho), the product cons_to_prim takes. WALLS = false: a launch whose every side wraps or is a part interface,
+// the ghost rules and wall tests compiled out (the sweep waits for instructions, 2.6 of its 16 cycles per issue, with them).
+template <int TX, int TY, int TZ, int NT, bool WALLS>
 __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
     using S = ViscShape<TX, TY, TZ>;
     constexpr int NC = S::NC, BX = S::BX, BY = S::BY, NB = S::NB;
     extern __shared__ double smem[];
-    double* B = smem;                 // [5][NB]
-    double* G = B + 5 * NB;           // [4][NE]
+    double* B = smem;                 // [6][NB]
+    double* G = B + 6 * NB;           // [4][NE]
     double* Fv = G + 4 * S::NE;       // [4][NF]
-    double* acc = Fv + 4 * S::NF;     // [5][NC]
-    double* red = acc + 5 * NC;
+    double* acc = Fv + 4 * S::NF;     // [4][NC] (component 0 of every viscous flux is +0)
+    double* red = acc + 4 * NC;
     if (!*a.gate) return;
     const Mesh& m = a.m;
     const int tid = threadIdx.x, b = blockIdx.x + a.b0;
     const int o3[3] = {(b % a.tiles[0]) * TX, ((b / a.tiles[0]) % a.tiles[1]) * TY, (b / (a.tiles[0] * a.tiles[1])) * TZ};
     const int n3[3] = {m.nx, m.ny, m.nz};
     const double h[3] = {m.dx, m.dy, m.dz};
-    // the momentum slots of the velocity components, and the (a, b) of the four gradient entries the faces of axis d read,
-    // in the reference's CrossGhosts order (cpp/src/Physics.cpp:653-667); compile-time tables, constant indices in the
-    // unrolled sweeps
-    constexpr int mom[3] = {1, 2, 4};
+    // the (a, b) of the four gradient entries the faces of axis d read, in the reference's CrossGhosts order
+    // (cpp/src/Physics.cpp:653-667); compile-time tables, constant indices in the unrolled sweeps
     constexpr int GA[3][4] = {{0, 1, 2, 0}, {0, 1, 2, 1}, {0, 1, 2, 2}};
     constexpr int GB[3][4] = {{1, 1, 2, 2}, {0, 0, 2, 2}, {0, 1, 0, 1}};
     // box position (tile-relative cell index -1 .. T per axis) -> shared-memory index
     auto bidx = [&](int i, int j, int k) { return ((k + 1) * BY + (j + 1)) * BX + (i + 1); };
-    auto cons = [&](int p) {
-        St<double, 5> u;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) u[q] = B[q * NB + p];
-        return u;
-    };
+    auto vel = [&](int c, int p) { return B[(1 + c) * NB + p] * B[5 * NB + p]; };   // cons_to_prim's rho u * (1 / rho)
 
     // whether a side of the tile lies on a side of the mesh that is neither periodic nor a part interface (without one,
     // every box position is a cell the arrays hold, after the periodic wrap, and no face of the tile has a wall rule),
     // and whether the tile lies wholly inside the mesh
     bool walls = false;
 #pragma unroll
-    for (int x = 0; x < 3; ++x)
+    for (int x = 0; x < 3 && WALLS; ++x)
         walls = walls || (o3[x] == 0 && !a.through[2 * x]) || (o3[x] + (x == 0 ? TX : (x == 1 ? TY : TZ)) >= n3[x] && !a.through[2 * x + 1]);
     const bool full = o3[0] + TX <= n3[0] && o3[1] + TY <= n3[1] && o3[2] + TZ <= n3[2];
 
+    double smax = 0.0;
     // ---- 0. the padded conservative state of the tile and one cell around it. A position beyond a periodic side is the
     // wrapped cell (so the box holds the neighbours the reference reads for that cell); the rest is the reference's
     // padded array (padded_cons). The eight corners are never read.
@@ -198,9 +196,24 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
         // a tile that overhangs the mesh: positions past the ghost layer are clamped onto it (their results are not used)
 #pragma unroll
         for (int x = 0; x < 3; ++x) g[x] = box_clamp(a, x, g[x], n3[x]);
-        const St<double, 5> u = walls ? padded_cons(a, g[0], g[1], g[2]) : cell_at(a, g[0], g[1], g[2]);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) B[q * NB + e] = u[q];
+        const St<double, 5> u = WALLS && walls ? padded_cons(a, g[0], g[1], g[2]) : cell_at(a, g[0], g[1], g[2]);
+        double inv;
+        const St<double, 5> W = c2p(a.eos, u, inv);
+        B[e] = u[0];
+        B[NB + e] = u[1];
+        B[2 * NB + e] = u[2];
+        B[3 * NB + e] = u[4];
+        B[4 * NB + e] = W[3] / W[0];
+        B[5 * NB + e] = inv;
+        const int bx = e % BX, by = (e / BX) % BY, bz = e / (BX * BY);
+        if (bx >= 1 && bx <= TX && by >= 1 && by <= TY && bz >= 1 && bz <= TZ && o3[0] + bx <= n3[0] && o3[1] + by <= n3[1] && o3[2] + bz <= n3[2]) {
+            // the cell's speed bound
+            const double rho = W[0];
+            const double nu_eff = vmax((4.0 / 3.0) * (a.mu / rho), (a.k_cond * (a.eos.gamma - 1.0)) / rho) + 1e-12;
+            const double vm = vmax(vmax(fabs(W[1]), fabs(W[2])), fabs(W[4]));
+            const double s = vm + sound_speed(a.eos, W[3], rho) + 2.0 * a.L * a.inv_h2 * nu_eff;
+            if (s > smax) smax = s;
+        }
     }
     __syncthreads();
 
@@ -215,15 +228,14 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
             int l[3] = {e % E[0], (e / E[0]) % E[1], e / (E[0] * E[1])};
             l[d] -= 1;
             const int p = bidx(l[0], l[1], l[2]);
-            const St<double, 5> w = c2p(a.eos, cons(p));
-            const double rho = w[0];
+            const double rho = vmax(B[p], Num<double>::eos_eps);
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 const int ga = GA[d][s], gb = GB[d][s];
                 const int off = gb == 0 ? 1 : (gb == 1 ? BX : BX * BY);
-                const double gq = (B[mom[ga] * NB + p + off] - B[mom[ga] * NB + p - off]) / (2.0 * h[gb]);
+                const double gq = (B[(1 + ga) * NB + p + off] - B[(1 + ga) * NB + p - off]) / (2.0 * h[gb]);
                 const double g0 = (B[p + off] - B[p - off]) / (2.0 * h[gb]);
-                G[s * S::NE + e] = (gq - velc(w, ga) * g0) / rho;
+                G[s * S::NE + e] = (gq - vel(ga, p) * g0) / rho;
             }
         }
         __syncthreads();
@@ -247,9 +259,8 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
                 int lc[3] = {f3[0], f3[1], f3[2]};
                 lc[d] -= 1;
                 const int pL = bidx(lc[0], lc[1], lc[2]), pR = pL + bstride;
-                const St<double, 5> wL = c2p(a.eos, cons(pL)), wR = c2p(a.eos, cons(pR));
-                const double vL[3] = {wL[1], wL[2], wL[4]}, vR[3] = {wR[1], wR[2], wR[4]};
-                const double TL = wL[3] / wL[0], TR = wR[3] / wR[0];
+                const double vL[3] = {vel(0, pL), vel(1, pL), vel(2, pL)}, vR[3] = {vel(0, pR), vel(1, pR), vel(2, pR)};
+                const double TL = B[4 * NB + pL], TR = B[4 * NB + pR];
                 // cross terms: the cells on either side; at a side that is not periodic the cell next to it (both slots)
                 const bool lo_wall = lo && !a.through[2 * d], hi_wall = hi && !a.through[2 * d + 1];
                 const int xL = lo_wall ? eR : eL;
@@ -258,7 +269,7 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
                 double Gc[4];
 #pragma unroll
                 for (int s = 0; s < 4; ++s) {
-                    if (phys) {
+                    if (WALLS && phys) {
                         // d u_a / d x_b from the tangential difference of the face values (ghost and cell averages)
                         const int ga = GA[d][s], gb = GB[d][s];
                         const int pg = lo ? pL : pR, pc = lo ? pR : pL;
@@ -267,9 +278,7 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
 #pragma unroll
                         for (int w2 = 0; w2 < 2; ++w2) {
                             const int o = w2 == 0 ? off : -off;
-                            const St<double, 5> wg = c2p(a.eos, cons(pg + o));
-                            const St<double, 5> wc = c2p(a.eos, cons(pc + o));
-                            fc[w2] = 0.5 * (velc(wg, ga) + velc(wc, ga));
+                            fc[w2] = 0.5 * (vel(ga, pg + o) + vel(ga, pc + o));
                         }
                         Gc[s] = (fc[0] - fc[1]) / (2.0 * h[gb]);
                     } else {
@@ -314,8 +323,8 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
             const int fl = (c3[2] * Fd[1] + c3[1]) * Fd[0] + c3[0];
             const int fr = fl + (d == 0 ? 1 : (d == 1 ? Fd[0] : Fd[0] * Fd[1]));
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                const double dif = q == 0 ? 0.0 - 0.0 : Fv[(q - 1) * S::NF + fr] - Fv[(q - 1) * S::NF + fl];
+            for (int q = 0; q < 4; ++q) {
+                const double dif = Fv[q * S::NF + fr] - Fv[q * S::NF + fl];
                 acc[q * NC + c] = d == 0 ? 0.0 + dif : acc[q * NC + c] + dif;
             }
         }
@@ -325,21 +334,15 @@ __global__ void __launch_bounds__(NT) viscous_kernel(const ViscArgs a) {
     sweep(std::integral_constant<int, 0>{});
     sweep(std::integral_constant<int, 1>{});
     sweep(std::integral_constant<int, 2>{});
-    // ---- residual and speed bound
-    double smax = 0.0;
+    // ---- the residual
     for (int c = tid; c < NC; c += NT) {
         const int c3[3] = {c % TX, (c / TX) % TY, c / (TX * TY)};
         const int g3[3] = {o3[0] + c3[0], o3[1] + c3[1], o3[2] + c3[2]};
         if (g3[0] >= m.nx || g3[1] >= m.ny || g3[2] >= m.nz) continue;
         const long long cell = ((long long)g3[2] * m.ny + g3[1]) * m.nx + g3[0];
+        a.Rv[cell] = 0.0;
 #pragma unroll
-        for (int q = 0; q < 5; ++q) a.Rv[q * m.plane + cell] = acc[q * NC + c] * m.inv_cell;
-        const St<double, 5> w = c2p(a.eos, cons(bidx(c3[0], c3[1], c3[2])));
-        const double rho = w[0];
-        const double nu_eff = vmax((4.0 / 3.0) * (a.mu / rho), (a.k_cond * (a.eos.gamma - 1.0)) / rho) + 1e-12;
-        const double vm = vmax(vmax(fabs(w[1]), fabs(w[2])), fabs(w[4]));
-        const double s = vm + sound_speed(a.eos, w[3], rho) + 2.0 * a.L * a.inv_h2 * nu_eff;
-        if (s > smax) smax = s;
+        for (int q = 1; q < 5; ++q) a.Rv[q * m.plane + cell] = acc[(q - 1) * NC + c] * m.inv_cell;
     }
     const double bm = block_max<NT>(smax, red);
     if (tid == 0) stage_finish(a.fin, a.blockmax, b, bm);
