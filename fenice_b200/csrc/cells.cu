@@ -110,8 +110,11 @@ template <int NV> __device__ __forceinline__ double entry(const CellArgs& a, int
     return c2p(a.eos, Ug)[q];
 }
 
+// Bound by the latency of FP64 chains: four CTAs per SM (32 warps, 64 registers, some spilled). 64^3 Taylor-Green, 5 steps:
+// 3.86 ms with two CTAs, 3.57 with three, 3.45 with four (3.76 with the ghost rules of entry
+// in a call instead of inlined).
 template <int NV, int RECON, int RIEMANN, int MODE = kFacesFlux>
-__global__ void __launch_bounds__(kCellsNT) k_cells_faces(const CellArgs a) {
+__global__ void __launch_bounds__(kCellsNT, 4) k_cells_faces(const CellArgs a) {
     __shared__ double red[32];
     const long long f = blockIdx.x * (long long)kCellsNT + threadIdx.x;
     double s = 0.0;
