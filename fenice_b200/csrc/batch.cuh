@@ -68,6 +68,7 @@ __device__ __forceinline__ void batch_item_args(const BatchArgs& b, const BatchP
     sa.Rvf = nullptr;
     sa.blockmax = nullptr;
     sa.fin = Fin{};
+    sa.Rd = nullptr;
     sa.ctl = nullptr;
     sa.gate = nullptr;
     sa.sens_flags = nullptr;   // (shared memory is not initialised: every pointer a stage sweep may test is set here)

@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(MarchShape::NT, MB) mixed_march_kernel(const S
 template <int W_> struct March2Shape {
     static constexpr int W = W_, NT = W_, NHALO = 5, RP = W_ + 8, RAW = W_ + 8;
     // doubles: red [32], raw row [4][RAW] (the column, three rows ahead, then the halo of the next row), u [4][W], u0 [4][W],
-    // viscous residual [4][W]; float4: P [RP], FX [W] (the fluxes of rho, rho E, rho u, rho v)
-    static constexpr size_t SMEM_BYTES = 8 * (32 + 4 * RAW + 12 * W) + 16 * (RP + W);
+    // viscous residual [4][W], the increments Rd of the raw row and of u; float4: P [RP], FX [W] (the fluxes of rho, rho E, rho u, rho v)
+    static constexpr size_t SMEM_BYTES = 8 * (32 + 8 * RAW + 16 * W) + 16 * (RP + W);
 };
 // the face along axis A from its six cells (rho, p, u, v)
 template <int A, int RIEMANN>
@@ -394,7 +394,9 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
     double* Ru = Rc + 4 * RAW;
     double* R0 = Ru + 4 * W;
     double* Rv = R0 + 4 * W;
-    float4* P4 = reinterpret_cast<float4*>(Rv + 4 * W);
+    double* Dc = Rv + 4 * W;
+    double* Du = Dc + 4 * RAW;
+    float4* P4 = reinterpret_cast<float4*>(Du + 4 * W);
     float4* FX4 = P4 + S::RP;
     if (!*a.gate) return;
     const Mesh& m = a.m;
@@ -411,31 +413,42 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
     const bool halo = tid < S::NHALO;
     const int hx = tid < 3 ? tid - 3 : W + tid - 3;
     if (halo) hoff = march_cell(a.bc, 0, x0 + hx, m.nx, hside);
-    auto prim = [&](const double* raw, long long stride, int side) {
+    const double dt = a.ctl->dt;
+    auto formed = [&](double u, double d) { return __dadd_rn(u, __dmul_rn(dt, d)); };   // (rounded as k_axpy rounds it)
+    auto prim = [&](const double* raw, const double* inc, long long stride, int side) {
         St<double, NV> u;
 #pragma unroll
-        for (int q = 0; q < NV; ++q) u[q] = raw[q * stride];
+        for (int q = 0; q < NV; ++q) u[q] = a.Rd ? formed(raw[q * stride], inc[q * stride]) : raw[q * stride];
         if (side >= 0) u = ghost_state(a.eos, a.bc, side, u);
         double inv;
         return prim_d(a.eos, u, inv);
     };
     auto fetch_core = [&](int g) {
         int sy;
-        const double* src = a.U + (long long)march_cell(a.bc, 1, g, m.ny, sy) * m.nx + coff;
+        const long long at = (long long)march_cell(a.bc, 1, g, m.ny, sy) * m.nx + coff;
 #pragma unroll
-        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * RAW + tid, src + q * m.plane);
+        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * RAW + tid, a.U + q * m.plane + at);
+        if (a.Rd)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(Dc + q * RAW + tid, a.Rd + q * m.plane + at);
     };
     auto fetch_halo = [&](int g) {
-        const double* src = a.U + (long long)g * m.nx + hoff;
+        const long long at = (long long)g * m.nx + hoff;
 #pragma unroll
-        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * RAW + W + tid, src + q * m.plane);
+        for (int q = 0; q < NV; ++q) cp_async8(Rc + q * RAW + W + tid, a.U + q * m.plane + at);
+        if (a.Rd)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(Dc + q * RAW + W + tid, a.Rd + q * m.plane + at);
     };
     auto fetch_cell = [&](int g) {
         const long long cell = (long long)g * m.nx + coff;
         if (a.mode != kStoreR)
 #pragma unroll
             for (int q = 0; q < NV; ++q) cp_async8(Ru + q * W + tid, a.U + q * m.plane + cell);
-        if (a.mode == kCombine)
+        if (a.Rd)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) cp_async8(Du + q * W + tid, a.Rd + q * m.plane + cell);
+        else if (a.mode == kCombine)
 #pragma unroll
             for (int q = 0; q < NV; ++q) cp_async8(R0 + q * W + tid, a.U0 + q * m.plane + cell);
         if (a.Rv)
@@ -464,11 +477,10 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
         int sy;
-        const double* src = a.U + (long long)march_cell(a.bc, 1, za - 3 + p, m.ny, sy) * m.nx + coff;
-        r[p] = rounded(prim(src, m.plane, sy >= 0 ? sy : cside));
+        const long long at = (long long)march_cell(a.bc, 1, za - 3 + p, m.ny, sy) * m.nx + coff;
+        r[p] = rounded(prim(a.U + at, a.Rd + at, m.plane, sy >= 0 ? sy : cside));
     }
     const float Ax = (float)m.area[0], Ay = (float)m.area[1];
-    const double dt = a.ctl->dt;
     float smax = 0.0f;
     float4 Fl = make_float4(0.0f, 0.0f, 0.0f, 0.0f), Fh;   // the y faces below and above the row
     int lin = 0, tile_end = za - 1;   // bit 0, 1: the thread's x and y faces are linear; the row after which to look again
@@ -481,9 +493,9 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
             for (int p = 0; p < 5; ++p) r[p] = r[p + 1];
             int sy;
             march_cell(a.bc, 1, k + 3, m.ny, sy);
-            r[5] = rounded(prim(Rc + tid, RAW, sy >= 0 ? sy : cside));
+            r[5] = rounded(prim(Rc + tid, Dc + tid, RAW, sy >= 0 ? sy : cside));
             P4[tid + 3] = r[2];
-            if (halo) P4[hx + 3] = rounded(prim(Rc + W + tid, RAW, hside));
+            if (halo) P4[hx + 3] = rounded(prim(Rc + W + tid, Dc + W + tid, RAW, hside));
             if (k + 1 < zb) {
                 fetch_core(k + 4);
                 if (halo) fetch_halo(k + 1);
@@ -516,7 +528,8 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
 #pragma unroll
             for (int q = 0; q < NV; ++q) {
                 in.u[q] = a.mode != kStoreR ? Ru[q * W + tid] : 0.0;
-                in.u0[q] = a.mode == kCombine ? R0[q * W + tid] : 0.0;
+                in.u0[q] = a.Rd ? in.u[q] : (a.mode == kCombine ? R0[q * W + tid] : 0.0);
+                if (a.Rd) in.u[q] = formed(in.u[q], Du[q * W + tid]);
                 in.rv[q] = a.Rv ? Rv[q * W + tid] : 0.0;
             }
             const float4 xl = FX4[tid], xr = FX4[tid + 1];

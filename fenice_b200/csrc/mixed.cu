@@ -93,6 +93,7 @@ cudaError_t mixed_viscous_prepare() {
         e = cudaFuncSetAttribute(mixed_viscous_march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscMarchShape::SMEM_BYTES);
     return e;
 }
+bool mixed_stage_marches(const StageArgs& a, int dim) { return can_march(a, dim); }
 cudaError_t mixed_viscous_launch(const ViscArgs& a, int nblocks, cudaStream_t s) {
     bool march = !a.bc.slot;
     for (int side = 0; side < 6; ++side) march = march && a.through[side];

@@ -34,6 +34,8 @@ struct StageArgs {
     int mode;
     double ca, cb;              // COMBINE coefficients
     const double* U;            // the state the residual is taken of (read with halos)
+    // mixed_march2_kernel (march.cuh): the state is U + dt Rd, formed as it is read (null: U); then U0 is U
+    const double* Rd;
     const double* U0;           // COMBINE: the state at the start of the step (read at the cell only)
     double* out;                // R or the updated state (never aliases U; may alias U0)
     const double* Rv;           // viscous residual to add (null: none)
