@@ -846,17 +846,17 @@ def gpu_arm(args, world, rank, local):
                "timing": "host wall clock around fvg_step_host: pinned host state in, one step, pinned host state out"}
     mixed.close()
 
-    rl_l = roofline_of(tm_l, ms_l, cells, "mixed_stage_kernel_tma<LowMach, gated> (FP32 reconstruction, linear or WENO5-Z per tile-axis, + "
-                       "Riemann + balance, FP64 RK update; the cross form on tiles linear along every axis)",
-                       ncu_traffic(n, "mixed_stage_kernel_tma_gated_3d.json"), ncu_profile("mixed_stage_kernel_tma_gated_3d.json"))
-    rl_m = roofline_of(tm_m, ms_m, cells, "mixed_stage_kernel_tma<LowMach> (the per-axis sweep: FP32 WENO5-Z + Riemann + balance, FP64 RK update)",
-                       ncu_traffic(n, "mixed_stage_kernel_weno5_3d.json"), ncu_profile("mixed_stage_kernel_weno5_3d.json"))
-    rl_p = roofline_of(tm_p, ms_p, cells, "stage_kernel<3, WENO5, LowMach> (FP64, the reference's arithmetic)",
+    rl_l = roofline_of(tm_l, ms_l, cells, "mixed_march_kernel<LowMach, gated> (FP32 reconstruction, linear or WENO5-Z per tile-axis, + "
+                       "Riemann + balance, FP64 RK update; columns marched along z)",
+                       ncu_traffic(n, "mixed_march_kernel_gated_3d.json"), ncu_profile("mixed_march_kernel_gated_3d.json"))
+    rl_m = roofline_of(tm_m, ms_m, cells, "mixed_march_kernel<LowMach> (FP32 WENO5-Z + Riemann + balance, FP64 RK update; columns marched along z)",
+                       ncu_traffic(n, "mixed_march_kernel_3d.json"), ncu_profile("mixed_march_kernel_3d.json"))
+    rl_p = roofline_of(tm_p, ms_p, cells, "stage3_kernel<WENO5, LowMach> (FP64, the reference's arithmetic)",
                        ncu_traffic(n, "stage_kernel_weno5_3d.json"), ncu_profile("stage_kernel_weno5_3d.json"))
-    # per RK3 step: 3 viscous + 3 stage + dt + axpy + 2 stage maxima + end; one begin per run; the gated run adds the
-    # sensor's refresh (network, 3 dilation passes, tile reduction) to every step (the kernels return at once off the
-    # refresh steps)
-    launches = 3 * (args.steps * 11 + 1) + args.steps * 5
+    # per RK3 step: 3 viscous + 3 stage, in the plain form an axpy (the stages set dt and end the step themselves, and
+    # the mixed form's third stage forms its state as it reads it); one begin per run; the gated run adds the sensor's
+    # refresh (network, rows, tiles) to every step (the kernels return at once off the refresh steps)
+    launches = 3 * (args.steps * 6 + 1) + args.steps * 4
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": ms_l / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32 stencil / f64 state (mixed form) with bf16 sensor; plain form f64",
