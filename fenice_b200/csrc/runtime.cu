@@ -110,16 +110,6 @@ __global__ void k_hancock_dt(Ctl* c) {
     if (!c->active) return;
     hancock_dt(c);
 }
-// the step's speed: the Hancock residual's, max the viscous bound (Simulation.cpp:1038-1041), lagged to the next step
-__global__ void k_hancock_end(Ctl* c, const double* bm, int nb, const double* bmv, int nbv) {
-    if (!c->active) return;
-    const double s = block_reduce_max(bm, nb, bmv, nbv);
-    if (threadIdx.x == 0) {
-        c->s_lag = s;
-        finish_step(c, s);
-    }
-}
-
 // the end of a step whose stages folded their speeds into the control block, where another kernel runs between the last
 // stage and it (the immersed body's reset)
 __global__ void k_end_folded(Ctl* c, int hancock) {
