@@ -348,6 +348,7 @@ __global__ void k_part_unpack(double* U, long long plane, long long area, int de
 
 // out = a + dt b over the state planes (TimeScheme.cpp:27-59: axpy)
 __global__ void k_axpy(const Ctl* c, double* out, const double* a, const double* b, long long plane, long long n, int nvar) {
+    after_launch_before();
     if (!c->active) return;
     const double dt = c->dt;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n * nvar; e += (long long)gridDim.x * blockDim.x) {
@@ -525,11 +526,12 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct StageK {
     // tiles a third as high (where its CTAs need not be its tiles: the speeds folded into the control block).
     static cudaError_t launch2d(const StageArgs& a, int nblocks, cudaStream_t s) {
         const int row0 = a.b0 / a.tiles[0] * Tl::Y, row_end = (a.b0 + nblocks) / a.tiles[0] * Tl::Y, row1 = row_end < a.m.ny ? row_end : a.m.ny;
-        if (a.fin.kind != kFinNone && nblocks < 148 * 2) {
+        if (a.fin.kind != kFinNone && nblocks < kEarlyTiles) {
             constexpr int TY = 5, NT = 192;
             StageArgs b = a;
             b.fin.ctas = a.tiles[0] * ((row1 - row0 + TY - 1) / TY);
-            stage2d_kernel<RECON, RIEMANN, Tl::X, TY, NT, 3><<<b.fin.ctas, NT, Stage2Shape<RECON, Tl::X, TY>::SMEM_BYTES, s>>>(b, row0, row1, a.tiles[0]);
+            return launch_early(stage2d_kernel<RECON, RIEMANN, Tl::X, TY, NT, 3>, b.fin.ctas, NT, Stage2Shape<RECON, Tl::X, TY>::SMEM_BYTES, s, b, row0, row1,
+                                a.tiles[0]);
         } else {
             stage2d_kernel<RECON, RIEMANN, Tl::X, Tl::Y, Tl::NT, 2><<<nblocks, Tl::NT, Stage2Shape<RECON, Tl::X, Tl::Y>::SMEM_BYTES, s>>>(a, row0, row1,
                                                                                                                                   a.tiles[0]);
@@ -1285,7 +1287,11 @@ cudaError_t enqueue_step(fvg_run* r, bool refresh = true) {
         return cudaGetLastError();
     }
     const bool formed = forms_stage_state(r);
-    if (!formed) k_axpy<<<axpy_blocks(r), 256, 0, r->stream>>>(c, r->Ut, r->U, r->R, r->m.plane, r->m.ncells, r->nvar);
+    if (!formed && r->dim == 2 && r->nb < kEarlyTiles)
+        e = launch_early(k_axpy, axpy_blocks(r), 256, 0, r->stream, c, r->Ut, r->U, r->R, r->m.plane, r->m.ncells, r->nvar);
+    else if (!formed)
+        k_axpy<<<axpy_blocks(r), 256, 0, r->stream>>>(c, r->Ut, r->U, r->R, r->m.plane, r->m.ncells, r->nvar);
+    if (e) return e;
     const int last = !fold ? kFinNone : (r->ibm ? kFinMax : kFinStep);
     const int nstages = ts == FVG_TS_SSPRK2 ? 2 : 3;
     if (ts == FVG_TS_SSPRK2) {

@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(NT, MB) stage2d_kernel(const StageArgs a, cons
     double* P = smem;             // [4][NP] primitive cross
     double* Fl = P + 4 * NP;      // [4][NF] x faces, then y faces
     double* red = Fl + 4 * NF;
+    after_launch_before();
     if (!*a.gate) return;
     const Mesh& m = a.m;
     const Eos<double>& e = a.eos;
