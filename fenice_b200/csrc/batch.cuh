@@ -126,7 +126,7 @@ __device__ __forceinline__ void thin_y_fp64(const StageArgs& a, double* __restri
             const St<double, 4> W = c2p(a.eos, UL, inv);
             const double cs = sound_speed_inv(a.eos, W[3], inv);
             const double s = vmax(fabs(W[2] - cs), fabs(W[2] + cs));
-            if (isfinite(s)) {
+            if (isfinite(16.0 * s * UL[3])) {   // (their fluxes are finite too)
                 if (s > smax) smax = s;
                 continue;
             }

@@ -27,8 +27,8 @@ __device__ __forceinline__ float thin_face_mixed(const StageArgs& a, const GasF&
 // A work item of a one-cell-high mesh whose bottom and top have no halo (a shock tube; thin_y): a thread loads its cell
 // (the first ones the halo too), solves the low x face of its cell with all variables in registers, and updates the cell
 // from its own and its neighbour's flux: two barriers, where the general sweep takes four and passes every face value
-// through shared memory. The y faces of a cell between copies of it cancel and only their speed counts (riemann_f's for
-// equal states). The bits of mixed_axis along x and of its boundary faces along y.
+// through shared memory. The y faces of a cell between copies of it cancel, where their fluxes are finite, and only their
+// speed counts (riemann_f's for equal states). The bits of mixed_axis along x and of its boundary faces along y.
 template <int RECON, int RIEMANN, int TX, int NT>
 __device__ __forceinline__ void thin_row_mixed(const StageArgs& a, const GasF& gas, float sb, float weps, float* __restrict__ P, float* __restrict__ FX,
                                                int ox, double dt, float& smax) {
@@ -87,13 +87,17 @@ __device__ __forceinline__ void thin_row_mixed(const StageArgs& a, const GasF& g
     float acc[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] = -__fmul_rn(FX[q * NT + tid + 1] - FX[q * NT + tid], Ax);
-    if (copy_side(a.bc.type[2]) && copy_side(a.bc.type[3])) {
+    bool same = copy_side(a.bc.type[2]) && copy_side(a.bc.type[3]);
+    if (same) {
         const float* w = P + tid + H;
-        const float r = max_nan(w[0], Num<float>::eos_eps), p = max_nan(w[3 * RP], Num<float>::eos_eps), v = w[2 * RP];
+        const float r = max_nan(w[0], Num<float>::eos_eps), p = max_nan(w[3 * RP], Num<float>::eos_eps), u = w[RP], v = w[2 * RP];
         const float cs = sqrt_f(__fmul_rn(__fmul_rn(gas.g, __fadd_rn(p, gas.pi)), rcp_f(r)));
         const float s = max_nan(fabsf(__fsub_rn(v, cs)), fabsf(__fadd_rn(v, cs)));
-        if (s > smax) smax = s;
-    } else {
+        const float rE = __fmaf_rn(__fmul_rn(0.5f, r), __fmaf_rn(u, u, __fmul_rn(v, v)), __fmul_rn(__fadd_rn(p, gas.gpi), gas.g1));
+        same = __fmul_rn(s, rE) < 0.25f * kFaceRange;   // (finite fluxes; a state beyond riemann_f's range is solved)
+        if (same && s > smax) smax = s;
+    }
+    if (!same) {
         St<float, NV> Fb, Ft;
         const float s_b = thin_face_mixed<RIEMANN>(a, gas, sb, 2, i, Fb), s_t = thin_face_mixed<RIEMANN>(a, gas, sb, 3, i, Ft);
         if (s_b > smax) smax = s_b;

@@ -68,7 +68,7 @@ __device__ __forceinline__ float march_face(const GasF& gas, float sb, float wep
     f2_get(r1, uR, vR_);
     const float L[3] = {uL, vv, lw}, R[3] = {uR, vR_, rw};
     float vL[3] = {L[A], L[(A + 1) % 3], L[(A + 2) % 3]}, vR[3] = {R[A], R[(A + 1) % 3], R[(A + 2) % 3]}, Fv[3];
-    const float s = riemann_f<RIEMANN>(gas, sb, rL, pL, vL, rR, pR, vR, F.a.x, F.a.y, Fv);
+    const float s = riemann_face<RIEMANN>(gas, sb, rL, pL, vL, rR, pR, vR, F.a.x, F.a.y, Fv);
     F.a.z = Fv[(3 - A) % 3];
     F.a.w = Fv[(4 - A) % 3];
     F.w = Fv[(5 - A) % 3];
@@ -357,9 +357,10 @@ template <int W_> struct March2Shape {
     // viscous residual [4][W], the increments Rd of the raw row and of u; float4: P [RP], FX [W] (the fluxes of rho, rho E, rho u, rho v)
     static constexpr size_t SMEM_BYTES = 8 * (32 + 8 * RAW + 16 * W) + 16 * (RP + W);
 };
-// the face along axis A from its six cells (rho, p, u, v)
-template <int A, int RIEMANN>
-__device__ __forceinline__ float march2_face(const GasF& gas, float sb, float weps, bool linear, const float4 (&c)[6], float4& F) {
+// the face values along axis A from its six cells (rho, p, u, v): density, pressure and the velocities, the normal one first
+template <int A>
+__device__ __forceinline__ void march2_values(float weps, bool linear, const float4 (&c)[6], float& rL, float& pL, float (&vL)[2], float& rR, float& pR,
+                                              float (&vR)[2]) {
     const auto lo = [&](int p) { return f2(c[p].x, c[p].y); };
     const auto hi = [&](int p) { return f2(c[p].z, c[p].w); };
     F2 l0, l1, r0, r1;
@@ -374,15 +375,34 @@ __device__ __forceinline__ float march2_face(const GasF& gas, float sb, float we
         l1 = weno5z_f2(hi(0), hi(1), hi(2), hi(3), hi(4), weps);
         r1 = weno5z_f2(hi(5), hi(4), hi(3), hi(2), hi(1), weps);
     }
-    float rL, pL, rR, pR, vL[2], vR[2], Fv[2];
     f2_get(l0, rL, pL);
     f2_get(r0, rR, pR);
     f2_get(l1, vL[A], vL[1 - A]);
     f2_get(r1, vR[A], vR[1 - A]);
-    const float s = riemann_f<RIEMANN>(gas, sb, rL, pL, vL, rR, pR, vR, F.x, F.y, Fv);
+}
+// the face along axis A: its flux, speed and range (riemann_f)
+template <int A, int RIEMANN>
+__device__ __forceinline__ float march2_face(const GasF& gas, float sb, float weps, bool linear, const float4 (&c)[6], float4& F, float& range) {
+    float rL, pL, rR, pR, vL[2], vR[2], Fv[2];
+    march2_values<A>(weps, linear, c, rL, pL, vL, rR, pR, vR);
+    const float s = riemann_f<RIEMANN>(gas, sb, rL, pL, vL, rR, pR, vR, F.x, F.y, Fv, range);
     F.z = Fv[A];
     F.w = Fv[1 - A];
     return s;
+}
+// the same by riemann_wide, its face values formed once more (out of line: a row has one test for both its faces)
+struct March2F {
+    float4 F;
+    float s;
+};
+template <int A, int RIEMANN>
+__device__ __noinline__ March2F march2_wide(GasF gas, float sb, float weps, bool linear, float4 c0, float4 c1, float4 c2, float4 c3, float4 c4, float4 c5) {
+    const float4 c[6] = {c0, c1, c2, c3, c4, c5};
+    float rL, pL, rR, pR;
+    FaceF<2> L, R;
+    march2_values<A>(weps, linear, c, rL, pL, L.v, rR, pR, R.v);
+    const FaceF<2> o = riemann_wide<RIEMANN, 2>(gas, sb, rL, pL, L, rR, pR, R);
+    return March2F{make_float4(o.m, o.e, o.v[A], o.v[1 - A]), o.s};
 }
 template <int RIEMANN, bool GATED, int W, int MB>
 __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, const int z0, const int z1, const int lz, const int nslots) {
@@ -510,14 +530,28 @@ __global__ void __launch_bounds__(W, MB) mixed_march2_kernel(const StageArgs a, 
             }
         }
         __syncthreads();
-        float s = march2_face<1, RIEMANN>(gas, sb, weps, GATED && (lin & 2), r, Fh);
-        if (cell_in && s > smax) smax = s;
+        float4 F = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float range, range_x = 0.0f, sx = 0.0f, sy = march2_face<1, RIEMANN>(gas, sb, weps, GATED && (lin & 2), r, Fh, range);
+        const float4* c4 = P4 + tid;
         if (!first) {
-            float4 c[6], F;
-#pragma unroll
-            for (int p = 0; p < 6; ++p) c[p] = P4[tid + p];
-            s = march2_face<0, RIEMANN>(gas, sb, weps, GATED && (lin & 1), c, F);
-            if (face_in && s > smax) smax = s;
+            const float4 c[6] = {c4[0], c4[1], c4[2], c4[3], c4[4], c4[5]};
+            sx = march2_face<0, RIEMANN>(gas, sb, weps, GATED && (lin & 1), c, F, range_x);
+        }
+        if (!(max_nan(range, range_x) < kFaceRange)) {
+            const March2F y = march2_wide<1, RIEMANN>(gas, sb, weps, GATED && (lin & 2), r[0], r[1], r[2], r[3], r[4], r[5]);
+            if (!(range < kFaceRange)) {
+                Fh = y.F;
+                sy = y.s;
+            }
+            if (!(range_x < kFaceRange)) {
+                const March2F x = march2_wide<0, RIEMANN>(gas, sb, weps, GATED && (lin & 1), c4[0], c4[1], c4[2], c4[3], c4[4], c4[5]);
+                F = x.F;
+                sx = x.s;
+            }
+        }
+        if (cell_in && sy > smax) smax = sy;
+        if (!first) {
+            if (face_in && sx > smax) smax = sx;
             FX4[tid] = F;
         }
         __syncthreads();

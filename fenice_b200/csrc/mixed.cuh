@@ -47,10 +47,65 @@ __device__ __forceinline__ float min_nan(float a, float b) {
     return r;
 }
 
+// The Riemann solver of a face whose numbers leave the range in which riemann_f's products are finite: the formulas of the
+// plain form in FP32, the wave order decided by the comparisons of vmin / vmax. A solution that blows up comes here: its
+// energy flux is the difference of two overflowed terms, a NaN, which the wave-speed maxima skip. (riemann_f's one-sided
+// products would give an infinity, and the run would stop as diverged where the plain formulas carry on.) Out of line, so
+// that the faces that never come here pay for a comparison: states in, flux (mass, energy, momenta) and speed out.
+template <int NA> struct FaceF {
+    float s, m, e, v[NA];
+};
+template <int RIEMANN, int NA>
+__device__ __noinline__ FaceF<NA> riemann_wide(GasF g, float shock_blend, float rL, float pL, FaceF<NA> L, float rR, float pR, FaceF<NA> R) {
+    constexpr int NV = NA + 2;
+    const Eos<float> e{g.pi == 0.0f ? kIdeal : kStiffened, g.g, g.pi, 0.0f};
+    St<float, NV> WL, WR, F;
+    WL[0] = vmax(rL, Num<float>::eos_eps);
+    WL[3] = vmax(pL, Num<float>::eos_eps);
+    WR[0] = vmax(rR, Num<float>::eos_eps);
+    WR[3] = vmax(pR, Num<float>::eos_eps);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {   // the normal velocity in slot 1
+        const int q = a < 2 ? 1 + a : 4;
+        WL[q] = L.v[a];
+        WR[q] = R.v[a];
+    }
+    const float inv_L = 1.0f / WL[0], inv_R = 1.0f / WR[0];
+    const float c_L = sound_speed_inv(e, WL[3], inv_L), c_R = sound_speed_inv(e, WR[3], inv_R);
+    if constexpr (RIEMANN == kLowMach) {
+        float mL = 0.0f, mR = 0.0f;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            mL += L.v[a] * L.v[a];
+            mR += R.v[a] * R.v[a];
+        }
+        const float M_L = sqrtf(mL) / (c_L + Num<float>::mach_eps), M_R = sqrtf(mR) / (c_R + Num<float>::mach_eps);
+        const float z = vmin(vmax(vmax(M_L, M_R), 1e-4f), 1.0f);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int q = a < 2 ? 1 + a : 4;
+            const float avg = 0.5f * (L.v[a] + R.v[a]), half = 0.5f * (L.v[a] - R.v[a]);
+            WL[q] = avg + z * half;
+            WR[q] = avg - z * half;
+        }
+    }
+    FaceF<NA> o;
+    o.s = hllc_core(WL, WR, p2c(e, WL), p2c(e, WR), inv_L, inv_R, c_L, c_R, 0, shock_blend, F);
+    o.m = F[0];
+    o.e = F[3];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) o.v[a] = F[a < 2 ? 1 + a : 4];
+    return o;
+}
+// Below this, a face's largest speed times its energies, no product of riemann_f or of the plain formulas overflows. A NaN is not
+// below it.
+constexpr float kFaceRange = 1e35f;
+
 // HLLC / low-Mach HLLC of a face from its two primitive states (the Riemann solver of the mixed form): density, pressure
 // and the NA velocity components of each side, the normal one first, the others in cyclic order; every operation rounded
 // explicitly, so that each kernel that solves a face gets the same flux. Fm: the mass flux, Fe: the energy flux, Fv: the
-// momentum fluxes in the order of the velocities; returns max(|S_L|, |S_R|).
+// momentum fluxes in the order of the velocities; returns max(|S_L|, |S_R|). `range`: below kFaceRange no product overflowed (at
+// or above it, or a NaN, the face is riemann_wide's).
 //
 // The star flux is written from the side the contact leaves to the other: with S the wave speed of that side, q =
 // rho (S - u_n) and f = q / (S - S_M), the mass flux is f S_M, the momentum flux f S_M v (+ p* = p + q (S_M - u_n) along
@@ -60,7 +115,7 @@ __device__ __forceinline__ float min_nan(float a, float b) {
 // p* = p. The Mach number of the low-Mach scaling takes one reciprocal and one square root for both sides.
 template <int RIEMANN, int NA>
 __device__ __forceinline__ float riemann_f(const GasF& e, float shock_blend, float rL, float pL, float (&vL)[NA], float rR, float pR, float (&vR)[NA],
-                                           float& Fm, float& Fe, float (&Fv)[NA]) {
+                                           float& Fm, float& Fe, float (&Fv)[NA], float& range) {
     rL = max_nan(rL, Num<float>::eos_eps);
     pL = max_nan(pL, Num<float>::eos_eps);
     rR = max_nan(rR, Num<float>::eos_eps);
@@ -94,7 +149,6 @@ __device__ __forceinline__ float riemann_f(const GasF& e, float shock_blend, flo
     float SM = __fmul_rn(num, rcp_f(max_nan(__fsub_rn(qR, qL), Num<float>::denom_eps)));   // (qR >= 0 >= qL)
     const bool sup = SL >= 0.0f || SR < 0.0f;
     const bool left = SR >= 0.0f && (SL >= 0.0f || SM >= 0.0f);
-    const bool fail = !sup && !(SM >= 0.0f) && !(SM < 0.0f);   // a NaN speed: no flux
     const float rho = left ? rL : rR, p = left ? pL : pR, q = left ? qL : qR;
     float v[NA];   // the side's velocity
 #pragma unroll
@@ -105,12 +159,15 @@ __device__ __forceinline__ float riemann_f(const GasF& e, float shock_blend, flo
     const float rc = rcp_f(copysignf(max_nan(fabsf(w), Num<float>::denom_eps), w));
     float f = __fmul_rn(q, rc), ps = __fmaf_rn(q, d, p);
     float Es = __fmaf_rn(f, __fmaf_rn(d, SM, E), __fmul_rn(__fmul_rn(d, p), rc));
+    const float rE = __fmul_rn(rho, E);
     if (sup) {
         SM = v[0];
         f = rho;
         ps = p;
-        Es = __fmul_rn(rho, E);
+        Es = rE;
     }
+    const float s = max_nan(fabsf(SL), fabsf(SR));
+    range = __fmul_rn(s, __fadd_rn(fabsf(Es), rE));
     Fm = __fmul_rn(f, SM);
     Fv[0] = __fmaf_rn(Fm, SM, ps);
 #pragma unroll
@@ -121,6 +178,7 @@ __device__ __forceinline__ float riemann_f(const GasF& e, float shock_blend, flo
         // a strong pressure jump: the HLL flux blended in
         const float phi = min_nan(__fmul_rn(__fsub_rn(__fmul_rn(jump, rcp_f(pm)), shock_blend), rcp_f(shock_blend)), 1.0f);
         const float inv = rcp_f(__fsub_rn(SR, SL)), ss = __fmul_rn(SL, SR);
+        range = max_nan(range, __fmul_rn(range, s));
         const float mL = __fmul_rn(rL, uL), mR = __fmul_rn(rR, uR);
         const float EL = __fmaf_rn(__fmul_rn(0.5f, rL), square(vL), __fmul_rn(__fadd_rn(pL, e.gpi), e.g1));
         const float ER = __fmaf_rn(__fmul_rn(0.5f, rR), square(vR), __fmul_rn(__fadd_rn(pR, e.gpi), e.g1));
@@ -135,14 +193,34 @@ __device__ __forceinline__ float riemann_f(const GasF& e, float shock_blend, flo
                           __fmul_rn(rL, vL[a]), __fmul_rn(rR, vR[a]));
         Fe = blend(Fe, __fmul_rn(uL, __fadd_rn(EL, pL)), __fmul_rn(uR, __fadd_rn(ER, pR)), EL, ER);
     }
-    if (fail) {
-        Fm = Fe = 0.0f;
-#pragma unroll
-        for (int a = 0; a < NA; ++a) Fv[a] = 0.0f;
-    }
-    return max_nan(fabsf(SL), fabsf(SR));
+    return s;
 }
-// riemann_f of two primitive states in the state's order, along a compile-time axis
+// riemann_f, or riemann_wide beyond its range
+template <int RIEMANN, int NA>
+__device__ __forceinline__ float riemann_face(const GasF& e, float shock_blend, float rL, float pL, const float (&vL)[NA], float rR, float pR,
+                                              const float (&vR)[NA], float& Fm, float& Fe, float (&Fv)[NA]) {
+    float l[NA], r[NA], range;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        l[a] = vL[a];
+        r[a] = vR[a];
+    }
+    const float s = riemann_f<RIEMANN>(e, shock_blend, rL, pL, l, rR, pR, r, Fm, Fe, Fv, range);
+    if (range < kFaceRange) return s;
+    FaceF<NA> L, R;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        L.v[a] = vL[a];
+        R.v[a] = vR[a];
+    }
+    const FaceF<NA> o = riemann_wide<RIEMANN, NA>(e, shock_blend, rL, pL, L, rR, pR, R);
+    Fm = o.m;
+    Fe = o.e;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) Fv[a] = o.v[a];
+    return o.s;
+}
+// riemann_face of two primitive states in the state's order, along a compile-time axis
 template <int RIEMANN, int NV>
 __device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend, const St<float, NV>& WL, const St<float, NV>& WR, int axis,
                                                 St<float, NV>& F) {
@@ -154,7 +232,7 @@ __device__ __forceinline__ float face_flux_prim(const GasF& e, float shock_blend
         vL[a] = WL[m];
         vR[a] = WR[m];
     }
-    const float s = riemann_f<RIEMANN>(e, shock_blend, WL[0], WL[3], vL, WR[0], WR[3], vR, F[0], F[3], Fv);
+    const float s = riemann_face<RIEMANN>(e, shock_blend, WL[0], WL[3], vL, WR[0], WR[3], vR, F[0], F[3], Fv);
 #pragma unroll
     for (int a = 0; a < NA; ++a) {
         const int c = (axis + a) % NA, m = c == 0 ? 1 : (c == 1 ? 2 : 4);
@@ -422,8 +500,11 @@ template <int NV> __device__ __forceinline__ double cell_out(const StageArgs& a,
 // The mixed-precision stage kernel: the tile sweep of stage_kernel (same phases, same launch geometry) with FP32 stencil
 // arithmetic; see the file comment for what stays FP64.
 // FULL = false: a run without part interfaces or non-reflecting sides (their code compiled out of the hot loop)
+// CTAs per SM: what the registers of the sweep alone allow, kept with the call to riemann_wide in it (left to itself the
+// compiler then takes 67 registers where 56 do, and two CTAs per SM for three).
+template <int DIM, int RECON, bool FULL> constexpr int kMixedCTAs = DIM == 3 ? (RECON == kWeno5 && !FULL ? 3 : 2) : (FULL ? 3 : 4);
 template <int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool GATED = false, bool FULL = true>
-__global__ void __launch_bounds__(NT) mixed_stage_kernel(const StageArgs a) {
+__global__ void __launch_bounds__(NT, kMixedCTAs<DIM, RECON, FULL>) mixed_stage_kernel(const StageArgs a) {
     using S = MixedShape<DIM, RECON, TX, TY, TZ>;
     constexpr int NV = S::NV, NC = S::NC;
     extern __shared__ double smem_d[];
