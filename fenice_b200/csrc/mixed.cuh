@@ -249,8 +249,10 @@ template <int NV> __device__ __forceinline__ St<double, NV> prim_d(const Eos<dou
     const double rho = vmax(U[0], Num<double>::eos_eps);
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(rho));
-    y = __fma_rn(__fma_rn(-rho, y, 1.0), y, y);
-    y = __fma_rn(__fma_rn(-rho, y, 1.0), y, y);
+    // (the steps take an infinite density as a finite one, whose y is 0 too: inf 0 is a NaN. A NaN is in y already.)
+    const double r = __hiloint2double(min(__double2hiint(rho), 0x7fefffff), __double2loint(rho));
+    y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+    y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
     inv = y;
     const double u = __dmul_rn(U[1], inv), v = __dmul_rn(U[2], inv);
     double k = __fma_rn(v, v, __dmul_rn(u, u));

@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
 
 CELLS = {"nan_energy": [1, 0.2, 0.1, np.nan, 0.1], "nan_density": [np.nan, 0.1, 0.1, 2.5, 0.1], "nan_momentum": [1, np.nan, 0.1, 2.5, 0.1],
          "nan_transverse": [1, 0.1, np.nan, 2.5, 0.1], "inf_energy": [1, 0.1, 0.1, -np.inf, 0.1],
+         "inf_density": [np.inf, 0.2, 0.1, 2.5, 0.1],   # (its velocity is 0)
          "overflow": [-9.6e5, 1.1e12, 0, -2.5e18, 0]}   # (finite in FP64; its density is floored, so its velocity is 1e22)
 # (cells, values) non-finite after one step and t after five, for meshes of 1, 2 and 3 dimensions
 EXPECTED = {
@@ -23,12 +24,14 @@ EXPECTED = {
     ("HLLC", "nan_momentum"): [(1, 1, 2.3641e-2), (1, 1, 2.4036e-2), (1, 1, 2.7130e-2)],
     ("HLLC", "nan_transverse"): [(1, 1, 2.3641e-2), (1, 1, 2.4036e-2), (1, 1, 2.7130e-2)],
     ("HLLC", "inf_energy"): [(1, 1, 2.6913e-2), (1, 1, 2.6415e-2), (1, 1, 2.9171e-2)],
+    ("HLLC", "inf_density"): [(1, 1, 2.3641e-2), (1, 1, 2.4036e-2), (1, 1, 2.7130e-2)],
     ("HLLC", "overflow"): [(3, 12, 2.4207e-2), (8, 22, 2.4056e-2), (13, 35, 2.6322e-2)],
     ("HLLC (Low-Mach Thornber)", "nan_energy"): [(1, 1, 2.3965e-2), (1, 1, 2.4744e-2), (1, 1, 2.7930e-2)],
     ("HLLC (Low-Mach Thornber)", "nan_density"): [(1, 1, 2.4699e-2), (1, 1, 2.4769e-2), (1, 1, 2.7930e-2)],
     ("HLLC (Low-Mach Thornber)", "nan_momentum"): [(1, 1, 2.4699e-2), (1, 1, 2.4769e-2), (1, 1, 2.7930e-2)],
     ("HLLC (Low-Mach Thornber)", "nan_transverse"): [(1, 1, 2.3986e-2), (1, 1, 2.4769e-2), (1, 1, 2.7909e-2)],
     ("HLLC (Low-Mach Thornber)", "inf_energy"): [(1, 1, 2.7106e-2), (1, 1, 2.6726e-2), (1, 1, 2.9391e-2)],
+    ("HLLC (Low-Mach Thornber)", "inf_density"): [(1, 1, 2.4027e-2), (1, 1, 2.4769e-2), (1, 1, 2.7828e-2)],
     ("HLLC (Low-Mach Thornber)", "overflow"): [(3, 12, 2.5555e-2), (7, 24, 2.4573e-2), (11, 43, 2.7266e-2)],
 }
 
