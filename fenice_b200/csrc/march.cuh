@@ -645,7 +645,7 @@ template <int RIEMANN, bool GATED> struct March2K {
 };
 
 // ---------------------------------------------------------------------------------------------- viscous fluxes
-// The mixed-precision viscous sweep of a launch whose every side wraps or is a part interface (no wall rules), marching
+// The mixed-precision viscous sweep of a mesh whose every side is periodic (parts of it included: no wall rules), marching
 // along z like the stage kernel: 32 x 8 columns per CTA, three planes of the columns and one cell around them in shared
 // memory (u, v, w, T in one float4, rho beside it). Per plane a thread forms the nine velocity-gradient entries of its cell
 // once (the tiled sweep formed four of them for each of three axes, on a tile extended along the axis) and shares them with

@@ -83,8 +83,10 @@ MixedStage mixed_stage_gated(int dim, int riemann, bool full) {
     return full ? pick_gated<2, true>(riemann) : pick_gated<2, false>(riemann);
 }
 
-// the FP32 viscous sweep: the marching kernel where every side of the launch wraps or is a part interface and no body is
-// immersed, else 8x8x8 tiles of 384 threads
+// the FP32 viscous sweep: the marching kernel where every side of the whole mesh is periodic and no body is immersed, else
+// 8x8x8 tiles of 384 threads. (By the configuration's sides, which the parts of a decomposed mesh share: the two sweeps round
+// their gradients differently, and both parts beside an interface must give its faces the same flux. An inner part of a mesh
+// with walls has none itself.)
 constexpr int kMixedViscNT = 384;
 cudaError_t mixed_viscous_prepare() {
     cudaError_t e = cudaFuncSetAttribute(mixed_viscous_kernel<8, 8, 8, kMixedViscNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -95,9 +97,7 @@ cudaError_t mixed_viscous_prepare() {
 }
 bool mixed_stage_marches(const StageArgs& a, int dim) { return can_march(a, dim); }
 cudaError_t mixed_viscous_launch(const ViscArgs& a, int nblocks, cudaStream_t s) {
-    bool march = !a.bc.slot;
-    for (int side = 0; side < 6; ++side) march = march && a.through[side];
-    if (march) return visc_march_launch(a, nblocks, s);
+    if (a.all_periodic && !a.bc.slot) return visc_march_launch(a, nblocks, s);
     mixed_viscous_kernel<8, 8, 8, kMixedViscNT><<<nblocks, kMixedViscNT, MixedViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);
     return cudaGetLastError();
 }

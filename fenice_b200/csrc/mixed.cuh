@@ -562,7 +562,7 @@ __device__ __forceinline__ float f4c(float4 v, int a) { return a == 0 ? v.x : (a
 // periodic sides and part interfaces around it) reads its box without the ghost rules and solves its faces without the
 // wall tests; a tile wholly inside the mesh skips the test for faces beyond it. The four values a position, a face or a
 // cell carries sit together in one float4 (one shared-memory access each); each axis's balance shares a phase with the
-// next axis's gradients (six barriers per tile). Launches without walls, inlets, outlets or an immersed body march instead
+// next axis's gradients (six barriers per tile). Meshes whose every side is periodic, without an immersed body, march instead
 // (march.cuh).
 template <int TX, int TY, int TZ, int NT>
 __global__ void __launch_bounds__(NT, 4) mixed_viscous_kernel(const ViscArgs a) {

@@ -937,6 +937,8 @@ ViscArgs visc_args(fvg_run* r, const double* Uin, double* bmv, const int* gate) 
         a.periodic[d] = r->cfg.bc[2 * d] == FVG_BC_PERIODIC && r->cfg.bc[2 * d + 1] == FVG_BC_PERIODIC && !(split && (r->peer[0] || r->peer[1]));
         for (int h = 0; h < 2; ++h) a.through[2 * d + h] = a.periodic[d] || r->bc.halo[2 * d + h] == kHaloPeer;
     }
+    a.all_periodic = true;
+    for (int side = 0; side < 6; ++side) a.all_periodic = a.all_periodic && r->cfg.bc[side] == FVG_BC_PERIODIC;
     a.U = Uin;
     a.Rv = r->Rv;
     a.Rvf = r->cfg.precision == FVG_PREC_MIXED && r->dim == 3 ? reinterpret_cast<float*>(r->Rv) : nullptr;

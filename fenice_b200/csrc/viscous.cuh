@@ -29,6 +29,7 @@ struct ViscArgs {
     int bface2;        // boundary_order == 2
     int periodic[3];   // both sides of the axis periodic
     int through[6];    // the side is periodic or a part interface (kHaloPeer): no wall rules at its faces
+    bool all_periodic; // every side of the whole mesh is periodic
     int nvar;          // state planes: 4 on a 2-D mesh (rho w is +0 there), 5 in 3-D
     const double* U;
     double* Rv;

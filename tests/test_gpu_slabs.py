@@ -38,6 +38,10 @@ SLAB_CASES = [
     # the whole run's mixed WENO5-Z kernel stages its interior tiles by TMA; the parts' kernels load every tile by index mapping
     ("mixed_w5_rk3_visc_64_tma", dict(nx=64, ny=64, nz=64, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3",
                                       use_viscous=True, mu=0.01, **TGV), 72, 4, (1, 2), 1),
+    # walls on the split axis: the end parts' viscous sweeps have wall rules, the inner ones' only interfaces
+    ("mixed_w5_rk3_visc_walls_z_3d", dict(nx=36, ny=20, nz=27, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3",
+                                          use_viscous=True, mu=0.01, Lx=1.0, Ly=1.0, Lz=1.0,
+                                          **B("periodic", "periodic", "periodic", "periodic", z=("no_slip", "wall"))), 73, 4, (2, 3, 4), 1),
     # non-reflecting outlets: on x, whose tangential z neighbours cross the part interfaces, and at the low z end
     ("nrbc_w5_rk3_visc_3d", dict(nx=12, ny=10, nz=13, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", use_viscous=True, mu=0.01,
                                  **B("transmissive", "nonreflecting", "periodic", "periodic", z=("nonreflecting", "wall"))), 71, 3, (2, 3), 0),
