@@ -3,7 +3,8 @@ caller owns U). The pipelined form uploads the state in slabs along the slowest 
 slabs that have arrived, and reads the last stage back slab by slab; it must give the bits of upload + fvg_step +
 download (which the parity tests pin to the reference) on every kind of run: 3-D and 2-D, periodic and bounded axes,
 slabs that do not line up with the stage tiles, viscous and inviscid, Euler / SSP-RK2 / SSP-RK3, FP64 and mixed
-precision, the learned sensor's gate, and the runs that take the unpipelined route (an immersed body)."""
+precision, the learned sensor's gate, and the runs that take the unpipelined route (an immersed body). A mesh goes up in
+one slab unless it has stage tiles for two rounds of the SMs in each of several: SPLIT_CASES are large enough for that."""
 import math
 
 import numpy as np
@@ -32,10 +33,9 @@ def tgv(nx, ny, nz):
 
 CYLP = dict(nx=64, ny=96, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", cfl=0.4, **cases.CYL)
 CASES = [
-    # 64 z planes: 8 slabs of one tile plane each, the first uploaded last-slab-first (periodic z)
+    # meshes of one slab
     ("tgv3d_fp64_rk3_viscous", dict(nx=24, ny=16, nz=64, **TGV), lambda: tgv(24, 16, 64), 3, 0),
     ("tgv3d_mixed_rk3_viscous", dict(nx=24, ny=16, nz=64, **TGV), lambda: tgv(24, 16, 64), 3, 1),
-    # 2-D, bounded y: 200 rows in 16 slabs of 13, stage tiles 15 rows high (tile planes straddle slabs)
     ("riemann2d_fp64_weno5_rk3", dict(nx=40, ny=200, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", cfl=0.4,
                                       **cases.bcs("transmissive", "transmissive", "transmissive", "transmissive")),
      lambda: cases.smooth_field(40, 200, seed=11, jump=True), 3, 0),
@@ -48,6 +48,45 @@ CASES = [
     # a run the overlap does not cover: the three calls in turn
     ("cylinder_ibm_rk3", CYLP, lambda: cases.ibm_field(CYLP, (1.4, 2.0, 0.0, 1.0), 42), 2, 0),
 ]
+SPLIT_CASES = [
+    # periodic z, 10 tile planes in 3 slabs (the last one short): uploaded last slab first
+    ("split_tgv3d_fp64_rk3_viscous", dict(nx=128, ny=112, nz=80, **TGV), lambda: tgv(128, 112, 80), 2, 0),
+    ("split_tgv3d_mixed_rk3_viscous", dict(nx=128, ny=112, nz=77, **TGV), lambda: tgv(128, 112, 77), 2, 1),
+    # bounded z, the mixed viscous sweep in tiles; then FP64 with one stage
+    ("split_walls3d_mixed_visc_rk3", dict(nx=120, ny=100, nz=90, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", cfl=0.3, use_viscous=True, mu=2e-3,
+                                          **cases.bcs("periodic", "periodic", "transmissive", "wall", z=("no_slip", "wall"))),
+     lambda: cases.smooth_field(120, 100, 90, seed=4), 2, 1),
+    ("split_box3d_weno3_euler_walls", dict(nx=160, ny=96, nz=61, reconstruction="weno3", time_scheme="Euler", cfl=0.3,
+                                           **cases.bcs("wall", "wall", "transmissive", "transmissive", z=("wall", "transmissive"))),
+     lambda: cases.smooth_field(160, 96, 61, seed=2), 2, 0),
+    # 2-D: 41 rows of stage tiles in 6 slabs, the mixed kernels marching over each; viscous tiles (16 rows) that straddle the
+    # slabs of 15-row stage tiles
+    ("split_riemann2d_fp64_weno5_rk3", dict(nx=1600, ny=610, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", cfl=0.4,
+                                            **cases.bcs("transmissive", "transmissive", "transmissive", "transmissive")),
+     lambda: cases.smooth_field(1600, 610, seed=11, jump=True), 2, 0),
+    ("split_periodic2d_mixed_weno5_rk3", dict(nx=1600, ny=610, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", cfl=0.4,
+                                              **cases.bcs("transmissive", "wall", "periodic", "periodic")),
+     lambda: cases.smooth_field(1600, 610, seed=12), 2, 1),
+    ("split_walls2d_visc_muscl_rk2", dict(nx=1200, ny=500, reconstruction="muscl", muscl_limiter="MC", time_scheme="SSP Runge-Kutta 2", use_viscous=True,
+                                          mu=2e-3, **cases.bcs("wall", "outlet", "no_slip", "vel_inlet"), u_in=0.2),
+     lambda: cases.smooth_field(1200, 500, seed=5), 2, 0),
+    ("split_periodic2d_visc_weno5_rk3", dict(nx=1200, ny=500, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", use_viscous=True, mu=2e-3,
+                                             **cases.bcs("periodic", "periodic", "periodic", "periodic")),
+     lambda: cases.smooth_field(1200, 500, seed=6), 2, 0),
+]
+
+
+def slab_count(params):
+    """The slabs a mesh goes up in: each holds stage tiles (8x8x8, 16x15) for two rounds of two CTAs on 148 SMs, at most 16."""
+    three = params.get("nz", 1) > 1
+    tile = 8 if three else 15
+    n = params["nz"] if three else params["ny"]
+    per = -(-params["nx"] // 8) * -(-params["ny"] // 8) if three else -(-params["nx"] // 16)
+    layers = -(-n // tile)
+    slabs = max(1, layers // -(-592 // per))
+    planes = -(-n // 16)
+    planes = max(8, -(-planes // 8) * 8 if three else planes, -(-layers // slabs) * tile)
+    return -(-n // planes)
 
 
 def reference_steps(params, U0, n, precision):
@@ -63,8 +102,9 @@ def reference_steps(params, U0, n, precision):
     return U, dts
 
 
-@pytest.mark.parametrize("name,params,init,n,precision", CASES, ids=[c[0] for c in CASES])
+@pytest.mark.parametrize("name,params,init,n,precision", CASES + SPLIT_CASES, ids=[c[0] for c in CASES + SPLIT_CASES])
 def test_step_host_equals_upload_step_download(name, params, init, n, precision):
+    assert (slab_count(params) > 1) == name.startswith("split")
     U0 = init()
     want, want_dt = reference_steps(params, U0, n, precision)
     run = Run(params, U=U0, precision=precision, device=0)
@@ -103,13 +143,14 @@ def test_step_host_against_the_oracle():
     run.close()
 
 
-def test_step_host_with_the_sensor_matches_the_graph_run():
+@pytest.mark.parametrize("nx,ny,nz", [(24, 16, 64), (128, 112, 80)])   # one slab, three
+def test_step_host_with_the_sensor_matches_the_graph_run(nx, ny, nz):
     """The gate refreshed every `every` calls, as the graph-launched run refreshes it every `every` steps."""
     pytest.importorskip("torch")
     from fenice_b200.sensor import Sensor
 
-    params = dict(nx=24, ny=16, nz=64, **TGV)
-    U0 = tgv(24, 16, 64)
+    params = dict(nx=nx, ny=ny, nz=nz, **TGV)
+    U0 = tgv(nx, ny, nz)
     s = Sensor(seed=3)
     graph = Run(params, U=U0, precision=1, device=0)
     graph.set_sensor(s, 0.0, every=3)
