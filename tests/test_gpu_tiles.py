@@ -3,13 +3,17 @@ columns, and remainders along every axis.
 
 The marching mixed kernels (32 x 8 columns in 3-D, 128 columns with 127 cells of their own in 2-D; the stage state formed as
 it is read) against the same run in parts, whose tiled kernels solve every face and update every cell with the same explicitly
-rounded operations: the same bits. The FP64 kernels (8x8x8 tiles, 16 x 15 and 16 x 5 tiles, 14 x 14 MUSCL-Hancock tiles) against
+rounded operations: the same bits; gated by the sensor, against the same run with an immersed body outside the mesh, which the tiled
+kernels serve (a face inside a CTA is solved once: only such a comparison shows which values it took). The FP64 kernels (8x8x8 tiles, 16 x 15 and 16 x 5 tiles, 14 x 14 MUSCL-Hancock tiles) against
 the restatement of the reference: the same bits. The batched rows (63, 127 and 255 cells) against single runs: the same bits."""
+import os
+
 import numpy as np
 import pytest
 
 import cases
 from fenice_b200 import Batch, Run, slabs
+from fenice_b200.sensor import Sensor
 from oracle.oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -44,6 +48,45 @@ def test_marching_2d(nx, ny, sides):
     assert run.run(1e30, max_steps=4) == 4
     U, steps, t = slabs.run_decomposed(params, U0, 2, 1e30, max_steps=4, precision=1)
     assert steps == 4 and t == run.t and same_bits(run.state(), U)
+
+
+GATED = [(33, 9, 13), (70, 17, 20), (64, 24, 31), (128, 31, 1), (127, 46, 1), (260, 46, 1), (33, 100, 1)]
+
+
+@pytest.mark.parametrize("sides", ["periodic", "walls"])
+@pytest.mark.parametrize("nx,ny,nz", GATED + [(256, 128, 40)])   # (the last: 20 planes a CTA, several rows of tiles)
+def test_gated_marching(nx, ny, nz, sides):
+    p = dict(nx=nx, ny=ny, reconstruction="weno5", riemann_solver="lowmach" if nz > 1 else "HLLC", time_scheme="SSP Runge-Kutta 3", cfl=0.4)
+    if nz > 1:
+        p.update(nz=nz, Lz=1.0)
+    p.update(PER if sides == "periodic" else WALLS3 if nz > 1 else B("transmissive", "wall", "wall", "transmissive"))
+    if nz == 1:
+        p = {k: v for k, v in p.items() if not k.startswith("bc_z")}
+    # smooth flow with a block of other gas in it, off the middle, so that linear and WENO5-Z tiles meet on every axis
+    z, y, x = np.meshgrid(*[(np.arange(n) + 0.5) / n for n in (nz, ny, nx)], indexing="ij")
+    W = np.zeros((x.size, 5))
+    wave = np.sin(2 * np.pi * x) * np.cos(2 * np.pi * y)
+    W[:, 0] = (1.0 + 0.02 * wave).ravel()
+    W[:, 1] = (0.3 + 0.02 * np.cos(2 * np.pi * y)).ravel()
+    W[:, 2] = (-0.2 + 0.02 * np.sin(2 * np.pi * x)).ravel()
+    W[:, 3] = (1.0 + 0.02 * wave).ravel()
+    if nz > 1:
+        W[:, 4] = (0.1 + 0.02 * np.sin(2 * np.pi * z)).ravel()
+    block = ((x > 0.1) & (x < 0.25) & (y > 0.55) & (y < 0.8) & ((z > 0.6) if nz > 1 else True)).ravel()
+    W[block, 0] *= 1.7
+    W[block, 3] *= 1.4
+    U0 = cases.prim_to_cons(W)
+    sensor = Sensor.load(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fenice_b200", "sensor_weights.npz"))
+    got = []
+    for body in ({}, dict(use_ibm=True, ibm_shape="Sphere" if nz > 1 else "Cylinder", ibm_radius=0.1, ibm_cx=-9.0, ibm_cy=-9.0)):
+        run = Run(dict(p, **body), U=U0, precision=1)
+        run.set_sensor(sensor, float(sensor.meta["threshold"]), every=2, radius=1)
+        assert run.run(1e30, max_steps=5) == 5
+        linear, evaluated = run.sensor_counts()
+        got.append((run.state(), run.t, linear, evaluated))
+    (a, ta, la, ea), (b, tb, lb, eb) = got
+    assert 0 < la < ea and (la, ea, ta) == (lb, eb, tb)
+    assert same_bits(a, b), f"{int((a != b).sum())} values differ"
 
 
 FP64 = [
