@@ -507,7 +507,7 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct StageK {
     static constexpr bool kLoop = DIM == 3 && (RECON == kWeno3 || RECON == kWeno5) && !FULL;
     static cudaError_t prepare() {
         if constexpr (kLoop)
-            return cudaFuncSetAttribute(stage3_kernel<RECON, RIEMANN, 512, FULL, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            return cudaFuncSetAttribute(stage3_kernel<RECON, RIEMANN, 512, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)Stage3Shape<RECON>::SMEM_BYTES);
         else
             return cudaFuncSetAttribute(stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -517,7 +517,7 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct StageK {
         if constexpr (DIM == 2 && RECON != kFirstOrder && !FULL)
             if (!a.bc.solid) return launch2d(a, nblocks, s);
         if constexpr (kLoop)
-            stage3_kernel<RECON, RIEMANN, 512, FULL, 2><<<nblocks, 512, Stage3Shape<RECON>::SMEM_BYTES, s>>>(a);
+            stage3_kernel<RECON, RIEMANN, 512, 2><<<nblocks, 512, Stage3Shape<RECON>::SMEM_BYTES, s>>>(a);
         else
             stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL><<<nblocks, Tl::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();

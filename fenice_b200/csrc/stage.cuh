@@ -451,14 +451,16 @@ __global__ void __launch_bounds__(NT, MB) stage2d_kernel(const StageArgs a, cons
 // (32 warps; 64 registers, some spilled) beat fewer warps with more registers. ms per launch at 128^3, WENO5-Z, low-Mach HLLC /
 // HLLC: the sweep with 256 threads 1.51 / 1.44, with 320 1.31 / 1.24; this loop with 256 1.52, 320 1.29 / 1.25, 384 1.30 / 1.21, 512
 // 1.24 / 1.16 (kept); a pair of lanes per face, one for each side, 1.37 / 1.32. MUSCL, whose faces have no WENO divisions, is no
-// faster in it (0.56 against 0.55): it keeps the sweep.
+// faster in it (0.56 against 0.55): it keeps the sweep. Runs without the features of FULL only (an immersed body's solid cells
+// are among what it serves).
 template <int RECON> struct Stage3Shape {
-    static constexpr int NV = 5, H = RECON == kWeno5 ? 3 : (RECON == kFirstOrder ? 1 : 2);
+    static_assert(RECON == kWeno3 || RECON == kWeno5, "the loop over the axes");
+    static constexpr int NV = 5, H = RECON == kWeno5 ? 3 : 2;
     static constexpr int ROW = 65, NS = 8 + 2 * H, EXT = NS * ROW, NF = 9 * 64, NC = 512;
     static constexpr int FLAG_BYTES = (EXT + 7) / 8 * 8;
     static constexpr size_t SMEM_BYTES = sizeof(double) * (NV * EXT + 2 * NV * NF + NV * NC + 32) + FLAG_BYTES;
 };
-template <int RECON, int RIEMANN, int NT, bool FULL, int MB>
+template <int RECON, int RIEMANN, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB) stage3_kernel(const StageArgs a) {
     using S = Stage3Shape<RECON>;
     constexpr int NV = 5, H = S::H, NC = S::NC, NF = S::NF, EXT = S::EXT, ROW = S::ROW;
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(NT, MB) stage3_kernel(const StageArgs a) {
             j = o3[1] + (axis == 1 ? s : (axis == 0 ? u : v));
             k = o3[2] + (axis == 2 ? s : v);
         };
-        // ---- 1. load (primitive; first order keeps the conservative state), x fastest
+        // ---- 1. load, x fastest
         for (int e = tid; e < S::NS * 64; e += NT) {
             int s, u, v, i, j, k;
             if (axis == 0) {
@@ -497,52 +499,40 @@ __global__ void __launch_bounds__(NT, MB) stage3_kernel(const StageArgs a) {
             }
             const int slot = s * ROW + v * 8 + u;
             place(s - H, u, v, i, j, k);
-            const St<double, NV> c = stencil_cons<3, NV, FULL>(m, a.bc, a.eos, a.U, i, j, k);
+            const St<double, NV> c = stencil_cons<3, NV, false>(m, a.bc, a.eos, a.U, i, j, k);
             if constexpr (RECON == kWeno5)
                 if (a.bc.solid) Sf[slot] = stencil_solid<3>(m, a.bc, i, j, k);
-            if constexpr (RECON == kFirstOrder) {
+            const St<double, NV> w = c2p(a.eos, c);
 #pragma unroll
-                for (int q = 0; q < NV; ++q) P[q * EXT + slot] = c[q];
-            } else {
-                const St<double, NV> w = c2p(a.eos, c);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) P[q * EXT + slot] = w[q];
-            }
+            for (int q = 0; q < NV; ++q) P[q * EXT + slot] = w[q];
         }
         __syncthreads();
         // ---- 2. face values: face t = f / 64 has its stencil at the rows t .. t + 2H - 1
-        if constexpr (RECON != kFirstOrder) {
-            for (int it = tid; it < NF * NV; it += NT) {
-                const int q = it / NF, f = it - q * NF, slot = (f >> 6) * ROW + (f & 63);
-                const double* c = P + q * EXT + slot;
-                double wl, wr;
-                if constexpr (RECON == kMuscl) {
-                    const double c0 = c[0], c1 = c[ROW], c2 = c[2 * ROW], c3 = c[3 * ROW];
-                    const double bb = c2 - c1;
-                    wl = c1 + 0.5 * limiter(a.limiter, c1 - c0, bb);
-                    wr = c2 - 0.5 * limiter(a.limiter, c3 - c2, bb);
-                } else if constexpr (RECON == kWeno3) {
-                    wl = weno3z(c[0], c[ROW], c[2 * ROW], a.weno_eps);
-                    wr = weno3z(c[3 * ROW], c[2 * ROW], c[ROW], a.weno_eps);
-                } else {
-                    const double c0 = c[0], c1 = c[ROW], c2 = c[2 * ROW], c3 = c[3 * ROW], c4 = c[4 * ROW], c5 = c[5 * ROW];
-                    bool four = false;   // a solid cell among the six: the four-cell WENO3-Z stencil (weno_line_states, Schemes.cpp:815-831)
-                    if (a.bc.solid)
+        for (int it = tid; it < NF * NV; it += NT) {
+            const int q = it / NF, f = it - q * NF, slot = (f >> 6) * ROW + (f & 63);
+            const double* c = P + q * EXT + slot;
+            double wl, wr;
+            if constexpr (RECON == kWeno3) {
+                wl = weno3z(c[0], c[ROW], c[2 * ROW], a.weno_eps);
+                wr = weno3z(c[3 * ROW], c[2 * ROW], c[ROW], a.weno_eps);
+            } else {
+                const double c0 = c[0], c1 = c[ROW], c2 = c[2 * ROW], c3 = c[3 * ROW], c4 = c[4 * ROW], c5 = c[5 * ROW];
+                bool four = false;   // a solid cell among the six: the four-cell WENO3-Z stencil (weno_line_states, Schemes.cpp:815-831)
+                if (a.bc.solid)
 #pragma unroll
-                        for (int s6 = 0; s6 < 6; ++s6) four = four || Sf[slot + s6 * ROW] != 0;
-                    if (four) {
-                        wl = weno3z(c1, c2, c3, a.weno_eps);
-                        wr = weno3z(c4, c3, c2, a.weno_eps);
-                    } else {
-                        wl = weno5z(c0, c1, c2, c3, c4, a.weno_eps);
-                        wr = weno5z(c5, c4, c3, c2, c1, a.weno_eps);
-                    }
+                    for (int s6 = 0; s6 < 6; ++s6) four = four || Sf[slot + s6 * ROW] != 0;
+                if (four) {
+                    wl = weno3z(c1, c2, c3, a.weno_eps);
+                    wr = weno3z(c4, c3, c2, a.weno_eps);
+                } else {
+                    wl = weno5z(c0, c1, c2, c3, c4, a.weno_eps);
+                    wr = weno5z(c5, c4, c3, c2, c1, a.weno_eps);
                 }
-                WL[q * NF + f] = wl;
-                WR[q * NF + f] = wr;
             }
-            __syncthreads();
+            WL[q * NF + f] = wl;
+            WR[q * NF + f] = wr;
         }
+        __syncthreads();
         // ---- 3. fluxes, written over the face values: slot f of WL is read and written by the thread of face f only
         const int na = axis == 0 ? m.nx : (axis == 1 ? m.ny : m.nz);
         const int lo_side = 2 * axis, hi_side = 2 * axis + 1;
@@ -560,35 +550,19 @@ __global__ void __launch_bounds__(NT, MB) stage3_kernel(const StageArgs a) {
                 St<double, NV> UL, UR;
                 if (lo_face || hi_face) {
                     const int d = hi_face ? 1 : 0;
-                    side_states<NV, FULL>(m, a.bc, a.eos, a.U, lo_face ? lo_side : hi_side, i - (axis == 0 ? d : 0), j - (axis == 1 ? d : 0),
+                    side_states<NV, false>(m, a.bc, a.eos, a.U, lo_face ? lo_side : hi_side, i - (axis == 0 ? d : 0), j - (axis == 1 ? d : 0),
                                           k - (axis == 2 ? d : 0), UL, UR);
-                    if constexpr (RECON != kFirstOrder) {
-                        UL = round_trip(a.eos, UL);
-                        UR = round_trip(a.eos, UR);
-                    }
-                } else if constexpr (RECON == kFirstOrder) {
-                    const int slot = (f >> 6) * ROW + (f & 63);   // the cell before the face, and the next row's after it
+                    UL = round_trip(a.eos, UL);
+                    UR = round_trip(a.eos, UR);
+                } else {
+                    St<double, NV> wl, wr;
 #pragma unroll
                     for (int q = 0; q < NV; ++q) {
-                        UL[q] = P[q * EXT + slot];
-                        UR[q] = P[q * EXT + slot + ROW];
+                        wl[q] = WL[q * NF + f];
+                        wr[q] = WR[q * NF + f];
                     }
-                } else {
-                    const int li = i - (axis == 0), lj = j - (axis == 1), lk = k - (axis == 2);
-                    if (FULL && a.fb && (fb_flagged<3>(m, a.bc, a.fb, li, lj, lk) || fb_flagged<3>(m, a.bc, a.fb, i, j, k))) {
-                        // next to a flagged cell: the two cells' states (the ghost of a side's halo beyond it)
-                        UL = stencil_cons<3, NV>(m, a.bc, a.eos, a.U, li, lj, lk);
-                        UR = stencil_cons<3, NV>(m, a.bc, a.eos, a.U, i, j, k);
-                    } else {
-                        St<double, NV> wl, wr;
-#pragma unroll
-                        for (int q = 0; q < NV; ++q) {
-                            wl[q] = WL[q * NF + f];
-                            wr[q] = WR[q * NF + f];
-                        }
-                        UL = p2c(a.eos, wl);
-                        UR = p2c(a.eos, wr);
-                    }
+                    UL = p2c(a.eos, wl);
+                    UR = p2c(a.eos, wr);
                 }
                 const double s = face_flux<RIEMANN>(a.eos, a.shock_blend, UL, UR, axis, F);
                 if (s > smax) smax = s;
@@ -621,12 +595,6 @@ __global__ void __launch_bounds__(NT, MB) stage3_kernel(const StageArgs a) {
         for (int q = 0; q < NV; ++q) {
             r[q] = acc[q * NC + c] * m.inv_cell;
             if (a.Rv) r[q] = r[q] + a.Rv[q * m.plane + cell];
-        }
-        // the body force, then the case's source terms, join after the viscous term (Simulation::assemble,
-        // cpp/src/Simulation.cpp:1038-1049; RhsSourceTerms in the order Simulation::setup adds them, :372-412)
-        if constexpr (FULL) {
-            if (a.bc.grav_on) add_body_force<NV>(a.bc, read_state<NV>(a.bc, a.U, m.plane, cell), r);
-            if (a.bc.src) add_source<NV>(a.bc, m.plane, cell, r);
         }
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
