@@ -81,7 +81,12 @@ __device__ __forceinline__ void after_launch_before() {
 // Launches of a step that are shorter than a launch's set-up is long: the next launch's CTAs are set up while the last ones
 // of the launch before still run. 131 x 97 vortex, SSP-RK2: 22.9 -> 22.0 us per step. Launches that fill the SMs keep the plain
 // form: CTAs that wait beside running ones cost the marching kernels 4 to 6 %.
-constexpr int kEarlyTiles = 148 * 2;   // of 16 x 15 cells: half the places of the one-pass 2-D kernel
+//
+// The line lies where the 16 x 5 tiles of the one-pass 2-D kernel (three for each of 16 x 15) no longer have a place each on the
+// SMs (three CTAs per SM). us per step, 16 x 15 tiles with plain launches / 16 x 5 with early ones, MUSCL SSP-RK2 and WENO5-Z
+// SSP-RK3: 72 tiles 24.8 / 18.6 and 57.6 / 39.0, 144 tiles 26.0 / 21.7 and 58.8 / 49.0, 150 tiles 27.5 / 27.9 and 64.6 / 66.2, 288 tiles
+// 28.9 / 34.0 and 67.8 / 82.6, 1120 tiles 82.0 / 102.8 and 227 / 263.
+constexpr int kEarlyTiles = 148;   // of 16 x 15 cells
 template <class... P, class... A>
 cudaError_t launch_early(void (*kern)(P...), unsigned ctas, unsigned threads, size_t smem, cudaStream_t s, const A&... args) {
     cudaLaunchAttribute at;

@@ -522,11 +522,11 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct StageK {
             stage_kernel<DIM, RECON, RIEMANN, Tl::X, Tl::Y, Tl::Z, Tl::NT, FULL><<<nblocks, Tl::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
-    // the one-pass kernel, over the rows of the launch's tiles. A launch whose tiles do not fill half the SMs' places takes
-    // tiles a third as high (where its CTAs need not be its tiles: the speeds folded into the control block).
+    // the one-pass kernel, over the rows of the launch's tiles. A launch of at most a tile per SM takes tiles a third as high
+    // (where its CTAs need not be its tiles: the speeds folded into the control block).
     static cudaError_t launch2d(const StageArgs& a, int nblocks, cudaStream_t s) {
         const int row0 = a.b0 / a.tiles[0] * Tl::Y, row_end = (a.b0 + nblocks) / a.tiles[0] * Tl::Y, row1 = row_end < a.m.ny ? row_end : a.m.ny;
-        if (a.fin.kind != kFinNone && nblocks < kEarlyTiles) {
+        if (a.fin.kind != kFinNone && nblocks <= kEarlyTiles) {
             constexpr int TY = 5, NT = 192;
             StageArgs b = a;
             b.fin.ctas = a.tiles[0] * ((row1 - row0 + TY - 1) / TY);
@@ -1289,7 +1289,7 @@ cudaError_t enqueue_step(fvg_run* r, bool refresh = true) {
         return cudaGetLastError();
     }
     const bool formed = forms_stage_state(r);
-    if (!formed && r->dim == 2 && r->nb < kEarlyTiles)
+    if (!formed && r->dim == 2 && r->nb <= kEarlyTiles)
         e = launch_early(k_axpy, axpy_blocks(r), 256, 0, r->stream, c, r->Ut, r->U, r->R, r->m.plane, r->m.ncells, r->nvar);
     else if (!formed)
         k_axpy<<<axpy_blocks(r), 256, 0, r->stream>>>(c, r->Ut, r->U, r->R, r->m.plane, r->m.ncells, r->nvar);

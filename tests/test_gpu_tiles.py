@@ -94,10 +94,11 @@ FP64 = [
     *[(dict(nx=n, ny=m, reconstruction="muscl", muscl_limiter=lim, time_scheme="MUSCL-Hancock", **s), 5)
       for n, m, lim, s in [(13, 14, "Minmod", PER), (14, 15, "Van Leer", PER), (15, 29, "MC", B("vel_inlet", "transmissive", "wall", "outlet")),
                            (43, 13, "Koren", B("wall", "transmissive", "periodic", "periodic"))]],
-    # 16 x 5 tiles, and 16 x 15 ones where the mesh has tiles enough (320 x 241: 340)
+    # 16 x 5 tiles up to 148 of 16 x 15 (222 x 149: 140), and those beyond (240 x 150: 150, 320 x 241: 340)
     *[(dict(nx=n, ny=m, reconstruction=r, time_scheme=ts, cfl=0.4, **s), 4)
       for n, m, r, ts, s in [(15, 4, "muscl", "SSP Runge-Kutta 2", PER), (16, 5, "weno5", "SSP Runge-Kutta 3", B("wall", "transmissive", "outlet", "wall")),
-                             (17, 6, "weno3", "SSP Runge-Kutta 3", PER), (320, 241, "weno5", "SSP Runge-Kutta 3", PER)]],
+                             (17, 6, "weno3", "SSP Runge-Kutta 3", PER), (222, 149, "weno5", "SSP Runge-Kutta 3", B("wall", "transmissive", "outlet", "wall")),
+                             (240, 150, "muscl", "SSP Runge-Kutta 2", PER), (320, 241, "weno5", "SSP Runge-Kutta 3", PER)]],
     # 8x8x8 tiles, the viscous box without and with wall rules; other gases (the quotient by gamma - 1)
     *[(dict(nx=7, ny=8, nz=9, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3", use_viscous=True, mu=0.01, gamma=g, **s), 3)
       for g, s in [(1.4, PER), (5.0 / 3.0, PER), (1.1, B("no_slip", "wall", "periodic", "periodic", z=("moving_wall", "no_slip")))]],
