@@ -102,7 +102,7 @@ __device__ __forceinline__ int march_cell(const Bc& bc, int axis, int g, int n, 
     return hi ? n - 1 : 0;
 }
 
-// z0 .. z1: the planes of the launch; lz: planes per CTA (a multiple of 8 where the CTAs write blockmax). GATED: a face is
+// z0 .. z1: the planes of the launch; lz: planes per CTA (march_launch). GATED: a face is
 // linear when the tiles of both its cells are linear along its axis (inside a tile: when the tile is), which is the seam
 // rule of mixed_axis face by face.
 template <int RIEMANN, bool GATED, int MB = 2>
@@ -593,53 +593,83 @@ inline bool can_march(const StageArgs& a, int dim) {
     for (int s = 0; s < 2 * dim; ++s) ok = ok && (a.bc.halo[s] == kHaloWrap || a.bc.halo[s] == kHaloSlab);
     return ok;
 }
-// The planes a CTA marches over, for `cols` column blocks and nz planes: the count that gives the fewest rounds of the
-// `resident` CTAs of 148 SMs times the planes of a round (3 more each for filling the column). 256^3: 32 planes, 7 rounds.
-inline int march_planes(int cols, int nz, int step, int resident) {
-    const int round = 148 * resident;
-    int best = step;
-    long long least = 0;
-    for (int lz = step; lz < nz + step; lz += step) {
-        const long long ctas = (long long)cols * ((nz + lz - 1) / lz), cost = (ctas + round - 1) / round * (lz + 3);
-        if (lz == step || cost < least) {
-            best = lz;
-            least = cost;
-        }
+// The planes a CTA marches over and the launch's time: a round with c CTAs to an SM takes fill + lz (base + per c) us, `resident`
+// the most that fit. Fitted to stage launches (FP32 issue grows with c, the chain of a plane does not), where it is within 10 %:
+// 3-D 32^3 .. 192^3, 2-D 64^2 .. 1500^2. A plane count that is a multiple of 4 throughout, for the rounds times (lz + 3) alone, took
+// 425 us a step at 80^3 (viscous; 333 now), 124 at 32^3 (62) and 45.6 at 128^2 (31.3).
+struct MarchCost {
+    int resident;
+    double fill, base, per;
+};
+constexpr MarchCost kMarch3Cost = {2, 13.0, 2.4, 3.0}, kMarch2Cost = {5, 8.0, 0.9, 0.77};
+struct MarchPlan {
+    int lz;
+    double us;
+};
+inline MarchPlan march_plan(const MarchCost& t, int resident, long long cols, int nz, int step) {
+    MarchPlan best = {step, 0.0};
+    const long long round = 148 * resident;
+    for (int lz = step; lz < nz + step; lz += lz < 32 ? step : (step > 4 ? step : 4)) {
+        const long long ctas = cols * ((nz + lz - 1) / lz), rem = ctas % round;
+        double us = (double)(ctas / round) * (t.fill + lz * (t.base + t.per * resident));
+        if (rem) us += t.fill + lz * (t.base + t.per * (double)((rem + 147) / 148));
+        if (lz == step || us < best.us) best = {lz, us};
     }
     return best;
+}
+// The part of the mesh a launch of `nblocks` tiles from a.b0 (whole layers of 8x8x8 ones, whole rows of 16 x 15 ones) marches
+// over, and how. A launch that writes one maximum per tile has at most as many CTAs as tiles: planes in whole tiles.
+struct MarchLaunch {
+    int z0, z1, cols;
+    MarchPlan plan;
+    int ctas() const { return cols * ((z1 - z0 + plan.lz - 1) / plan.lz); }
+};
+constexpr int kMarch2W = 128;
+inline MarchLaunch march_launch(const StageArgs& a, int dim, int nblocks) {
+    const int T = dim == 3 ? 8 : 15, layer = dim == 3 ? a.tiles[0] * a.tiles[1] : a.tiles[0], n = dim == 3 ? a.m.nz : a.m.ny;
+    const int end = (a.b0 + nblocks) / layer * T;
+    MarchLaunch l;
+    l.z0 = a.b0 / layer * T;
+    l.z1 = end < n ? end : n;
+    l.cols = dim == 3 ? ((a.m.nx + MarchShape::W - 1) / MarchShape::W) * ((a.m.ny + MarchShape::H - 1) / MarchShape::H) : (a.m.nx + kMarch2W - 2) / (kMarch2W - 1);
+    const MarchCost& t = dim == 3 ? kMarch3Cost : kMarch2Cost;
+    l.plan = march_plan(t, t.resident, l.cols, l.z1 - l.z0, a.fin.kind == kFinNone ? T : 1);
+    return l;
+}
+// Whether a launch marches: where it can, and the tiles (three CTAs to an SM in 3-D, four in 2-D; there with the pass for U + dt R
+// that marching spares) would take longer. Same bits either way. Meshes that leave most of their column blocks idle take the tiles:
+// 72^3 without viscosity 209 us a step against 244 marching, 128 x 2048 87 against 113, 128 x 900 53 against 70; and 256^2 39 against 44, a
+// round of whose tiles is short. Marching: 96^3 343 against 468, 64^3 136 against 176, 400^2 62 against 66, 2048 x 128 72 against 87.
+inline bool marches(const StageArgs& a, int dim, int nblocks) {
+    if (a.Rd) return true;   // (only for a launch this chose)
+    if (!can_march(a, dim)) return false;
+    const int resident = dim == 3 ? 3 : 4, round = 148 * resident, rem = nblocks % round;
+    double us = dim == 3 ? 0.0 : 1.0;
+    us += (nblocks / round) * (dim == 3 ? 35.0 : 12.0);
+    if (rem) us += (dim == 3 ? 19.0 : 8.0) + (dim == 3 ? 7.5 : 1.9) * ((rem + 147) / 148);
+    return march_launch(a, dim, nblocks).plan.us < us;
 }
 template <int RIEMANN, bool GATED> struct MarchK {
     static cudaError_t prepare() {
         return cudaFuncSetAttribute(mixed_march_kernel<RIEMANN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MarchShape::SMEM_BYTES);
     }
-    // `nblocks` 8x8x8 tiles from a.b0, whole layers of tiles
     static cudaError_t launch(const StageArgs& a0, int nblocks, cudaStream_t s) {
         StageArgs a = a0;
-        const int layer = a.tiles[0] * a.tiles[1];
-        const int z0 = a.b0 / layer * 8, z_end = (a.b0 + nblocks) / layer * 8, z1 = z_end < a.m.nz ? z_end : a.m.nz;
-        const int cols = ((a.m.nx + MarchShape::W - 1) / MarchShape::W) * ((a.m.ny + MarchShape::H - 1) / MarchShape::H);
-        const int lz = march_planes(cols, z1 - z0, a.fin.kind == kFinNone ? 8 : 4, 2);
-        const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
-        a.fin.ctas = ctas;
-        mixed_march_kernel<RIEMANN, GATED><<<ctas, MarchShape::NT, MarchShape::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
+        const MarchLaunch l = march_launch(a, 3, nblocks);
+        a.fin.ctas = l.ctas();
+        mixed_march_kernel<RIEMANN, GATED><<<l.ctas(), MarchShape::NT, MarchShape::SMEM_BYTES, s>>>(a, l.z0, l.z1, l.plan.lz, nblocks);
         return cudaGetLastError();
     }
 };
-
-// `nblocks` 16x15 tiles from a.b0, whole rows of tiles
-constexpr int kMarch2W = 128, kMarch2CTAs = 5;
 template <int RIEMANN, bool GATED> struct March2K {
     using S = March2Shape<kMarch2W>;
-    static constexpr auto kern = mixed_march2_kernel<RIEMANN, GATED, kMarch2W, kMarch2CTAs>;
+    static constexpr auto kern = mixed_march2_kernel<RIEMANN, GATED, kMarch2W, kMarch2Cost.resident>;
     static cudaError_t prepare() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES); }
     static cudaError_t launch(const StageArgs& a0, int nblocks, cudaStream_t s) {
         StageArgs a = a0;
-        const int z0 = a.b0 / a.tiles[0] * 15, z_end = (a.b0 + nblocks) / a.tiles[0] * 15, z1 = z_end < a.m.ny ? z_end : a.m.ny;
-        const int cols = (a.m.nx + S::W - 2) / (S::W - 1);
-        const int lz = march_planes(cols, z1 - z0, a.fin.kind == kFinNone ? 15 : 4, kMarch2CTAs);
-        const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
-        a.fin.ctas = ctas;
-        kern<<<ctas, S::NT, S::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
+        const MarchLaunch l = march_launch(a, 2, nblocks);
+        a.fin.ctas = l.ctas();
+        kern<<<l.ctas(), S::NT, S::SMEM_BYTES, s>>>(a, l.z0, l.z1, l.plan.lz, nblocks);
         return cudaGetLastError();
     }
 };
@@ -886,7 +916,7 @@ inline cudaError_t visc_march_launch(const ViscArgs& a0, int nblocks, cudaStream
     const int layer = a.tiles[0] * a.tiles[1];
     const int z0 = a.b0 / layer * 8, z_end = (a.b0 + nblocks) / layer * 8, z1 = z_end < a.m.nz ? z_end : a.m.nz;
     const int cols = ((a.m.nx + ViscMarchShape::W - 1) / ViscMarchShape::W) * ((a.m.ny + ViscMarchShape::H - 1) / ViscMarchShape::H);
-    const int lz = march_planes(cols, z1 - z0, a.fin.kind == kFinNone ? 8 : 4, 3);
+    const int lz = march_plan(kMarch3Cost, 3, cols, z1 - z0, a.fin.kind == kFinNone ? 8 : 1).lz;
     const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
     mixed_viscous_march_kernel<<<ctas, ViscMarchShape::NT, ViscMarchShape::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
     return cudaGetLastError();

@@ -13,7 +13,7 @@ template <int DIM> struct MTile;
 template <> struct MTile<3> { static constexpr int X = 8, Y = 8, Z = 8, NT = 384; };
 template <> struct MTile<2> { static constexpr int X = 16, Y = 15, Z = 1, NT = 256; };
 
-// the marching kernels (march.cuh): the WENO5-Z lean kernels, where can_march
+// the marching kernels (march.cuh): the WENO5-Z lean kernels, where marches
 template <int DIM, int RECON, bool FULL> constexpr bool kHasMarch = RECON == kWeno5 && !FULL;
 template <int DIM, int RIEMANN, bool GATED> using MarchOf = std::conditional_t<DIM == 3, MarchK<RIEMANN, GATED>, March2K<RIEMANN, GATED>>;
 
@@ -29,7 +29,7 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct MixedK {
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
         if constexpr (kHasMarch<DIM, RECON, FULL>)
-            if (can_march(a, DIM)) return MarchOf<DIM, RIEMANN, false>::launch(a, nblocks, s);
+            if (marches(a, DIM, nblocks)) return MarchOf<DIM, RIEMANN, false>::launch(a, nblocks, s);
         mixed_stage_kernel<DIM, RECON, RIEMANN, T::X, T::Y, T::Z, T::NT, false, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
@@ -48,7 +48,7 @@ template <int DIM, int RIEMANN, bool FULL> struct GatedK {
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
         if constexpr (kHasMarch<DIM, kWeno5, FULL>)
-            if (can_march(a, DIM)) return MarchOf<DIM, RIEMANN, true>::launch(a, nblocks, s);
+            if (marches(a, DIM, nblocks)) return MarchOf<DIM, RIEMANN, true>::launch(a, nblocks, s);
         mixed_stage_kernel<DIM, kWeno5, RIEMANN, T::X, T::Y, T::Z, T::NT, true, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
@@ -95,7 +95,7 @@ cudaError_t mixed_viscous_prepare() {
         e = cudaFuncSetAttribute(mixed_viscous_march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscMarchShape::SMEM_BYTES);
     return e;
 }
-bool mixed_stage_marches(const StageArgs& a, int dim) { return can_march(a, dim); }
+bool mixed_stage_marches(const StageArgs& a, int dim, int nblocks) { return marches(a, dim, nblocks); }
 cudaError_t mixed_viscous_launch(const ViscArgs& a, int nblocks, cudaStream_t s) {
     if (a.all_periodic && !a.bc.slot) return visc_march_launch(a, nblocks, s);
     mixed_viscous_kernel<8, 8, 8, kMixedViscNT><<<nblocks, kMixedViscNT, MixedViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);

@@ -18,8 +18,9 @@ MixedStage mixed_stage(int dim, int recon, int riemann, bool full);
 // the mixed WENO5-Z stage kernel with the learned troubled-cell sensor choosing linear or WENO5-Z reconstructions
 // (StageArgs::sens_flags)
 MixedStage mixed_stage_gated(int dim, int riemann, bool full);
-// whether a launch of their lean WENO5-Z kernels with these arguments marches (march.cuh); the 2-D one then takes StageArgs::Rd
-bool mixed_stage_marches(const StageArgs& a, int dim);
+// whether a launch of their lean WENO5-Z kernels with these arguments (fin among them) over `nblocks` tiles marches (march.cuh);
+// the 2-D one then takes StageArgs::Rd
+bool mixed_stage_marches(const StageArgs& a, int dim, int nblocks);
 cudaError_t mixed_viscous_prepare();
 cudaError_t mixed_viscous_launch(const ViscArgs& a, int nblocks, cudaStream_t s);
 }   // namespace fvg

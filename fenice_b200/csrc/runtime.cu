@@ -1238,7 +1238,9 @@ bool forms_stage_state(fvg_run* r) {
     if (r->dim != 2 || c.time_scheme != FVG_TS_SSPRK3 || c.precision != FVG_PREC_MIXED || c.reconstruction != FVG_RECON_WENO5 || c.use_viscous ||
         r->full || r->ibm || r->d_utarget || r->fourth)
         return false;
-    return mixed_stage_marches(stage_args(r, r->U, nullptr, r->Ut, kCombine, 0, 0, nullptr, nullptr, nullptr), r->dim);
+    StageArgs a = stage_args(r, r->U, nullptr, r->Ut, kCombine, 0, 0, nullptr, nullptr, nullptr);
+    a.fin = Fin{r->ctl, kFinMax, r->nb};
+    return mixed_stage_marches(a, r->dim, r->nb);
 }
 
 // The launches of one time step on the run's stream (no host synchronisation). refresh = false leaves out the sensor's

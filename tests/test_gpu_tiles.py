@@ -27,9 +27,28 @@ def same_bits(a, b):
     return np.array_equal(np.ascontiguousarray(a).view(np.uint64), np.ascontiguousarray(b).view(np.uint64))
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(31, 7, 8), (32, 8, 9), (33, 9, 16), (70, 17, 13)])
+def march_planes(nx, ny, nz=1):
+    """The planes a CTA of the marching kernels owns on a whole mesh; 0 where the mesh takes the tiles."""
+    three = nz > 1
+    n, cols = (nz, -(-nx // 32) * -(-ny // 8)) if three else (ny, -(-nx // 127))
+    tiles = -(-nx // 8) * -(-ny // 8) * -(-nz // 8) if three else -(-nx // 16) * -(-ny // 15)
+    fill, base, per, resident = (13.0, 2.4, 3.0, 2) if three else (8.0, 0.9, 0.77, 5)
+
+    def us(lz):
+        full, rest = divmod(cols * -(-n // lz), 148 * resident)
+        return full * (fill + lz * (base + per * resident)) + (fill + lz * (base + per * -(-rest // 148)) if rest else 0.0)
+
+    lz = min([k for k in range(1, n + 1) if k < 32 or k % 4 == 0], key=us)
+    full, rest = divmod(tiles, 148 * (3 if three else 4))
+    tiled = (0.0 if three else 1.0) + full * (35.0 if three else 12.0) + ((19.0 + 7.5 * -(-rest // 148) if three else 8.0 + 1.9 * -(-rest // 148)) if rest else 0.0)
+    return lz if us(lz) < tiled else 0
+
+
+# (the last one of each list: several planes or rows to a CTA)
+@pytest.mark.parametrize("nx,ny,nz", [(31, 7, 8), (32, 8, 9), (33, 9, 16), (70, 17, 13), (161, 83, 37)])
 @pytest.mark.parametrize("sides", ["periodic_viscous", "walls"])
 def test_marching_3d(nx, ny, nz, sides):
+    assert march_planes(nx, ny, nz) == (10 if nx == 161 else 1)
     params = dict(nx=nx, ny=ny, nz=nz, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3", cfl=0.4)
     params.update(dict(PER, use_viscous=True, mu=0.01) if sides == "periodic_viscous" else WALLS3)
     U0 = cases.case_field(params, nx + ny)
@@ -39,9 +58,10 @@ def test_marching_3d(nx, ny, nz, sides):
     assert steps == 3 and t == run.t and same_bits(run.state(), U)
 
 
-@pytest.mark.parametrize("nx,ny", [(126, 15), (127, 16), (128, 31), (260, 46)])
+@pytest.mark.parametrize("nx,ny", [(126, 15), (127, 16), (128, 31), (260, 46), (1300, 203)])
 @pytest.mark.parametrize("sides", [PER, B("transmissive", "wall", "wall", "transmissive")], ids=["periodic", "walls"])
 def test_marching_2d(nx, ny, sides):
+    assert march_planes(nx, ny) == (4 if nx == 1300 else 1)
     params = dict(nx=nx, ny=ny, reconstruction="weno5", time_scheme="SSP Runge-Kutta 3", cfl=0.4, **sides)
     U0 = cases.case_field(params, 3 * (nx // 3))   # (a seed whose field has a jump: the HLL blend)
     run = Run(params, U=U0, precision=1)
@@ -50,12 +70,15 @@ def test_marching_2d(nx, ny, sides):
     assert steps == 4 and t == run.t and same_bits(run.state(), U)
 
 
-GATED = [(33, 9, 13), (70, 17, 20), (64, 24, 31), (128, 31, 1), (127, 46, 1), (260, 46, 1), (33, 100, 1)]
+# (planes or rows a CTA owns: 1, then 10, 20, 4 and 6, several rows of tiles)
+GATED = {(33, 9, 13): 1, (70, 17, 20): 1, (64, 24, 31): 1, (128, 31, 1): 1, (127, 46, 1): 1, (260, 46, 1): 1, (33, 100, 1): 1, (161, 83, 37): 10, (256, 128, 40): 20,
+         (1300, 203, 1): 4, (700, 700, 1): 6}
 
 
 @pytest.mark.parametrize("sides", ["periodic", "walls"])
-@pytest.mark.parametrize("nx,ny,nz", GATED + [(256, 128, 40)])   # (the last: 20 planes a CTA, several rows of tiles)
+@pytest.mark.parametrize("nx,ny,nz", list(GATED))
 def test_gated_marching(nx, ny, nz, sides):
+    assert march_planes(nx, ny, nz) == GATED[nx, ny, nz]
     p = dict(nx=nx, ny=ny, reconstruction="weno5", riemann_solver="lowmach" if nz > 1 else "HLLC", time_scheme="SSP Runge-Kutta 3", cfl=0.4)
     if nz > 1:
         p.update(nz=nz, Lz=1.0)
