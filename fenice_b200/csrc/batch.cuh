@@ -6,7 +6,7 @@
 // scheme, precision) and differ in mesh, lengths, boundary conditions, gas and initial state. Their states live in three
 // pools (the state U, the stage state Ut, the residual / stage buffer R), problem p's NV planes at offset off_p of each
 // pool. A work list of (problem, tile) items covers the tiles of the problems still running; a stage launch has a fixed
-// grid (a whole number of CTAs per SM) whose CTAs take the items in turn, so the launch shape and the CUDA graph of a
+// grid (a whole number of CTAs per SM) whose CTAs take runs of consecutive items, so the launch shape and the CUDA graph of a
 // step never change while problems finish and drop out of the list. Each problem reduces its stage wave speeds with
 // atomicMax on the bits of a non-negative double (their integer order is their value order), so the maxima and every
 // dt are the bits the problem gets when it runs alone.

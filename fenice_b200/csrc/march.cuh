@@ -5,8 +5,8 @@
 // - the primitive state of a cell is recovered once as its plane arrives and once more where the cell lies beside another
 //   CTA's columns (1.9 recoveries per cell; an 8x8x8 tile with its three halos takes 3.25);
 // - a thread keeps the six planes of its column around its z face in registers; the plane being solved lies in shared
-//   memory with three cells around the columns, for the x and y faces (rows of 40 floats: a warp reads 32 neighbours of
-//   one row, no two on a bank);
+//   memory with three cells around the columns, for the x and y faces (rows of 40 float4 and 40 floats: a warp
+//   reads 32 neighbours of one row, no two words on a bank);
 // - per plane a thread solves its low x, its low y and its high z face; the 40 faces on the high sides of the columns fall
 //   to two of the warps in turn;
 // - four of the five variables lie in one float4, so a stencil cell is two loads and its pairs (rho, p) and (u, v) are

@@ -7,7 +7,7 @@
 // single-precision division and square root, and contraction into FMAs): the WENO-Z / MUSCL reconstruction of the
 // primitives, the Riemann solver, the flux balance, the viscous stresses and heat flux. The linear and WENO5-Z face values,
 // the balance and the FP64 update round every operation explicitly instead, so that every kernel that solves a face or
-// updates a cell (the per-axis sweep, the cross form, the batched kernels) gives it the same bits.
+// updates a cell (the per-axis sweep, the marching kernels, the batched kernels) gives it the same bits.
 //
 // One algorithmic difference from the plain form: the Riemann solver takes the reconstructed primitive states directly
 // (their density and pressure floored as cons_to_prim floors them) instead of converting them to conservative form and

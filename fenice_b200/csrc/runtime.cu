@@ -6,16 +6,19 @@
 // graph and replayed.
 //
 // Step sequences (the reference's TimeScheme::step, cpp/src/TimeScheme.cpp:110-319):
-//   Euler:    [viscous] stage(U -> R) ; dt ; U = U + dt R ; end
-//   SSP-RK2:  [viscous] stage(U -> R) ; dt ; Ut = U + dt R ; [viscous] stage(Ut, U0 = U -> U: 1/2 U0 + 1/2 (Ut + dt R)) ; end
-//   SSP-RK3:  [viscous] stage(U -> R) ; dt ; Ut = U + dt R ; [viscous] stage(Ut, U0 = U -> R: 3/4 U0 + 1/4 (Ut + dt R)) ;
-//             [viscous] stage(R, U0 = U -> U: 1/3 U0 + 2/3 (R + dt R3)) ; end
-//   MUSCL-Hancock: seed (first step only: one plain residual for the wave speed) ; dt from the lagged speed ;
-//             hancock(U -> Ut = U + dt R) ; end (the speed of this step is the next step's) ; the state then lives in Ut
-//             (ping-pong, tracked by the host).
-// "dt" reduces the CTA maxima of stage 1 into s1 and sets dt = cfl L / (s1 + 1e-10), clamped to t_end - t and dt_max;
-// "end" reduces the later stages, applies check_progress, advances t and the step count and decides whether the next
-// step runs (t < t_end, step limit, no error).
+//   Euler:    [viscous] stage(U -> R), dt ; U = U + dt R ; end
+//   SSP-RK2:  [viscous] stage(U -> R), dt ; Ut = U + dt R ; [viscous] stage(Ut, U0 = U -> U: 1/2 U0 + 1/2 (Ut + dt R)), end
+//   SSP-RK3:  [viscous] stage(U -> R), dt ; Ut = U + dt R ; [viscous] stage(Ut, U0 = U -> R: 3/4 U0 + 1/4 (Ut + dt R)) ;
+//             [viscous] stage(R, U0 = U -> U: 1/3 U0 + 2/3 (R + dt R3)), end
+//             (a 2-D marching run, forms_stage_state: stage(U + dt R, U0 = U -> Ut) without the pass before it, stage 3 reads Ut)
+//   MUSCL-Hancock: at the start of a call (hancock_start) the seed, one plain residual for the wave speed if there is none yet, and
+//             dt from the lagged speed ; then per step hancock(U -> Ut = U + dt R), end and the next dt (the speed of this step is
+//             the next step's) ; the state then lives in Ut (ping-pong, tracked by the host).
+// "dt" sets dt = cfl L / (s1 + 1e-10) from the largest speed of stage 1, clamped to t_end - t and dt_max; "end" takes the largest
+// of the later stages, applies check_progress, advances t and the step count and decides whether the next step runs (t <
+// t_end, step limit, no error). After a comma they are the work of the launch's last CTA (stage_finish, grid.cuh); behind an
+// immersed body's reset, and in the launch sequences that keep per-CTA maxima (parts, the fourth-order passes, fvg_step_host,
+// fvg_residual), kernels of their own.
 #include "../../include/fenice_gpu.h"
 #include "expr.cuh"
 #include "fourth.cuh"

@@ -35,8 +35,8 @@ SLAB_CASES = [
      69, 4, (1, 2, 3), 0),
     ("mixed_w5_rk3_visc_3d", dict(nx=20, ny=16, nz=18, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3",
                                   use_viscous=True, mu=0.01, **TGV), 70, 4, (2, 3), 1),
-    # the whole run's mixed WENO5-Z kernel stages its interior tiles by TMA; the parts' kernels load every tile by index mapping
-    ("mixed_w5_rk3_visc_64_tma", dict(nx=64, ny=64, nz=64, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3",
+    # the whole run's mixed WENO5-Z kernel marches, several planes to a CTA; the parts' kernels sweep tiles
+    ("mixed_w5_rk3_visc_64_march", dict(nx=64, ny=64, nz=64, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3",
                                       use_viscous=True, mu=0.01, **TGV), 72, 4, (1, 2), 1),
     # walls on the split axis: the end parts' viscous sweeps have wall rules, the inner ones' only interfaces
     ("mixed_w5_rk3_visc_walls_z_3d", dict(nx=36, ny=20, nz=27, reconstruction="weno5", riemann_solver="lowmach", time_scheme="SSP Runge-Kutta 3",
