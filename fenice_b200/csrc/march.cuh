@@ -606,25 +606,27 @@ struct MarchPlan {
     int lz;
     double us;
 };
-inline MarchPlan march_plan(const MarchCost& t, int resident, long long cols, int nz, int step) {
-    MarchPlan best = {step, 0.0};
+inline MarchPlan march_plan(const MarchCost& t, int resident, long long cols, int nz, long long most) {
+    MarchPlan best = {0, 0.0};
     const long long round = 148 * resident;
-    for (int lz = step; lz < nz + step; lz += lz < 32 ? step : (step > 4 ? step : 4)) {
+    for (int lz = 1; lz < nz + 4; lz += lz < 32 ? 1 : 4) {
         const long long ctas = cols * ((nz + lz - 1) / lz), rem = ctas % round;
+        if (ctas > most) continue;
         double us = (double)(ctas / round) * (t.fill + lz * (t.base + t.per * resident));
         if (rem) us += t.fill + lz * (t.base + t.per * (double)((rem + 147) / 148));
-        if (lz == step || us < best.us) best = {lz, us};
+        if (!best.lz || us < best.us) best = {lz, us};
     }
     return best;
 }
 // The part of the mesh a launch of `nblocks` tiles from a.b0 (whole layers of 8x8x8 ones, whole rows of 16 x 15 ones) marches
-// over, and how. A launch that writes one maximum per tile has at most as many CTAs as tiles: planes in whole tiles.
+// over, and how. A launch that writes its CTAs' maxima has at most as many CTAs as tiles (the array's entries).
 struct MarchLaunch {
     int z0, z1, cols;
     MarchPlan plan;
     int ctas() const { return cols * ((z1 - z0 + plan.lz - 1) / plan.lz); }
 };
 constexpr int kMarch2W = 128;
+inline long long march_most(const Fin& f, int nblocks) { return f.kind == kFinNone ? nblocks : 1ll << 40; }
 inline MarchLaunch march_launch(const StageArgs& a, int dim, int nblocks) {
     const int T = dim == 3 ? 8 : 15, layer = dim == 3 ? a.tiles[0] * a.tiles[1] : a.tiles[0], n = dim == 3 ? a.m.nz : a.m.ny;
     const int end = (a.b0 + nblocks) / layer * T;
@@ -633,7 +635,7 @@ inline MarchLaunch march_launch(const StageArgs& a, int dim, int nblocks) {
     l.z1 = end < n ? end : n;
     l.cols = dim == 3 ? ((a.m.nx + MarchShape::W - 1) / MarchShape::W) * ((a.m.ny + MarchShape::H - 1) / MarchShape::H) : (a.m.nx + kMarch2W - 2) / (kMarch2W - 1);
     const MarchCost& t = dim == 3 ? kMarch3Cost : kMarch2Cost;
-    l.plan = march_plan(t, t.resident, l.cols, l.z1 - l.z0, a.fin.kind == kFinNone ? T : 1);
+    l.plan = march_plan(t, t.resident, l.cols, l.z1 - l.z0, march_most(a.fin, nblocks));
     return l;
 }
 // Whether a launch marches: where it can, and the tiles (three CTAs to an SM in 3-D, four in 2-D; there with the pass for U + dt R
@@ -916,7 +918,7 @@ inline cudaError_t visc_march_launch(const ViscArgs& a0, int nblocks, cudaStream
     const int layer = a.tiles[0] * a.tiles[1];
     const int z0 = a.b0 / layer * 8, z_end = (a.b0 + nblocks) / layer * 8, z1 = z_end < a.m.nz ? z_end : a.m.nz;
     const int cols = ((a.m.nx + ViscMarchShape::W - 1) / ViscMarchShape::W) * ((a.m.ny + ViscMarchShape::H - 1) / ViscMarchShape::H);
-    const int lz = march_plan(kMarch3Cost, 3, cols, z1 - z0, a.fin.kind == kFinNone ? 8 : 1).lz;
+    const int lz = march_plan(kMarch3Cost, 3, cols, z1 - z0, march_most(a.fin, nblocks)).lz;
     const int ctas = cols * ((z1 - z0 + lz - 1) / lz);
     mixed_viscous_march_kernel<<<ctas, ViscMarchShape::NT, ViscMarchShape::SMEM_BYTES, s>>>(a, z0, z1, lz, nblocks);
     return cudaGetLastError();

@@ -502,9 +502,10 @@ template <int NV> __device__ __forceinline__ double cell_out(const StageArgs& a,
 // The mixed-precision stage kernel: the tile sweep of stage_kernel (same phases, same launch geometry) with FP32 stencil
 // arithmetic; see the file comment for what stays FP64.
 // FULL = false: a run without part interfaces or non-reflecting sides (their code compiled out of the hot loop)
-// CTAs per SM: what the registers of the sweep alone allow, kept with the call to riemann_wide in it (left to itself the
-// compiler then takes 67 registers where 56 do, and two CTAs per SM for three).
-template <int DIM, int RECON, bool FULL> constexpr int kMixedCTAs = DIM == 3 ? (RECON == kWeno5 && !FULL ? 3 : 2) : (FULL ? 3 : 4);
+// CTAs per SM, which the compiler left to itself misses by a few registers (it weighs neither the packed face values nor the
+// call to riemann_wide). us per step at 128^3, two / three CTAs: WENO3-Z 877 / 748, low-Mach 900 / 767, MUSCL 833 / 701, low-Mach 854 / 721
+// (before the packed operands, with 56 registers, low-Mach 816 and 766); 2-D MUSCL at 1024^2, four / five: 233 / 218.
+template <int DIM, int RECON, bool FULL> constexpr int kMixedCTAs = DIM == 3 ? (FULL ? 2 : 3) : (FULL ? 3 : (RECON == kMuscl ? 5 : 4));
 template <int DIM, int RECON, int RIEMANN, int TX, int TY, int TZ, int NT, bool GATED = false, bool FULL = true>
 __global__ void __launch_bounds__(NT, kMixedCTAs<DIM, RECON, FULL>) mixed_stage_kernel(const StageArgs a) {
     using S = MixedShape<DIM, RECON, TX, TY, TZ>;
