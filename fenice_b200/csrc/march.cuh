@@ -606,14 +606,16 @@ struct MarchPlan {
     int lz;
     double us;
 };
-inline MarchPlan march_plan(const MarchCost& t, int resident, long long cols, int nz, long long most) {
+inline MarchPlan march_plan(const MarchCost& t, int resident, int cols, int nz, int most) {
     MarchPlan best = {0, 0.0};
-    const long long round = 148 * resident;
-    for (int lz = 1; lz < nz + 4; lz += lz < 32 ? 1 : 4) {
-        const long long ctas = cols * ((nz + lz - 1) / lz), rem = ctas % round;
-        if (ctas > most) continue;
-        double us = (double)(ctas / round) * (t.fill + lz * (t.base + t.per * resident));
-        if (rem) us += t.fill + lz * (t.base + t.per * (double)((rem + 147) / 148));
+    const unsigned round = 148u * resident;
+    // for each count of parts along the march the fewest planes that give it (a captured launch does this once, others each time)
+    for (int lz = 1, parts; lz <= nz; lz = parts > 1 ? (nz + parts - 2) / (parts - 1) : nz + 1) {
+        parts = (nz + lz - 1) / lz;
+        if (parts > most / cols) continue;
+        const unsigned ctas = (unsigned)cols * parts, full = ctas / round, rem = ctas - full * round;
+        double us = full * (t.fill + lz * (t.base + t.per * resident));
+        if (rem) us += t.fill + lz * (t.base + t.per * ((rem + 147u) / 148u));
         if (!best.lz || us < best.us) best = {lz, us};
     }
     return best;
@@ -626,7 +628,7 @@ struct MarchLaunch {
     int ctas() const { return cols * ((z1 - z0 + plan.lz - 1) / plan.lz); }
 };
 constexpr int kMarch2W = 128;
-inline long long march_most(const Fin& f, int nblocks) { return f.kind == kFinNone ? nblocks : 1ll << 40; }
+inline int march_most(const Fin& f, int nblocks) { return f.kind == kFinNone ? nblocks : 0x7fffffff; }
 inline MarchLaunch march_launch(const StageArgs& a, int dim, int nblocks) {
     const int T = dim == 3 ? 8 : 15, layer = dim == 3 ? a.tiles[0] * a.tiles[1] : a.tiles[0], n = dim == 3 ? a.m.nz : a.m.ny;
     const int end = (a.b0 + nblocks) / layer * T;
@@ -642,22 +644,22 @@ inline MarchLaunch march_launch(const StageArgs& a, int dim, int nblocks) {
 // that marching spares) would take longer. Same bits either way. Meshes that leave most of their column blocks idle take the tiles:
 // 72^3 without viscosity 209 us a step against 244 marching, 128 x 2048 87 against 113, 128 x 900 53 against 70; and 256^2 39 against 44, a
 // round of whose tiles is short. Marching: 96^3 343 against 468, 64^3 136 against 176, 400^2 62 against 66, 2048 x 128 72 against 87.
-inline bool marches(const StageArgs& a, int dim, int nblocks) {
-    if (a.Rd) return true;   // (only for a launch this chose)
+inline bool marches(const StageArgs& a, int dim, int nblocks, MarchLaunch& l) {
     if (!can_march(a, dim)) return false;
+    l = march_launch(a, dim, nblocks);
+    if (a.Rd) return true;   // (only for a launch this chose)
     const int resident = dim == 3 ? 3 : 4, round = 148 * resident, rem = nblocks % round;
     double us = dim == 3 ? 0.0 : 1.0;
     us += (nblocks / round) * (dim == 3 ? 35.0 : 12.0);
     if (rem) us += (dim == 3 ? 19.0 : 8.0) + (dim == 3 ? 7.5 : 1.9) * ((rem + 147) / 148);
-    return march_launch(a, dim, nblocks).plan.us < us;
+    return l.plan.us < us;
 }
 template <int RIEMANN, bool GATED> struct MarchK {
     static cudaError_t prepare() {
         return cudaFuncSetAttribute(mixed_march_kernel<RIEMANN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MarchShape::SMEM_BYTES);
     }
-    static cudaError_t launch(const StageArgs& a0, int nblocks, cudaStream_t s) {
+    static cudaError_t launch(const StageArgs& a0, const MarchLaunch& l, int nblocks, cudaStream_t s) {
         StageArgs a = a0;
-        const MarchLaunch l = march_launch(a, 3, nblocks);
         a.fin.ctas = l.ctas();
         mixed_march_kernel<RIEMANN, GATED><<<l.ctas(), MarchShape::NT, MarchShape::SMEM_BYTES, s>>>(a, l.z0, l.z1, l.plan.lz, nblocks);
         return cudaGetLastError();
@@ -667,9 +669,8 @@ template <int RIEMANN, bool GATED> struct March2K {
     using S = March2Shape<kMarch2W>;
     static constexpr auto kern = mixed_march2_kernel<RIEMANN, GATED, kMarch2W, kMarch2Cost.resident>;
     static cudaError_t prepare() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES); }
-    static cudaError_t launch(const StageArgs& a0, int nblocks, cudaStream_t s) {
+    static cudaError_t launch(const StageArgs& a0, const MarchLaunch& l, int nblocks, cudaStream_t s) {
         StageArgs a = a0;
-        const MarchLaunch l = march_launch(a, 2, nblocks);
         a.fin.ctas = l.ctas();
         kern<<<l.ctas(), S::NT, S::SMEM_BYTES, s>>>(a, l.z0, l.z1, l.plan.lz, nblocks);
         return cudaGetLastError();

@@ -28,8 +28,10 @@ template <int DIM, int RECON, int RIEMANN, bool FULL> struct MixedK {
         return e;
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
-        if constexpr (kHasMarch<DIM, RECON, FULL>)
-            if (marches(a, DIM, nblocks)) return MarchOf<DIM, RIEMANN, false>::launch(a, nblocks, s);
+        if constexpr (kHasMarch<DIM, RECON, FULL>) {
+            MarchLaunch l;
+            if (marches(a, DIM, nblocks, l)) return MarchOf<DIM, RIEMANN, false>::launch(a, l, nblocks, s);
+        }
         mixed_stage_kernel<DIM, RECON, RIEMANN, T::X, T::Y, T::Z, T::NT, false, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
@@ -47,8 +49,10 @@ template <int DIM, int RIEMANN, bool FULL> struct GatedK {
         return e;
     }
     static cudaError_t launch(const StageArgs& a, int nblocks, cudaStream_t s) {
-        if constexpr (kHasMarch<DIM, kWeno5, FULL>)
-            if (marches(a, DIM, nblocks)) return MarchOf<DIM, RIEMANN, true>::launch(a, nblocks, s);
+        if constexpr (kHasMarch<DIM, kWeno5, FULL>) {
+            MarchLaunch l;
+            if (marches(a, DIM, nblocks, l)) return MarchOf<DIM, RIEMANN, true>::launch(a, l, nblocks, s);
+        }
         mixed_stage_kernel<DIM, kWeno5, RIEMANN, T::X, T::Y, T::Z, T::NT, true, FULL><<<nblocks, T::NT, S::SMEM_BYTES, s>>>(a);
         return cudaGetLastError();
     }
@@ -95,7 +99,10 @@ cudaError_t mixed_viscous_prepare() {
         e = cudaFuncSetAttribute(mixed_viscous_march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ViscMarchShape::SMEM_BYTES);
     return e;
 }
-bool mixed_stage_marches(const StageArgs& a, int dim, int nblocks) { return marches(a, dim, nblocks); }
+bool mixed_stage_marches(const StageArgs& a, int dim, int nblocks) {
+    MarchLaunch l;
+    return marches(a, dim, nblocks, l);
+}
 cudaError_t mixed_viscous_launch(const ViscArgs& a, int nblocks, cudaStream_t s) {
     if (a.all_periodic && !a.bc.slot) return visc_march_launch(a, nblocks, s);
     mixed_viscous_kernel<8, 8, 8, kMixedViscNT><<<nblocks, kMixedViscNT, MixedViscShape<8, 8, 8>::SMEM_BYTES, s>>>(a);

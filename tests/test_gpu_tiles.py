@@ -38,7 +38,7 @@ def march_planes(nx, ny, nz=1):
         full, rest = divmod(cols * -(-n // lz), 148 * resident)
         return full * (fill + lz * (base + per * resident)) + (fill + lz * (base + per * -(-rest // 148)) if rest else 0.0)
 
-    lz = min([k for k in range(1, n + 1) if k < 32 or k % 4 == 0], key=us)
+    lz = min(range(1, n + 1), key=us)
     full, rest = divmod(tiles, 148 * (3 if three else 4))
     tiled = (0.0 if three else 1.0) + full * (35.0 if three else 12.0) + ((19.0 + 7.5 * -(-rest // 148) if three else 8.0 + 1.9 * -(-rest // 148)) if rest else 0.0)
     return lz if us(lz) < tiled else 0
