@@ -93,8 +93,9 @@ __device__ __forceinline__ void thin_row_mixed(const StageArgs& a, const GasF& g
         const float r = max_nan(w[0], Num<float>::eos_eps), p = max_nan(w[3 * RP], Num<float>::eos_eps), u = w[RP], v = w[2 * RP];
         const float cs = sqrt_f(__fmul_rn(__fmul_rn(gas.g, __fadd_rn(p, gas.pi)), rcp_f(r)));
         const float s = max_nan(fabsf(__fsub_rn(v, cs)), fabsf(__fadd_rn(v, cs)));
-        const float rE = __fmaf_rn(__fmul_rn(0.5f, r), __fmaf_rn(u, u, __fmul_rn(v, v)), __fmul_rn(__fadd_rn(p, gas.gpi), gas.g1));
-        same = __fmul_rn(s, rE) < 0.25f * kFaceRange;   // (finite fluxes; a state beyond riemann_f's range is solved)
+        // finite fluxes: with s = |v| + c the energy per volume is at most r (u^2 + s^2) times 1 / (gamma - 1) or a half, and s times
+        // it their bound (a state beyond riemann_f's range is solved)
+        same = __fmul_rn(__fmul_rn(s, r), __fmaf_rn(u, u, __fmul_rn(s, s))) < 0.01f * kFaceRange;
         if (same && s > smax) smax = s;
     }
     if (!same) {
